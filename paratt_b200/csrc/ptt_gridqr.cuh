@@ -1,71 +1,115 @@
-// Cholesky QR of unfoldings with up to 64 columns by the whole GPU (included
+// Cholesky QR of unfoldings with 33 to 128 columns by the whole GPU (included
 // by ptt_round.cu inside its anonymous namespace, after ptt_cholqr.cuh).
 //
 // At 64 columns a bond's unfolding (16384 x 64 doubles at d = 40, n = 256,
-// rank 64: 8.4 MB) no longer fits in one cluster's shared memory, and the
+// rank 64: 8.4 MB) does not fit one cluster's shared memory, and the
 // Householder TSQR costs one block barrier per reflector and tree level.
-// Here the rows are spread over all SMs and the same Gram-stage sequence as
-// the cluster kernel (ptt_cholqr.cuh) runs as one launch per stage:
+// Here the rows are spread over all SMs and A = Q R is a sequence of Gram
+// stages (the decisions are those of gq::decide below), two launches each:
 //
-//   stage 0        CTA b loads rows [b rpb, (b+1) rpb) of A, forms the
-//                  partial Gram matrix of its rows;
-//   stage s >= 1   CTA b loads its rows of Q_{s-1} (A for s = 1), applies the
-//                  factor of the previous stage by a row-wise triangular solve
-//                  (Q_s = Q_{s-1} R_s^{-1}), writes Q_s and forms the partial
-//                  Gram matrix of Q_s;
+//   k_gq_rows    CTA b loads its rows of Q_{s-1} (A for s <= 1), applies the
+//                factor of the previous stage by a row-wise triangular solve
+//                (s >= 1: Q_s = Q_{s-1} R_s^{-1}, written back) and forms the
+//                partial Gram matrix of its rows of Q_s;
+//   k_gq_decide  CTA t sums upper 8 x 8 tile t over all partials in a fixed
+//                order; the last CTA to finish (atomic ticket, no waiting)
+//                takes the decision of the stage from the whole Gram matrix.
 //
-// and the partials are summed in a fixed order by the last-arriving CTA of
-// each group of GROUP CTAs (atomic ticket, no waiting), then by the
-// last-arriving group, which takes the decision of the stage exactly as the
-// cluster kernel does: done (max|Q^T Q - I| <= 1e-13), a first-order factor
-// I + striu(E) + diag(E)/2 (finishing without another Gram stage when
-// max|E| <= 1e-8), a Cholesky factor of G, or of G + sigma I when a pivot is
-// not positive or the pivots span more than 12 decades (shifted Cholesky QR,
-// Fukaya, Kannan, Nakatsukasa, Yamamoto, Yanagisawa, SIAM J. Sci. Comput. 42
-// (2020), sigma = 11 (m c + c (c + 1)) u ||Q||_F^2).  The host launches MAXST
-// stages; a stage finds the state left by the previous one and returns at
-// once when the factorisation is finished or has fallen back.  The row-wise
-// triangular solve changes A = Q R by O(u ||A||) per stage, so R carries the
-// singular values to the accuracy of a Householder R.
+// The sum is a launch of its own because one SM reading all partials took
+// longer than everything else it had to do (the partials are 18 KB each at 64
+// columns and 70 KB at 128; a single SM reads them at ~64 bytes a cycle).
+//
+// A stage with Gram matrix G = Q_s^T Q_s, accumulated R = T (A = Q_s T):
+//   * columns whose part of A is below the rounding of A are dropped: column
+//     j of Q_s adds q_j T_j: to A, at most |q_j| max_i |T_ji| / |a_i| of each
+//     column a_i; where that is below 0.5 sqrt(c) u it is rounding noise of A,
+//     and q_j and T_j: are set to zero (exactly zero columns of A likewise).
+//     Unfoldings of sums are numerically rank-deficient: without this the
+//     noise directions kept the sequence busy for up to eight stages, and 11
+//     of the 78 factorisations of a rank-64 rounding with d = 40 fell back;
+//   * s >= 1 and max|G - I| <= TAU over the other columns: done, R = T;
+//   * s >= 1 and max|G - I| <= FIRST: R_{s+1} = I + striu(E) + diag(E)/2, the
+//     Cholesky factor of I + E to first order; when max|E| <= FIRST_DONE that
+//     finishes without another Gram stage;
+//   * otherwise R_{s+1} = chol(H) D with D = diag(|q_j|) and H = D^-1 G D^-1
+//     (unit diagonal, so the scale of a column does not matter).  A pivot
+//     below PIV is set to PIV and the rest of its row of R to zero: the column
+//     is only rescaled and is orthogonalised against the others in the next
+//     stage, where it has unit norm again.  So every stage resolves another
+//     seven decades of the spectrum, whatever the condition: condition 1e25
+//     and exactly repeated columns take four or five stages.  (Shifted
+//     Cholesky QR -- Fukaya, Kannan, Nakatsukasa, Yamamoto, Yanagisawa, SIAM
+//     J. Sci. Comput. 42 (2020) -- resolves five decades a stage at this size
+//     and perturbs the columns that need no shift.)
+// The row-wise triangular solve changes A = Q R by O(u |a_j|) per column and
+// stage, so R carries the singular values to the accuracy of a Householder R.
+// The host launches MAXST stages; a launch finds the state left by the
+// previous one and returns at once when the factorisation is finished.
 //
 // Q is written to Qbuf: LEFT -> alt[k] (m x c, column-major, its final place);
 // RIGHT_T -> a scratch region (row-major rows of c), from which k_gq_write
 // forms Q V_r after the bond's SVD.  A never changes, so a bond that falls
-// back (NaN, zero matrix or column, no convergence in MAXST stages) is
-// factored by the Householder TSQR from the same input; those kernels skip
-// the bonds finished here (Plan::gqstate).
+// back (NaN, zero matrix, more columns than rows, no convergence in MAXST
+// stages) is factored by the Householder TSQR from the same input; those
+// kernels skip the bonds finished here (Plan::gqstate).
 #pragma once
 
 namespace gq {
 
 constexpr int NT = 256;
-constexpr int CB = 64;                 // column bound
-constexpr int XP = CB + 8;             // pitch of the rows in shared memory: 8 mod 16 doubles, so the
-                                       // four rows of an mma fragment load fall in the two halves of the banks
-constexpr int RP = CB + 2;             // pitch of a factor R (row-major, upper triangular)
-constexpr int GP = CB + 1;             // pitch of the Gram matrix of the deciding CTA
-constexpr int TS = CB / 8;             // Gram tiles are TS x TS, 8 x 8 of them
-constexpr int UP = 36 * TS * TS;       // entries of the 36 upper tiles
-constexpr int GROUP = 8;               // CTAs summed by the first level
-constexpr int RPB_MAX = 112;           // rows per CTA
 constexpr int RPB_MIN = 16;
-constexpr int MAXST = 8;               // stage launches per factorisation: an unfolding of condition ~1e16
-                                       // (numerically rank-deficient) takes three shifted stages, a plain
-                                       // one and a first-order finish -- seven launches
+constexpr int MAXST = 6;               // Gram stages per factorisation
+constexpr int GROUP = 8;               // k_gram: CTAs summed by the first level
 constexpr double TAU = 1e-13;
 constexpr double FIRST = 1e-7;
 constexpr double FIRST_DONE = 1e-8;
 constexpr double U = 1.1102230246251565e-16;
-constexpr int FSZ = CB * RP + CB;      // a factor and its inverse pivots
-constexpr int SCR = CB * GP + 2 * FSZ + 64;  // Gram, two candidate factors, row broadcasts of the deciding CTA
-constexpr size_t SMEM = sizeof(double) * ((size_t)RPB_MAX * XP + (size_t)SCR);
-// the Ozaki Gram (ptt_ozaki.cuh): the digit slices take the scratch region
+constexpr double PIV = 1e-13;          // smallest pivot of the equilibrated Gram matrix that is trusted: its
+                                       // relative error is ~1e-15 / PIV, so the next stage sees max|E| ~ 1e-2
+constexpr double DROP = 0.5 * U;       // times sqrt(c): a column's part of A that is rounding noise
+constexpr double SMALL = 1e-280;       // squared norms below this lose digits to underflow: fall back
+
+// A symmetric or upper triangular CB x CB matrix is kept as its upper 8 x 8
+// tiles: tile (I, J), I <= J, is number J (J + 1) / 2 + I (independent of CB,
+// so c columns use the first tiles), entry (i, j) of a tile at tix(i, j).
+// The swizzle puts the four rows of an mma fragment load, and the four
+// columns of a transposed one, in different banks.
+template <int CB>
+struct Cfg {
+    static constexpr int NB = CB / 8;
+    static constexpr int NTI = NB * (NB + 1) / 2;
+    static constexpr int UP = NTI * 64;          // doubles of the upper tiles
+    static constexpr int XP = CB + 4;            // pitch of the rows in shared memory: 4 mod 16 doubles, so the
+                                                 // 4 x 4 elements of a half-warp's fragment load fall in different
+                                                 // banks (a pitch of 8 mod 16 cost two wavefronts more per load)
+    static constexpr int RPB_MAX = CB <= 64 ? 112 : 128;  // rows per CTA: 16 for each of eight warps
+    static constexpr int FL = UP + CB;           // a factor and its inverse pivots
+    static constexpr size_t SM_ROWS = sizeof(double) * ((size_t)RPB_MAX * XP + FL);
+    static constexpr size_t SM_DEC = sizeof(double) * (2 * (size_t)UP);
+    // record (doubles): State, factor + inverse pivots, accumulated R, 1 / |a_j|, max_j |T_ij| / |a_j|, Gram sums
+    static constexpr long long O_FAC = 8, O_T = O_FAC + FL, O_AN = O_T + UP, O_TM = O_AN + CB, O_G = O_TM + CB;
+    static constexpr long long REC = O_G + UP;
+};
+__device__ __forceinline__ int tix(int i, int j) { return i * 8 + (j ^ ((i & 2) << 1)); }
+__device__ __forceinline__ int tnum(int I, int J) { return (J * (J + 1)) / 2 + I; }
+__device__ __forceinline__ void tile_of(int t, int* I, int* J) {
+    int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((j + 1) * (j + 2) / 2 <= t) j++;
+    while (j * (j + 1) / 2 > t) j--;
+    *J = j;
+    *I = t - j * (j + 1) / 2;
+}
+__device__ __forceinline__ void mma884(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+// the Ozaki Gram (ptt_ozaki.cuh): the digit slices take the factor's region
 // and beyond once the rows are solved; its 64 x 65 sum buffer the rows' region
-constexpr size_t SMEM_OZ = sizeof(double) * (size_t)RPB_MAX * XP + oz::SMEM;
-static_assert(RPB_MAX == oz::KMAX, "one CTA's rows are one exact FP32 accumulation");
-static_assert(SMEM_OZ >= SMEM && RPB_MAX * XP >= 64 * 65, "Ozaki buffers");
-static_assert(CB * GP <= FSZ, "the accumulated R fits a factor buffer");
-static_assert(CB * RP + CB <= SCR, "factor fits the scratch");
+constexpr size_t SM_ROWS_OZ = sizeof(double) * (size_t)Cfg<64>::RPB_MAX * Cfg<64>::XP + oz::SMEM;
+static_assert(Cfg<64>::RPB_MAX == oz::KMAX, "one CTA's rows are one exact FP32 accumulation");
+static_assert(SM_ROWS_OZ >= Cfg<64>::SM_ROWS && Cfg<64>::RPB_MAX * Cfg<64>::XP >= 64 * 65, "Ozaki buffers");
+static_assert(Cfg<128>::SM_ROWS <= 227 * 1024 && Cfg<128>::SM_DEC <= 227 * 1024, "shared memory");
 
 enum { RUN = 0, DONE = 1, FALLBACK = 2, FINISH = 4, CHOL = 8 };
 
@@ -76,303 +120,235 @@ struct State {
     int state;   // RUN, DONE, FALLBACK, FINISH
     int fin;     // FINISH: the stage launch that applies the last factor
     int nst;     // factors applied
-    int nshift;  // shifted stages (diagnostic)
+    int ndrop;   // columns dropped (diagnostic)
     int m, c;
     int pad[2];
 };
 
 struct GQ {
-    double* rec;         // State, then the factor and the accumulated R
+    double* rec;         // State, then the arrays of Cfg
     double* part;        // per-CTA partial Gram matrices (UP each)
-    double* gpart;       // per-group sums
     double* qscr;        // Q rows of a RIGHT_T factorisation (row-major, pitch c)
-    int* cnt;            // tickets: [group] ... [ngroups] = top; zero between launches
-    int rpb;             // rows per CTA
+    int* cnt;            // ticket, zero between launches
+    int rpb;             // rows a CTA has room for
+    int nb;              // CTAs of the row launches
 };
-constexpr long long O_FAC = 8;                   // CB x RP factor, then CB inverse pivots
-constexpr long long O_T = O_FAC + CB * RP + CB;  // CB x CB accumulated R (row-major)
-constexpr long long REC = O_T + CB * CB;
 
 // rows per CTA and CTAs for an unfolding of at most mcap rows
-__host__ __forceinline__ int rows_per_cta(long long mcap, int nsm) {
+__host__ __forceinline__ int rows_per_cta(long long mcap, int nsm, int rmax) {
     long long r = (mcap + nsm - 1) / nsm;
     if (r < RPB_MIN) r = RPB_MIN;
-    if (r > RPB_MAX) r = RPB_MAX;
+    if (r > rmax) r = rmax;
     return (int)r;
 }
 __host__ __forceinline__ int ctas(long long mcap, int rpb) {
     long long b = (mcap + rpb - 1) / rpb;
     return (int)(b < 1 ? 1 : b);
 }
+// the rows a CTA takes: the actual ones spread evenly over the launched CTAs
+// (the launch is sized from a bound on m)
+__device__ __forceinline__ int rows_taken(int m, int nb) {
+    const int r = (m + nb - 1) / nb;
+    return r < RPB_MIN ? RPB_MIN : r;
+}
+__device__ __forceinline__ bool shape_ok(int m, int c, int cb, const GQ& g) {
+    return c <= cb && c >= 1 && m >= c && (long long)m <= (long long)g.rpb * g.nb;
+}
 
 // x <- x R^{-1} for the CTA's rows (h of them, zero rows up to a multiple of
-// 8), one warp per 8-row tile, by 8-column blocks in order: the update of
-// block J by the solved blocks, X_J - Y_{<J} R_{<J,J}, on the FP64 tensor
-// cores (mma.m8n8k4, four columns of Y a step), then forward substitution in
-// the 8 x 8 diagonal block, the row's four lanes passing each solved entry by
-// a shuffle.  Rows are independent, so a warp needs no barrier.  R upper
-// triangular (pitch RP), zero outside the c x c triangle; iv = inverse
-// pivots, zero beyond c.
-__device__ __forceinline__ void tile_solve(double* Xs, int h, const double* R, const double* iv, int c) {
+// 16), one warp per 16 rows, by 8-column blocks in order: the update of block
+// J by the solved blocks, X_J - Y_{<J} R_{<J,J}, on the FP64 tensor cores
+// (two accumulators a tile, so the chain is J products long), then forward
+// substitution in the 8 x 8 diagonal block with one lane per row, the block
+// passed through shared memory: 8 dependent multiply-add pairs, where passing
+// each solved entry between the row's four lanes by shuffles took ~65 cycles
+// an entry.  Rows are independent, so a warp needs no block barrier.  R upper
+// triangular in tiles, iv = inverse pivots, zero beyond c and for a dropped
+// column.
+template <int CB>
+__device__ __forceinline__ void tile_solve(double* Xs, int h, const double* R, const double* iv, int nbc) {
+    constexpr int XP = Cfg<CB>::XP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int li = lane >> 2, lk = lane & 3;
-    const int ntile = (h + 7) >> 3, nb = (c + 7) >> 3;
-    constexpr int NW = NT / 32;
-    // two tiles at a time (t and t + NW), their dependent chains interleaved;
-    // a warp with one tile left solves it twice and stores it once
-    for (int t = warp; t < ntile; t += 2 * NW) {
-        const bool two = t + NW < ntile;
-        double* xa = Xs + (t * 8 + li) * XP;  // this lane's rows
-        double* xb = two ? Xs + ((t + NW) * 8 + li) * XP : xa;
-        for (int J = 0; J < nb; J++) {
+    for (int u = warp; u * 16 < h; u += NT / 32) {
+        double* xa = Xs + (u * 16 + li) * XP;  // this lane's fragment rows
+        double* xb = xa + 8 * XP;
+        double* xr = Xs + (u * 16 + (lane & 15)) * XP;
+        for (int J = 0; J < nbc; J++) {
             const double2 ca = *(const double2*)(xa + 8 * J + 2 * lk);
             const double2 cb = *(const double2*)(xb + 8 * J + 2 * lk);
-            double a0 = ca.x, a1 = ca.y, b0 = cb.x, b1 = cb.y;  // columns 8J + 2lk, 8J + 2lk + 1
-            for (int kk = 0; kk < 2 * J; kk++) {
-                const double bv = R[(4 * kk + lk) * RP + 8 * J + li];
-                const double ava = -xa[4 * kk + lk], avb = -xb[4 * kk + lk];
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                             : "+d"(a0), "+d"(a1)
-                             : "d"(ava), "d"(bv));
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                             : "+d"(b0), "+d"(b1)
-                             : "d"(avb), "d"(bv));
+            double a0 = ca.x, a1 = ca.y, b0 = cb.x, b1 = cb.y;
+            double e0 = 0.0, e1 = 0.0, f0 = 0.0, f1 = 0.0;
+            if (J > 0) {
+                for (int I = 0; I < J; I++) {
+                    const double* Rt = R + tnum(I, J) * 64;
+                    const double r0 = Rt[tix(lk, li)], r1 = Rt[tix(lk + 4, li)];
+                    mma884(a0, a1, -xa[8 * I + lk], r0);
+                    mma884(b0, b1, -xb[8 * I + lk], r0);
+                    mma884(e0, e1, -xa[8 * I + 4 + lk], r1);
+                    mma884(f0, f1, -xb[8 * I + 4 + lk], r1);
+                }
+                *(double2*)(xa + 8 * J + 2 * lk) = make_double2(a0 + e0, a1 + e1);
+                *(double2*)(xb + 8 * J + 2 * lk) = make_double2(b0 + f0, b1 + f1);
+                __syncwarp();
             }
-            const double* Rb = R + 8 * J * RP + 8 * J;
+            if (lane < 16) {
+                const double* Rd = R + tnum(J, J) * 64;
+                double x[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int own = j >> 1;
-                const double ivj = iv[8 * J + j];
-                if (lk == own) {
-                    if (j & 1) {
-                        a1 *= ivj;
-                        b1 *= ivj;
-                    } else {
-                        a0 *= ivj;
-                        b0 *= ivj;
-                    }
+                for (int j = 0; j < 8; j += 2) {
+                    const double2 v = *(const double2*)(xr + 8 * J + j);
+                    x[j] = v.x;
+                    x[j + 1] = v.y;
                 }
-                const double ya = __shfl_sync(0xffffffffu, (j & 1) ? a1 : a0, (lane & ~3) | own);
-                const double yb = __shfl_sync(0xffffffffu, (j & 1) ? b1 : b0, (lane & ~3) | own);
-                if (2 * lk > j) {
-                    const double r = Rb[j * RP + 2 * lk];
-                    a0 = fma(-ya, r, a0);
-                    b0 = fma(-yb, r, b0);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const double y = x[j] * iv[8 * J + j];
+                    x[j] = y;
+#pragma unroll
+                    for (int l = j + 1; l < 8; l++) x[l] = fma(-y, Rd[tix(j, l)], x[l]);
                 }
-                if (2 * lk + 1 > j) {
-                    const double r = Rb[j * RP + 2 * lk + 1];
-                    a1 = fma(-ya, r, a1);
-                    b1 = fma(-yb, r, b1);
-                }
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) *(double2*)(xr + 8 * J + j) = make_double2(x[j], x[j + 1]);
             }
-            *(double2*)(xa + 8 * J + 2 * lk) = make_double2(a0, a1);
-            if (two) *(double2*)(xb + 8 * J + 2 * lk) = make_double2(b0, b1);
             __syncwarp();
         }
     }
 }
 
-// Cholesky of one 32-column panel by one warp, lane = column: g[t] holds
-// entry (t, lane) of the panel's symmetric block (rows t < 32); row j of the
-// factor is broadcast through sRow.  Writes R[off + j][off + lane] (pitch RP)
-// and iv[off + j] = 1 / R[off + j][off + j] for j < cc; tracks the pivots.
-__device__ __forceinline__ void chol_panel(double (&g)[32], int cc, int off, double* R, double* iv, double* sRow,
-                                           bool& ok, double& dmin, double& dmax) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-        if (j >= cc) continue;
-        const double d = __shfl_sync(0xffffffffu, g[j], j);
-        ok = ok && (d > 0.0);  // false for NaN
-        dmin = fmin(dmin, d);
-        dmax = fmax(dmax, d);
-        const double dd = d > 0.0 ? d : 1.0;
-        const double inv = rsqrt(dd);
-        const double rj = (lane == j) ? dd * inv : ((lane > j && lane < cc) ? g[j] * inv : 0.0);
-        sRow[lane] = rj;
-        __syncwarp();
-        if (lane > j && lane < cc) {
-#pragma unroll
-            for (int t = j + 1; t < 32; t++) g[t] = fma(-sRow[t], rj, g[t]);
-        }
-        if (lane >= j && lane < cc) R[(off + j) * RP + off + lane] = rj;
-        if (lane == j) iv[off + j] = inv;
-        __syncwarp();
-    }
+// Partial Gram matrix of the CTA's rows on the FP64 tensor cores
+// (mma.m8n8k4, four rows a step; a block's fragment serves as A and as B):
+// four sets of tiles x two halves of the rows for the eight warps, so a
+// fragment loaded once serves every tile of its set.
+template <int CB>
+__host__ __device__ constexpr bool in_set(int s, int I, int J) {
+    constexpr int HB = CB / 16, QB = CB / 32;  // half and quarter of the column blocks
+    return I <= J && (s == 0 ? J < HB : s == 1 ? I >= HB : s == 2 ? (I < QB && J >= HB) : (I >= QB && I < HB && J >= HB));
 }
-
-// Cholesky factor of G + shift I (c x c, pitch GP) by ONE warp in two
-// 32-column panels: R11 = chol(G11); R12 = R11^{-T} G12 (forward
-// substitution, lane = column); S = G22 - R12^T R12 (lane = column, in
-// registers); R22 = chol(S).  Result R (row-major, pitch RP, zero outside the
-// upper c x c triangle), iv[j] = 1 / R[j][j].  Returns false when a pivot is
-// not positive (NaN included); *ratio = min/max pivot.  Two warps can form
-// the plain and the shifted factor at once into different R buffers.
-__device__ bool warp_chol64(const double* G, int c, double shift, double* R, double* iv, double* sRow, double* ratio) {
-    const int lane = threadIdx.x & 31;
-    for (int e = lane; e < CB * RP; e += 32) R[e] = 0.0;
-    for (int e = lane; e < CB; e += 32) iv[e] = 0.0;
-    __syncwarp();
-    bool ok = true;
-    double dmin = 1.0 / 0.0, dmax = 0.0;
-    const int c1 = c < 32 ? c : 32;
-    double g[32];
+template <int CB>
+__host__ __device__ constexpr int set_max() {
+    int mx = 0;
+    for (int s = 0; s < 4; s++) {
+        int n = 0;
+        for (int J = 0; J < CB / 8; J++)
+            for (int I = 0; I <= J; I++) n += in_set<CB>(s, I, J) ? 1 : 0;
+        mx = n > mx ? n : mx;
+    }
+    return mx;
+}
+template <int CB, int S>
+__device__ __forceinline__ void gram_set(const double* Xs, int ks0, int ks1, int nbc, double (&d0)[set_max<CB>()],
+                                         double (&d1)[set_max<CB>()]) {
+    constexpr int XP = Cfg<CB>::XP, NB = CB / 8;
+    const int lane = threadIdx.x & 31, li = lane >> 2, lk = lane & 3;
+    for (int ks = ks0; ks < ks1; ks++) {
+        const double* xr = Xs + (4 * ks + lk) * XP + li;
+        double f[NB];
 #pragma unroll
-    for (int t = 0; t < 32; t++) g[t] = (t < c1 && lane < c1) ? G[t * GP + lane] + (t == lane ? shift : 0.0) : 0.0;
-    chol_panel(g, c1, 0, R, iv, sRow, ok, dmin, dmax);
-    if (c > 32) {
-        const int c2 = c - 32, k = 32 + lane;
-        const bool mine = lane < c2;
-        // R12[:, k]: R11^T y = G[0:32, k]
-        double y[32];
+        for (int b = 0; b < NB; b++) f[b] = b < nbc ? xr[8 * b] : 0.0;  // the blocks no tile of the set uses fold away
+        int t = 0;
 #pragma unroll
-        for (int i = 0; i < 32; i++) y[i] = mine ? G[i * GP + k] : 0.0;
+        for (int J = 0; J < NB; J++) {
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-            const double yi = y[i] * iv[i];
-            y[i] = yi;
-#pragma unroll
-            for (int t = i + 1; t < 32; t++) y[t] = fma(-R[i * RP + t], yi, y[t]);
-        }
-        if (mine) {
-#pragma unroll
-            for (int i = 0; i < 32; i++) R[i * RP + k] = y[i];
-        }
-        __syncwarp();
-        // P = R12^T R12 on the FP64 tensor cores (the 10 upper 8 x 8 tiles, k
-        // over the 32 rows of R12), parked in the lower-left quarter of R,
-        // which is zero in the result; S[32 + t][k] = G[32 + t][k] + shift
-        // [t == lane] - P[t][lane] (only the upper entries t <= lane are used)
-        {
-            const int li = lane >> 2, lk = lane & 3;
-            double p0[10], p1[10];
-#pragma unroll
-            for (int q = 0; q < 10; q++) {
-                p0[q] = 0.0;
-                p1[q] = 0.0;
-            }
-#pragma unroll
-            for (int k0 = 0; k0 < 32; k0 += 4) {
-                double f[4];
-#pragma unroll
-                for (int bb = 0; bb < 4; bb++) f[bb] = R[(k0 + lk) * RP + 32 + 8 * bb + li];
-                int q = 0;
-#pragma unroll
-                for (int I = 0; I < 4; I++)
-#pragma unroll
-                    for (int J = I; J < 4; J++, q++)
-                        asm volatile(
-                            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                            : "+d"(p0[q]), "+d"(p1[q])
-                            : "d"(f[I]), "d"(f[J]));
-            }
-            int q = 0;
-#pragma unroll
-            for (int I = 0; I < 4; I++)
-#pragma unroll
-                for (int J = I; J < 4; J++, q++) {
-                    R[(32 + 8 * I + li) * RP + 8 * J + 2 * lk] = p0[q];
-                    R[(32 + 8 * I + li) * RP + 8 * J + 2 * lk + 1] = p1[q];
+            for (int I = 0; I <= J; I++) {
+                if (in_set<CB>(S, I, J)) {
+                    if (J < nbc) mma884(d0[t], d1[t], f[I], f[J]);
+                    t++;
                 }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < 32; t++) {
-            const double pt = R[(32 + t) * RP + lane];
-            g[t] = (mine && t < c2) ? G[(32 + t) * GP + k] + (t == lane ? shift : 0.0) - pt : 0.0;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < 32; t++) R[(32 + t) * RP + lane] = 0.0;
-        __syncwarp();
-        chol_panel(g, c2, 32, R, iv, sRow, ok, dmin, dmax);
-    }
-    __syncwarp();
-    *ratio = dmax > 0.0 ? dmin / dmax : 0.0;
-    return ok;
-}
-
-// Partial Gram matrix (upper 8 x 8 tiles) of the CTA's rows on the FP64
-// tensor cores: warp w accumulates tiles w, w + 8, ... over all rows, four
-// rows per mma.m8n8k4 (A = the tile's row-block columns transposed, B = its
-// column-block columns), and writes them straight to P (tile q at P + 64 q).
-__device__ __forceinline__ void gram_fp64(const double* Xs, int h, double* P) {
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int li = lane >> 2, lk = lane & 3;
-    constexpr int NWP = NT / 32, TPW = (36 + NWP - 1) / NWP;
-    double c0[TPW], c1[TPW];
-    int oa[TPW], ob[TPW];
-#pragma unroll
-    for (int t = 0; t < TPW; t++) {
-        int ti = 0, tj = 0;
-        if (warp + NWP * t < 36) cq::upper_tile(warp + NWP * t, &ti, &tj);
-        oa[t] = ti * TS + li;
-        ob[t] = tj * TS + li;
-        c0[t] = 0.0;
-        c1[t] = 0.0;
-    }
-    for (int r = 0; r < h; r += 4) {
-        const int row = r + lk;
-        const double* xr = Xs + row * XP;
-        const bool ok = row < h;
-#pragma unroll
-        for (int t = 0; t < TPW; t++) {
-            if (warp + NWP * t < 36) {
-                const double av = ok ? xr[oa[t]] : 0.0;
-                const double bv = ok ? xr[ob[t]] : 0.0;
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                             : "+d"(c0[t]), "+d"(c1[t])
-                             : "d"(av), "d"(bv));
             }
         }
     }
+}
+// store (how 0), or add what is stored at `red` and write to P (how 1)
+template <int CB, int S>
+__device__ __forceinline__ void gram_out(int nbc, const double (&d0)[set_max<CB>()], const double (&d1)[set_max<CB>()],
+                                         double* red, double* P, bool first) {
+    constexpr int NB = CB / 8;
+    const int lane = threadIdx.x & 31, li = lane >> 2, lk = lane & 3;
+    const int o = tix(li, 2 * lk);
+    int t = 0;
 #pragma unroll
-    for (int t = 0; t < TPW; t++)
-        if (warp + NWP * t < 36)
-            *(double2*)(P + (warp + NWP * t) * TS * TS + li * TS + 2 * lk) = make_double2(c0[t], c1[t]);
+    for (int J = 0; J < NB; J++) {
+#pragma unroll
+        for (int I = 0; I <= J; I++) {
+            if (in_set<CB>(S, I, J)) {
+                if (J < nbc) {
+                    const int at = tnum(I, J) * 64 + o;
+                    if (first) {
+                        *(double2*)(red + at) = make_double2(d0[t], d1[t]);
+                    } else {
+                        const double2 v = *(const double2*)(red + at);
+                        *(double2*)(P + at) = make_double2(d0[t] + v.x, d1[t] + v.y);
+                    }
+                }
+                t++;
+            }
+        }
+    }
+}
+// Xs: h rows, zero rows up to a multiple of 4; red: UP doubles of shared memory
+template <int CB>
+__device__ __forceinline__ void gram_fp64(const double* Xs, int h, int nbc, double* red, double* P) {
+    const int warp = threadIdx.x >> 5, set = warp & 3, half = warp >> 2;
+    const int nks = (h + 3) >> 2, mid = (nks + 1) >> 1;
+    const int ks0 = half ? mid : 0, ks1 = half ? nks : mid;
+    double d0[set_max<CB>()], d1[set_max<CB>()];
+#pragma unroll
+    for (int t = 0; t < set_max<CB>(); t++) d0[t] = d1[t] = 0.0;
+    switch (set) {
+        case 0: gram_set<CB, 0>(Xs, ks0, ks1, nbc, d0, d1); break;
+        case 1: gram_set<CB, 1>(Xs, ks0, ks1, nbc, d0, d1); break;
+        case 2: gram_set<CB, 2>(Xs, ks0, ks1, nbc, d0, d1); break;
+        default: gram_set<CB, 3>(Xs, ks0, ks1, nbc, d0, d1);
+    }
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++) {
+        if ((half == 1) == (pass == 0)) {
+            switch (set) {
+                case 0: gram_out<CB, 0>(nbc, d0, d1, red, P, pass == 0); break;
+                case 1: gram_out<CB, 1>(nbc, d0, d1, red, P, pass == 0); break;
+                case 2: gram_out<CB, 2>(nbc, d0, d1, red, P, pass == 0); break;
+                default: gram_out<CB, 3>(nbc, d0, d1, red, P, pass == 0);
+            }
+        }
+        if (pass == 0) __syncthreads();
+    }
 }
 
-// One stage of the factorisation of core k's unfolding (mode); gridDim.x CTAs
-// of g.rpb rows each.  OZ: the Gram partials by the Ozaki split on the
-// fifth-generation tensor cores (ptt_ozaki.cuh) instead of FP64 mma.
-template <bool OZ>
-__global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int mode, Plan pl, GQ g, double* ws,
-                                                    int stage, long long* qstat) {
+// The rows of one stage of the factorisation of core k's unfolding (mode);
+// g.nb CTAs with room for g.rpb rows each.  OZ: the Gram partials by the
+// Ozaki split on the fifth-generation tensor cores (ptt_ozaki.cuh) instead
+// of FP64 mma (64 columns only).
+// Bound by latency: at 111 rows x 64 columns the loads, the solve's chain of
+// 8 blocks and 126 products a warp.  One stage at 16384 x 64 (first / later
+// stages): see the figures in k_gq_decide.
+template <int CB, bool OZ>
+__global__ void __launch_bounds__(NT, 1) k_gq_rows(const DevDesc* D, int k, int mode, Plan pl, GQ g, int stage) {
     PTT_PDL_ENTRY();
+    using C = Cfg<CB>;
+    constexpr int XP = C::XP;
     extern __shared__ __align__(128) double gsm[];
-    double* Xs = gsm;                     // rpb x XP rows
-    double* sScr = Xs + RPB_MAX * XP;     // factor; Gram partials; decision arrays
-    __shared__ int s_state, s_fin, s_ticket, s_flags, s_cok[2];
-    __shared__ double s_cratio[2];
-    __shared__ double s_red[NT / 32][2];
-    State* st = (State*)g.rec;
+    double* Xs = gsm;                       // RPB_MAX x XP rows
+    double* sF = Xs + C::RPB_MAX * XP;      // factor tiles, inverse pivots; then the Gram halves
+    __shared__ int s_go, s_fin;
+    const State* st = (const State*)g.rec;
     const View A = make_view(D, k, mode, false);
     const int m = A.m, c = A.c;
-    const int tid = threadIdx.x;
-    const int rpb = g.rpb, nb = (int)gridDim.x, b = (int)blockIdx.x;
-    if (stage == 0) {
-        if (c > CB || c < 1 || m < c || (long long)m > (long long)rpb * nb) {  // uniform
-            if (b == 0 && tid == 0) {
-                st->state = FALLBACK;
-                st->nst = 0;
-                st->m = m;
-                st->c = c;
-                if (qstat) atomicAdd((unsigned long long*)(qstat + 1), 1ull);
-            }
-            return;
-        }
-        if (pl.work && b == 0 && tid == 0) atomicAdd(pl.work, 16.0 * (double)m * (double)c);
-    } else {
+    const int tid = threadIdx.x, b = (int)blockIdx.x;
+    if (!shape_ok(m, c, CB, g)) return;  // uniform; k_gq_decide records the fallback
+    const int rt = rows_taken(m, g.nb), r0 = b * rt;
+    if (r0 >= m) return;
+    if (stage > 0) {
         if (tid == 0) {
-            s_state = ldcg(&st->state);
-            s_fin = ldcg(&st->fin);
+            const int s = ldcg(&st->state);
+            s_fin = s == FINISH;
+            s_go = s == RUN || (s == FINISH && ldcg(&st->fin) == stage);
         }
         __syncthreads();
-        if (!(s_state == RUN || (s_state == FINISH && s_fin == stage))) return;
+        if (!s_go) return;
     }
-    const int r0 = b * rpb;
-    const int h = (m - r0) < rpb ? ((m - r0) > 0 ? (m - r0) : 0) : rpb;
+    const int h = (m - r0) < rt ? (m - r0) : rt;
+    const int h16 = (h + 15) & ~15, nbc = (c + 7) >> 3;
     // Qbuf: where the Q_s rows live
     View Qv;
     if (mode == LEFT) {
@@ -385,56 +361,71 @@ __global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int
         Qv.cs = 1;
     }
     const View& src = (stage <= 1) ? A : Qv;
-    // this CTA's rows (zero beyond c), every element in flight by cp.async
-    for (int e = tid; e < ((h + 7) & ~7) * XP; e += NT) Xs[e] = 0.0;  // whole 8-row tiles
-    if (stage >= 1) {  // the factor of the previous stage (all loads in flight first)
-        const double* F = g.rec + O_FAC;
-        constexpr int FL = CB * RP + CB, FPT = (FL + NT - 1) / NT;
-        double f[FPT];
-#pragma unroll
-        for (int k = 0; k < FPT; k++) f[k] = (tid + k * NT < FL) ? ldcg(F + tid + k * NT) : 0.0;
-#pragma unroll
-        for (int k = 0; k < FPT; k++)
-            if (tid + k * NT < FL) sScr[tid + k * NT] = f[k];
+    const unsigned xs0 = (unsigned)__cvta_generic_to_shared(Xs);
+    if (stage > 0) {  // the factor of the previous stage, 16 bytes at a time (UP and CB are even)
+        const unsigned f0 = (unsigned)__cvta_generic_to_shared(sF);
+        const double* F = g.rec + C::O_FAC;
+        const int used = nbc * (nbc + 1) * 32;
+        for (int e = 2 * tid; e < used; e += 2 * NT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(f0 + 8u * e), "l"(F + e) : "memory");
+        for (int e = 2 * tid; e < CB; e += 2 * NT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(f0 + 8u * (C::UP + e)), "l"(F + C::UP + e)
+                         : "memory");
     }
-    __syncthreads();
-    {
-        const unsigned xs0 = (unsigned)__cvta_generic_to_shared(Xs);
-        if (src.rs == 1) {
-            // column-major: a warp copies 4 rows x 8 columns at a time (32
-            // contiguous bytes of each column; the 4 rows fall in different
-            // bank halves)
-            const int nrb = (h + 3) / 4, ncb = (c + 7) / 8;
-            const int lr = (tid & 31) & 3, lc = (tid & 31) >> 2;
-            for (int t = tid >> 5; t < nrb * ncb; t += NT / 32) {
-                const int cb = t / nrb, rb = t - cb * nrb;
-                const int row = rb * 4 + lr, col = cb * 8 + lc;
-                if (row < h && col < c) {
-                    const double* gp = src.p + (long long)(r0 + row) + (long long)col * src.cs;
-                    const unsigned sa = xs0 + 8u * (unsigned)(row * XP + col);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gp) : "memory");
-                }
-            }
-        } else {  // row-major rows of c: element f = row c + col, stepped without divisions
-            const int dq = NT / c, dr = NT - dq * c;
-            int row = tid / c, col = tid - row * c;
-            for (; row < h;) {
-                const double* gp = src.p + (long long)(r0 + row) * src.rs + (long long)col * src.cs;
+    // this CTA's rows, every element in flight by cp.async; zeros beyond c up
+    // to the block and beyond h up to 16 rows
+    if (src.rs == 1) {
+        // column-major: a warp copies 4 rows x 8 columns at a time (32
+        // contiguous bytes of each column)
+        const int nrb = (h + 3) / 4, ncb = (c + 7) / 8;
+        const int lr = (tid & 31) & 3, lc = (tid & 31) >> 2;
+        for (int t = tid >> 5; t < nrb * ncb; t += NT / 32) {
+            const int cb = t / nrb, rb = t - cb * nrb;
+            const int row = rb * 4 + lr, col = cb * 8 + lc;
+            if (row < h && col < c) {
+                const double* gp = src.p + (long long)(r0 + row) + (long long)col * src.cs;
                 const unsigned sa = xs0 + 8u * (unsigned)(row * XP + col);
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gp) : "memory");
-                row += dq;
-                col += dr;
-                if (col >= c) {
-                    col -= c;
-                    row++;
-                }
             }
         }
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
+    } else if ((c & 1) == 0) {  // row-major rows of an even c: pairs (every row starts on 16 bytes)
+        const int c2 = c >> 1, dq = NT / c2, dr = NT - dq * c2;
+        int row = tid / c2, col = tid - row * c2;
+        const double* base = src.p + (long long)r0 * c;
+        for (; row < h;) {
+            const unsigned sa = xs0 + 8u * (unsigned)(row * XP + 2 * col);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(base + (long long)row * c + 2 * col)
+                         : "memory");
+            row += dq;
+            col += dr;
+            if (col >= c2) {
+                col -= c2;
+                row++;
+            }
+        }
+    } else {
+        const int dq = NT / c, dr = NT - dq * c;
+        int row = tid / c, col = tid - row * c;
+        const double* base = src.p + (long long)r0 * c;
+        for (; row < h;) {
+            const unsigned sa = xs0 + 8u * (unsigned)(row * XP + col);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(base + (long long)row * c + col)
+                         : "memory");
+            row += dq;
+            col += dr;
+            if (col >= c) {
+                col -= c;
+                row++;
+            }
+        }
     }
+    const int cz = (OZ ? CB : 8 * nbc) - c;
+    for (int e = tid; e < h * cz; e += NT) Xs[(e / cz) * XP + c + e % cz] = 0.0;
+    for (int e = tid; e < (h16 - h) * XP; e += NT) Xs[h * XP + e] = 0.0;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
-    if (stage >= 1) {
-        tile_solve(Xs, h, sScr, sScr + CB * RP, c);
+    if (stage > 0) {
+        tile_solve<CB>(Xs, h, sF, sF + C::UP, nbc);
         __syncthreads();
         if (Qv.rs == 1) {  // column-major, in the load's 4 x 8 warp tiles
             const int nrb = (h + 3) / 4, ncb = (c + 7) / 8;
@@ -448,7 +439,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int
             const int dq = NT / c, dr = NT - dq * c;
             int row = tid / c, col = tid - row * c;
             for (; row < h;) {
-                Qv.p[(long long)(r0 + row) * Qv.rs + (long long)col * Qv.cs] = Xs[row * XP + col];
+                Qv.p[(long long)(r0 + row) * c + col] = Xs[row * XP + col];
                 row += dq;
                 col += dr;
                 if (col >= c) {
@@ -457,249 +448,325 @@ __global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int
                 }
             }
         }
-        if (s_state == FINISH) return;  // the last factor is applied: Q is final
+        if (s_fin) return;  // the last factor is applied: Q is final
     }
-    // partial Gram matrix (upper 8 x 8 tiles) of this CTA's rows
+    double* P = g.part + (long long)b * C::UP;
     if constexpr (OZ)
-        oz::gram_partial<NT>(Xs, XP, h, c, (unsigned char*)sScr, Xs, g.part + (long long)b * UP);
+        oz::gram_partial<NT>(Xs, XP, h, c, (unsigned char*)sF, Xs, P);
     else
-        gram_fp64(Xs, h, g.part + (long long)b * UP);
-    // first level: the last CTA of each group sums the group's partials
-    const int ngroups = (nb + GROUP - 1) / GROUP;
-    const int grp = b / GROUP;
-    const int gsize = (nb - grp * GROUP) < GROUP ? (nb - grp * GROUP) : GROUP;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_ticket = atomicAdd(&g.cnt[grp], 1);
-    __syncthreads();
-    if (s_ticket != gsize - 1) return;
-    if (tid == 0) g.cnt[grp] = 0;
-    __threadfence();
-    {
-        // every load of the thread's entries in flight before the sums (in
-        // CTA order; absent CTAs add exact zeros)
-        const double* P = g.part + (long long)grp * GROUP * UP;
-        double* Gp = g.gpart + (long long)grp * UP;
-        constexpr int UPT = (UP + NT - 1) / NT;
-        double v[UPT][GROUP];
+        gram_fp64<CB>(Xs, h, nbc, sF, P);
+}
+
+// Cholesky factor of H in the tiles at sG (nbc column blocks), in place, by
+// the whole CTA: per block column, every panel thread factors the 8 x 8
+// diagonal block in its own registers (the same 8 steps in every thread, so
+// nothing is broadcast), solves one column of the block row against it, and
+// after a barrier all warps update the trailing tiles on the FP64 tensor
+// cores.  A pivot not above PIV is set to PIV and its row to zero; a column
+// outside `alive` (one byte of bits per block) gets a zero row.  rinv[j] =
+// 1 / R[j][j] (zero where not alive).
+// 64 columns: 8 x ~1.7k cycles where one warp with lane = column took ~45k
+// (540 a column: a shuffle, the reciprocal square root and a shared-memory
+// broadcast on the chain of every column).
+template <int CB>
+__device__ void chol_tiles(double* sG, int nbc, int c, const unsigned char* alive, double* rinv) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, li = lane >> 2, lk = lane & 3;
+    for (int J = 0; J < nbc; J++) {
+        double r[8][8], inv[8];
+        const int col = 8 * J + 8 + tid;  // this thread's column of the block row
+        const unsigned live = alive[J];
+        if (tid < CB) {
+            const double* G = sG + tnum(J, J) * 64;
 #pragma unroll
-        for (int k = 0; k < UPT; k++) {
-            const int u = tid + k * NT;
+            for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int t = 0; t < GROUP; t++) v[k][t] = (u < UP && t < gsize) ? ldcg(P + (long long)t * UP + u) : 0.0;
-        }
+                for (int j = i; j < 8; j++) r[i][j] = G[tix(i, j)];
+            unsigned weak = 0;
 #pragma unroll
-        for (int k = 0; k < UPT; k++) {
-            const int u = tid + k * NT;
-            double a = 0.0;
+            for (int j = 0; j < 8; j++) {
+                const bool on = (live >> j) & 1u;
+                const double p = r[j][j];
+                const bool good = p > PIV;  // false for NaN
+                const double pp = good ? p : PIV;
+                const double iv = on ? rsqrt(pp) : 0.0;
+                const double io = good ? iv : 0.0;
+                r[j][j] = on ? pp * iv : 0.0;
+                inv[j] = iv;
+                if (!(on && good)) weak |= 1u << j;
 #pragma unroll
-            for (int t = 0; t < GROUP; t++) a += v[k][t];
-            if (u < UP) Gp[u] = a;
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_ticket = atomicAdd(&g.cnt[ngroups], 1);
-    __syncthreads();
-    if (s_ticket != ngroups - 1) return;
-    if (tid == 0) g.cnt[ngroups] = 0;
-    __threadfence();
-    // ---- the deciding CTA: G = sum of the groups in order --------------------
-    double* sG = sScr;              // CB x GP
-    double* sFa = sG + CB * GP;     // CB x RP factor + CB inverse pivots: plain Cholesky (or first order)
-    double* sFb = sFa + FSZ;        // the same for the shifted Cholesky
-    double* sRow = sFb + FSZ;       // 2 x 32 row broadcasts of the two Cholesky warps
-    for (int e = tid; e < CB * GP; e += NT) sG[e] = 0.0;
-    if (tid == 0) s_flags = 0;
-    __syncthreads();
-    {
-        // the groups' sums in order, all of a thread's entries of eight groups
-        // in flight at a time
-        constexpr int UPT = (UP + NT - 1) / NT;
-        double vs[UPT];
+                for (int l = j + 1; l < 8; l++) r[j][l] *= io;
 #pragma unroll
-        for (int k = 0; k < UPT; k++) vs[k] = 0.0;
-        for (int t0 = 0; t0 < ngroups; t0 += 8) {
-            double w8[UPT][8];
+                for (int i = j + 1; i < 8; i++)
 #pragma unroll
-            for (int k = 0; k < UPT; k++) {
-                const int u = tid + k * NT;
-#pragma unroll
-                for (int t = 0; t < 8; t++)
-                    w8[k][t] = (u < UP && t0 + t < ngroups) ? ldcg(g.gpart + (long long)(t0 + t) * UP + u) : 0.0;
+                    for (int l = i; l < 8; l++) r[i][l] = fma(-r[j][i], r[j][l], r[i][l]);
             }
+            if (col < 8 * nbc) {
+                double* Gc = sG + tnum(J, col >> 3) * 64;
+                double y[8];
 #pragma unroll
-            for (int k = 0; k < UPT; k++)
+                for (int i = 0; i < 8; i++) y[i] = Gc[tix(i, col & 7)];
 #pragma unroll
-                for (int t = 0; t < 8; t++) vs[k] += w8[k][t];
-        }
+                for (int i = 0; i < 8; i++) {
+                    y[i] = ((weak >> i) & 1u) ? 0.0 : y[i] * inv[i];
 #pragma unroll
-        for (int k = 0; k < UPT; k++) {
-            const int u = tid + k * NT;
-            if (u >= UP) continue;
-            const int qq = u / (TS * TS), w = u - qq * (TS * TS);
-            int a0, b0;
-            cq::upper_tile(qq, &a0, &b0);
-            const int gi = a0 * TS + w / TS, gj = b0 * TS + w % TS;
-            if (gi < c && gj < c) {
-                sG[gi * GP + gj] = vs[k];
-                sG[gj * GP + gi] = vs[k];
+                    for (int l = i + 1; l < 8; l++) y[l] = fma(-r[i][l], y[i], y[l]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) Gc[tix(i, col & 7)] = y[i];
             }
         }
+        __syncthreads();
+        if (tid == 0) {  // the diagonal block, read by every panel thread until the barrier
+            double* G = sG + tnum(J, J) * 64;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) G[tix(i, j)] = j >= i ? r[i][j] : 0.0;
+                rinv[8 * J + i] = inv[i];
+            }
+        }
+        const int n = nbc - J - 1;
+        for (int t = warp; t < n * (n + 1) / 2; t += NT / 32) {
+            int I, K;
+            tile_of(t, &I, &K);
+            I += J + 1;
+            K += J + 1;
+            const double* Ra = sG + tnum(J, I) * 64;
+            const double* Rb = sG + tnum(J, K) * 64;
+            double2* Ct = (double2*)(sG + tnum(I, K) * 64 + tix(li, 2 * lk));
+            double2 v = *Ct;
+            mma884(v.x, v.y, -Ra[tix(lk, li)], Rb[tix(lk, li)]);
+            mma884(v.x, v.y, -Ra[tix(lk + 4, li)], Rb[tix(lk + 4, li)]);
+            *Ct = v;
+        }
+        __syncthreads();
+    }
+}
+
+// Sum of the partial Gram matrices (CTA t: tile t) and, in the last CTA to
+// finish, the decision of the stage.
+template <int CB>
+__global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, int mode, Plan pl, GQ g, double* ws,
+                                                     int stage, long long* qstat) {
+    PTT_PDL_ENTRY();
+    using C = Cfg<CB>;
+    extern __shared__ __align__(128) double gsm[];
+    __shared__ int s_state, s_ticket, s_flags, s_nd;
+    __shared__ double s_red[NT];
+    __shared__ double s_d[CB], s_di[CB], s_an[CB], s_rinv[CB];
+    __shared__ unsigned long long s_tm[CB];
+    __shared__ unsigned char s_alive[CB / 8];
+    State* st = (State*)g.rec;
+    const View A = make_view(D, k, mode, false);
+    const int m = A.m, c = A.c;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, li = lane >> 2, lk = lane & 3;
+    if (stage == 0) {
+        if (!shape_ok(m, c, CB, g)) {  // uniform
+            if (blockIdx.x == 0 && tid == 0) {
+                st->state = FALLBACK;
+                st->nst = 0;
+                st->m = m;
+                st->c = c;
+                if (qstat) atomicAdd((unsigned long long*)(qstat + 1), 1ull);
+            }
+            return;
+        }
+        if (pl.work && blockIdx.x == 0 && tid == 0) atomicAdd(pl.work, 16.0 * (double)m * (double)c);
+    } else {
+        if (tid == 0) s_state = ldcg(&st->state);
+        __syncthreads();
+        if (s_state != RUN) return;
+    }
+    const int nbc = (c + 7) >> 3, nt = nbc * (nbc + 1) / 2;
+    if ((int)blockIdx.x >= nt) return;
+    {
+        // tile blockIdx.x: four quarters of the partials, each in CTA order
+        // (eight loads in flight), the quarters in order
+        const int rt = rows_taken(m, g.nb), np = (m + rt - 1) / rt;
+        const int q = tid >> 6, p0 = np * q / 4, p1 = np * (q + 1) / 4;
+        const double* P = g.part + (long long)blockIdx.x * 64 + (tid & 63);
+        double a = 0.0;
+        int p = p0;
+        for (; p + 8 <= p1; p += 8) {
+            double v[8];
+#pragma unroll
+            for (int t = 0; t < 8; t++) v[t] = ldcg(P + (long long)(p + t) * C::UP);
+#pragma unroll
+            for (int t = 0; t < 8; t++) a += v[t];
+        }
+        for (; p < p1; p++) a += ldcg(P + (long long)p * C::UP);
+        s_red[tid] = a;
+        __syncthreads();
+        if (tid < 64)
+            g.rec[C::O_G + blockIdx.x * 64 + tid] = ((s_red[tid] + s_red[64 + tid]) + s_red[128 + tid]) + s_red[192 + tid];
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_ticket = atomicAdd(g.cnt, 1);
+    __syncthreads();
+    if (s_ticket != nt - 1) return;
+    // ---- the deciding CTA ----------------------------------------------------
+    if (tid == 0) {
+        *g.cnt = 0;
+        s_flags = 0;
+        s_nd = 0;
+    }
+    __threadfence();
+    double* sG = gsm;            // Gram matrix, then the factor
+    double* sT = gsm + C::UP;    // accumulated R of the factors applied so far
+    {
+        const unsigned g0 = (unsigned)__cvta_generic_to_shared(sG);
+        const double* G = g.rec + C::O_G;
+        const double* T = g.rec + C::O_T;
+        for (int e = 2 * tid; e < nt * 64; e += 2 * NT) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(g0 + 8u * e), "l"(G + e) : "memory");
+            if (stage > 0)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(g0 + 8u * (C::UP + e)), "l"(T + e)
+                             : "memory");
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
     }
     __syncthreads();
-    // trace, max |G - I|, NaN, zero column
-    double tr = 0.0, emax = 0.0;
-    int fl = 0;  // bit 0: NaN, bit 1: a zero diagonal entry (an exactly zero column)
-    for (int u = tid; u < c * c; u += NT) {
-        const int i = u / c, j = u - (u / c) * c;
-        const double v = sG[i * GP + j] - (i == j ? 1.0 : 0.0);
-        if (!(v == v)) fl |= 1;
-        emax = fmax(emax, fabs(v));
-        if (i == j) {
-            tr += sG[i * GP + j];
-            if (sG[i * GP + j] == 0.0) fl |= 2;
+    if (tid < CB) {
+        const int j = tid;
+        const double gjj = j < c ? sG[tnum(j >> 3, j >> 3) * 64 + tix(j & 7, j & 7)] : 0.0;
+        const double dj = gjj > 0.0 ? sqrt(gjj) : 0.0;
+        bool on = gjj > 0.0;
+        if (stage > 0) {
+            on = on && dj * ldcg(g.rec + C::O_TM + j) > DROP * sqrt((double)c);
+            s_an[j] = ldcg(g.rec + C::O_AN + j);
+        } else {
+            s_an[j] = on ? 1.0 / dj : 0.0;
+            g.rec[C::O_AN + j] = s_an[j];
         }
+        s_d[j] = on ? dj : 0.0;
+        s_di[j] = on ? 1.0 / dj : 0.0;
+        s_tm[j] = 0ull;
+        if (j < c && !(gjj >= 0.0 && gjj < 1e300)) atomicOr(&s_flags, 1);      // NaN, Inf or near overflow
+        if (j < c && gjj != 0.0 && gjj < SMALL) atomicOr(&s_flags, 1);
+        const unsigned bits = __ballot_sync(0xffffffffu, on);
+        if ((lane & 7) == 0) s_alive[j >> 3] = (unsigned char)((bits >> lane) & 0xffu);
+        if (lane == 0 && j < c) atomicAdd(&s_nd, __popc(bits));
+    }
+    __syncthreads();
+    const int nlive = s_nd;
+    double emax = 0.0;
+    for (int t = warp; t < nt; t += NT / 32) {
+        int I, J;
+        tile_of(t, &I, &J);
+        const double2 v = *(const double2*)(sG + t * 64 + tix(li, 2 * lk));
+        const int i = 8 * I + li, j = 8 * J + 2 * lk;
+        const bool oi = (s_alive[I] >> li) & 1, o0 = (s_alive[J] >> (2 * lk)) & 1, o1 = (s_alive[J] >> (2 * lk + 1)) & 1;
+        const double e0 = (oi && o0) ? fabs(v.x - (i == j ? 1.0 : 0.0)) : 0.0;
+        const double e1 = (oi && o1) ? fabs(v.y - (i == j + 1 ? 1.0 : 0.0)) : 0.0;
+        if (!(v.x - v.x == 0.0) || !(v.y - v.y == 0.0)) atomicOr(&s_flags, 1);
+        emax = fmax(emax, fmax(e0, e1));
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        tr += __shfl_xor_sync(0xffffffffu, tr, o);
-        emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-        fl |= __shfl_xor_sync(0xffffffffu, fl, o);
-    }
-    if ((tid & 31) == 0) {
-        s_red[tid >> 5][0] = tr;
-        s_red[tid >> 5][1] = emax;
-        if (fl) atomicOr(&s_flags, fl);
-    }
+    for (int o = 16; o > 0; o >>= 1) emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+    if (lane == 0) s_red[warp] = emax;
     __syncthreads();
-    tr = 0.0;
-    emax = 0.0;
-    for (int w = 0; w < NT / 32; w++) {  // every thread, same order: same values
-        tr += s_red[w][0];
-        emax = fmax(emax, s_red[w][1]);
-    }
-    const bool nan = (s_flags & 1) || !(emax == emax);
-    const bool zcol = (s_flags & 2) != 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; w++) emax = fmax(emax, s_red[w]);
     int nst = (stage == 0) ? 0 : ldcg(&st->nst);
-    int nshift = (stage == 0) ? 0 : ldcg(&st->nshift);
     int dec;
-    if (nan || !(tr > 0.0) || !(tr < 1.0 / 0.0) || (stage == 0 && zcol)) {
+    if (s_flags || nlive == 0) {
         dec = FALLBACK;
     } else if (stage >= 1 && emax <= TAU) {
         dec = DONE;
-    } else if (stage >= 1 && emax <= FIRST) {
-        for (int e = tid; e < CB * RP; e += NT) {
-            const int j = e / RP, l = e - (e / RP) * RP;
-            double v = 0.0;
-            if (j < c && l < c) {
-                if (l > j)
-                    v = sG[j * GP + l];
-                else if (l == j)
-                    v = 1.0 + 0.5 * (sG[j * GP + j] - 1.0);
-            }
-            sFa[e] = v;
-        }
-        for (int j = tid; j < CB; j += NT) sFa[CB * RP + j] = j < c ? 1.0 / (1.0 + 0.5 * (sG[j * GP + j] - 1.0)) : 0.0;
-        dec = emax <= FIRST_DONE ? FINISH : RUN;
     } else if (stage == MAXST - 1) {
-        dec = FALLBACK;
+        dec = FALLBACK;  // no launch left to apply another factor
+    } else if (stage >= 1 && emax <= FIRST) {
+        dec = emax <= FIRST_DONE ? FINISH : RUN;
+        for (int t = warp; t < nt; t += NT / 32) {
+            int I, J;
+            tile_of(t, &I, &J);
+            double2* pv = (double2*)(sG + t * 64 + tix(li, 2 * lk));
+            const double2 v = *pv;
+            const int i = 8 * I + li, j = 8 * J + 2 * lk;
+            const bool oi = (s_alive[I] >> li) & 1, o0 = (s_alive[J] >> (2 * lk)) & 1,
+                       o1 = (s_alive[J] >> (2 * lk + 1)) & 1;
+            double2 w;
+            w.x = !(oi && o0) || j < i ? 0.0 : (i == j ? 1.0 + 0.5 * (v.x - 1.0) : v.x);
+            w.y = !(oi && o1) || j + 1 < i ? 0.0 : (i == j + 1 ? 1.0 + 0.5 * (v.y - 1.0) : v.y);
+            *pv = w;
+            if (i == j) s_rinv[i] = w.x != 0.0 ? 1.0 / w.x : 0.0;
+            if (i == j + 1) s_rinv[i] = w.y != 0.0 ? 1.0 / w.y : 0.0;
+        }
     } else {
-        // plain (warp 0) and shifted (warp 1) Cholesky at once; the plain one
-        // is kept when its pivots span less than 12 decades
-        if (tid < 64) {
-            const int w = tid >> 5;
-            const double sigma = w ? 11.0 * ((double)m * c + (double)c * (c + 1)) * U * tr : 0.0;
-            double ratio;
-            double* F = w ? sFb : sFa;
-            const bool ok = warp_chol64(sG, c, sigma, F, F + CB * RP, sRow + 32 * w, &ratio);
-            if ((tid & 31) == 0) {
-                s_cok[w] = ok;
-                s_cratio[w] = ratio;
-            }
+        dec = RUN;
+        for (int t = warp; t < nt; t += NT / 32) {  // H = D^-1 G D^-1, zero for the dropped columns
+            int I, J;
+            tile_of(t, &I, &J);
+            double2* pv = (double2*)(sG + t * 64 + tix(li, 2 * lk));
+            const double di = s_di[8 * I + li];
+            pv->x = pv->x * di * s_di[8 * J + 2 * lk];
+            pv->y = pv->y * di * s_di[8 * J + 2 * lk + 1];
         }
-        dec = CHOL;
-    }
-    __syncthreads();
-    bool use_b = false;
-    if (dec == CHOL) {
-        if (s_cok[0] && s_cratio[0] >= 1e-12) {
-            dec = RUN;
-        } else if (s_cok[1]) {
-            dec = RUN;
-            use_b = true;
-            nshift++;
-        } else {
-            dec = FALLBACK;
+        __syncthreads();
+        chol_tiles<CB>(sG, nbc, c, s_alive, s_rinv);
+        for (int t = warp; t < nt; t += NT / 32) {  // R = chol(H) D
+            int I, J;
+            tile_of(t, &I, &J);
+            double2* pv = (double2*)(sG + t * 64 + tix(li, 2 * lk));
+            pv->x *= s_d[8 * J + 2 * lk];
+            pv->y *= s_d[8 * J + 2 * lk + 1];
         }
-    }
-    if (stage == MAXST - 1 && (dec == RUN || dec == FINISH)) dec = FALLBACK;  // no launch left to apply it
-    double* sF = use_b ? sFb : sFa;  // the factor applied next
-    double* sT = use_b ? sFa : sFb;  // the accumulated R of the factors applied so far
-    {
-        constexpr int TPT = (CB * GP + NT - 1) / NT;
-        double tv[TPT];
-#pragma unroll
-        for (int k = 0; k < TPT; k++) {
-            const int e = tid + k * NT;
-            const int i = e / GP, j = e - (e / GP) * GP;
-            tv[k] = (e >= CB * GP) ? 0.0
-                    : (stage == 0) ? ((i == j && i < c) ? 1.0 : 0.0)
-                    : ((j < CB) ? ldcg(g.rec + O_T + i * CB + j) : 0.0);
-        }
-#pragma unroll
-        for (int k = 0; k < TPT; k++)
-            if (tid + k * NT < CB * GP) sT[tid + k * NT] = tv[k];
+        if (tid < 8 * nbc) s_rinv[tid] *= s_di[tid];
     }
     __syncthreads();
     if (dec == RUN || dec == FINISH) {
-        // new accumulated R = F T (both upper triangular) into sG: each thread
-        // a 4 x 4 block; at stage 0 T = I and it is F itself
-        {
-            const int bi = (tid >> 4) * 4, bj = (tid & 15) * 4;
-            double acc[4][4];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
+        // the factor for the next launch, and the accumulated R = F T in tiles
+        double* F = g.rec + C::O_FAC;
+        for (int e = tid; e < nt * 32; e += NT) ((double2*)F)[e] = ((const double2*)sG)[e];
+        if (tid < CB) F[C::UP + tid] = tid < 8 * nbc ? s_rinv[tid] : 0.0;
+        double* T = g.rec + C::O_T;
+        double* Rs = ws + pl.o_Rn;  // root slot (row-major CT x CT)
+        for (int t = warp; t < nt; t += NT / 32) {
+            int I, J;
+            tile_of(t, &I, &J);
+            double2 v;
             if (stage == 0) {
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) acc[a][b] = sF[(bi + a) * RP + bj + b];
-            } else if (bj + 3 >= bi) {
-                for (int t = bi; t <= bj + 3 && t < CB; t++) {
-                    double fa[4], tb[4];
-#pragma unroll
-                    for (int a = 0; a < 4; a++) fa[a] = sF[(bi + a) * RP + t];
-#pragma unroll
-                    for (int b = 0; b < 4; b++) tb[b] = sT[t * GP + bj + b];
-#pragma unroll
-                    for (int a = 0; a < 4; a++)
-#pragma unroll
-                        for (int b = 0; b < 4; b++) acc[a][b] = fma(fa[a], tb[b], acc[a][b]);
+                v = *(const double2*)(sG + t * 64 + tix(li, 2 * lk));
+            } else {
+                double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+                for (int K = I; K <= J; K++) {
+                    const double* Fk = sG + tnum(I, K) * 64;
+                    const double* Tk = sT + tnum(K, J) * 64;
+                    mma884(a0, a1, Fk[tix(li, lk)], Tk[tix(lk, li)]);
+                    mma884(b0, b1, Fk[tix(li, lk + 4)], Tk[tix(lk + 4, li)]);
                 }
+                v = make_double2(a0 + b0, a1 + b1);
             }
-            // F and T are upper triangular and zero beyond c: the products
-            // outside the upper c x c triangle are exact zeros
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) sG[(bi + a) * GP + bj + b] = (bj + b >= bi + a) ? acc[a][b] : 0.0;
+            *(double2*)(T + t * 64 + tix(li, 2 * lk)) = v;
+            const int i = 8 * I + li, j = 8 * J + 2 * lk;
+            if (dec == FINISH) {
+                Rs[(long long)i * CB + j] = j >= i ? v.x : 0.0;
+                Rs[(long long)i * CB + j + 1] = j + 1 >= i ? v.y : 0.0;
+            }
+            const double w = fmax(fabs(v.x) * s_an[j], fabs(v.y) * s_an[j + 1]);
+            atomicMax(&s_tm[i], (unsigned long long)__double_as_longlong(w));
         }
         __syncthreads();
-        double* F = g.rec + O_FAC;
-        for (int e = tid; e < CB * RP + CB; e += NT) F[e] = sF[e];
-        double* T = g.rec + O_T;
-        for (int e = tid; e < CB * CB; e += NT) T[e] = sG[(e / CB) * GP + (e % CB)];
+        if (tid < CB) g.rec[C::O_TM + tid] = __longlong_as_double((long long)s_tm[tid]);
         nst++;
+    } else if (dec == DONE) {
+        double* Rs = ws + pl.o_Rn;
+        for (int t = warp; t < nt; t += NT / 32) {
+            int I, J;
+            tile_of(t, &I, &J);
+            const double2 v = *(const double2*)(sT + t * 64 + tix(li, 2 * lk));
+            const int i = 8 * I + li, j = 8 * J + 2 * lk;
+            const bool oi = (s_alive[I] >> li) & 1;  // a column dropped in this stage takes its row of R with it
+            Rs[(long long)i * CB + j] = oi && j >= i ? v.x : 0.0;
+            Rs[(long long)i * CB + j + 1] = oi && j + 1 >= i ? v.y : 0.0;
+        }
     }
-    const double* Rfin = (dec == DONE) ? sT : sG;  // FINISH: the new accumulated R
-    if (dec == DONE || dec == FINISH) {
-        double* Rs = ws + pl.o_Rn;  // root slot (row-major CT x CT)
-        for (int e = tid; e < pl.CT * pl.CT; e += NT) {
-            const int i = e / pl.CT, j = e - (e / pl.CT) * pl.CT;
-            Rs[e] = (i < c && j < c && j >= i) ? Rfin[i * GP + j] : 0.0;
+    if (finished(dec)) {
+        double* Rs = ws + pl.o_Rn;  // zeros: the tiles below the diagonal and the columns beyond the blocks
+        for (int e = tid; e < CB * CB; e += NT) {
+            const int i = e / CB, j = e - (e / CB) * CB;
+            if ((j >> 3) < (i >> 3) || j >= 8 * nbc || i >= 8 * nbc) Rs[e] = 0.0;
         }
         if (tid == 0) {
             Info* info = pl.info;
@@ -718,7 +785,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int
         if (dec == FALLBACK && qstat) atomicAdd((unsigned long long*)(qstat + 1), 1ull);
         st->fin = stage + 1;
         st->nst = nst;
-        st->nshift = nshift;
+        st->ndrop = c - nlive;
         st->m = m;
         st->c = c;
         __threadfence();
@@ -726,57 +793,35 @@ __global__ void __launch_bounds__(NT, 1) k_gq_stage(const DevDesc* D, int k, int
     }
 }
 
-// alt[k][row * rank + col] = (Q V_r)(row, col) for a RIGHT_T bond this path
-// finished: Q rows in g.qscr (row-major, pitch c), V_r at the root B slot
-// (row-major CT x KC).  One block per WROWS rows; the writes of a block are
-// one contiguous range.
-constexpr int WROWS = 16;
+// alt[k] = Q V_r (m x rank, row-major) for a RIGHT_T bond this path finished:
+// Q rows in g.qscr (row-major, pitch c), V_r at the root B slot (row-major CT
+// x KC).  64 x 64 tiles on the FP64 tensor cores.
 __global__ void __launch_bounds__(NT) k_gq_write(const DevDesc* D, int k, Plan pl, GQ g, double* ws) {
     PTT_PDL_ENTRY();
-    __shared__ double sB[CB * (CB + 1)];
-    __shared__ double sQ[WROWS * (CB + 1)];
     if (!finished(ldcg((const int*)g.rec))) return;
     const Info* info = pl.info;
     if (info->status) return;
     const int m = info->m, c = info->c, rank = info->rank;
-    const int tid = threadIdx.x;
-    const double* Bn = ws + pl.o_Bn;
-    for (int e = tid; e < CB * CB; e += NT) {
-        const int t = e / CB, l = e - (e / CB) * CB;
-        sB[t * (CB + 1) + l] = (t < c && l < rank) ? Bn[(long long)t * pl.KC + l] : 0.0;
-    }
-    double* out = D->alt[k];
-    for (int r0 = blockIdx.x * WROWS; r0 < m; r0 += gridDim.x * WROWS) {
-        const int h = (m - r0) < WROWS ? (m - r0) : WROWS;
-        __syncthreads();
-        for (int e = tid; e < WROWS * CB; e += NT) {
-            const int row = e / CB, t = e - (e / CB) * CB;
-            sQ[row * (CB + 1) + t] = (row < h && t < c) ? g.qscr[(long long)(r0 + row) * c + t] : 0.0;
-        }
-        __syncthreads();
-        for (int e = tid; e < h * rank; e += NT) {
-            const int row = e / rank, col = e - (e / rank) * rank;
-            double y0 = 0.0, y1 = 0.0;
-#pragma unroll 8
-            for (int t = 0; t < CB; t += 2) {
-                y0 = fma(sQ[row * (CB + 1) + t], sB[t * (CB + 1) + col], y0);
-                y1 = fma(sQ[row * (CB + 1) + t + 1], sB[(t + 1) * (CB + 1) + col], y1);
-            }
-            out[(long long)r0 * rank + e] = y0 + y1;
-        }
-    }
+    if ((int)blockIdx.y * GT >= rank) return;
+    GV Q{g.qscr, c, 1};
+    GV V{ws + pl.o_Bn, pl.KC, 1};
+    for (int t = blockIdx.x; t * GT < m; t += gridDim.x)
+        gemm_tile(Q, V, D->alt[k], rank, 1, m, rank, c, t, blockIdx.y);
 }
 
-// G = A^T A of a column-major m x c matrix (c <= CB, leading dimension lda),
+// G = A^T A of a column-major m x c matrix (c <= 64, leading dimension lda),
 // the Gram matrix of an unfolding on its own (ptt_gram): CTA b forms the
 // partial of rows [b RPB_MAX, (b + 1) RPB_MAX) -- on the FP64 tensor cores,
 // or by the Ozaki split on tcgen05 when OZ -- the last-arriving CTA of each
 // group of GROUP sums the group's partials in CTA order, the last-arriving
 // group sums the groups in order and writes G (c x c, column-major, both
 // triangles).  Deterministic; no CTA waits for another.
+constexpr size_t SM_GRAM = sizeof(double) * ((size_t)Cfg<64>::RPB_MAX * Cfg<64>::XP + Cfg<64>::UP);
 template <bool OZ>
 __global__ void __launch_bounds__(NT, 1) k_gram(const double* A, long long m, int c, long long lda, double* part,
                                                 double* gpart, int* cnt, double* G) {
+    using C = Cfg<64>;
+    constexpr int UP = C::UP, XP = C::XP, RPB_MAX = C::RPB_MAX;
     extern __shared__ __align__(128) double gsm[];
     double* Xs = gsm;
     __shared__ int s_ticket;
@@ -793,7 +838,7 @@ __global__ void __launch_bounds__(NT, 1) k_gram(const double* A, long long m, in
     if constexpr (OZ)
         oz::gram_partial<NT>(Xs, XP, h, c, (unsigned char*)(Xs + RPB_MAX * XP), Xs, part + (long long)b * UP);
     else
-        gram_fp64(Xs, h, part + (long long)b * UP);
+        gram_fp64<64>(Xs, h, 8, Xs + RPB_MAX * XP, part + (long long)b * UP);
     const int ngroups = (nb + GROUP - 1) / GROUP, grp = b / GROUP;
     const int gsize = (nb - grp * GROUP) < GROUP ? (nb - grp * GROUP) : GROUP;
     __threadfence();
@@ -815,13 +860,14 @@ __global__ void __launch_bounds__(NT, 1) k_gram(const double* A, long long m, in
     if (s_ticket != ngroups - 1) return;
     if (tid == 0) cnt[ngroups] = 0;
     __threadfence();
-    for (int u = tid; u < UP; u += NT) {
-        double a = 0.0;
-        for (int t = 0; t < ngroups; t++) a += ldcg(gpart + (long long)t * UP + u);
-        int ti = 0, tj = 0;
-        cq::upper_tile(u >> 6, &ti, &tj);
-        const int i = ti * TS + ((u >> 3) & 7), j = tj * TS + (u & 7);
-        if (i < c && j < c && (ti < tj || i <= j)) {  // a diagonal tile's upper half
+    for (int e = tid; e < UP; e += NT) {
+        int ti, tj;
+        tile_of(e >> 6, &ti, &tj);
+        const int i = ti * 8 + ((e >> 3) & 7), j = tj * 8 + (e & 7);
+        if (i < c && j < c && i <= j) {
+            const int u = (e & ~63) + tix((e >> 3) & 7, e & 7);
+            double a = 0.0;
+            for (int t = 0; t < ngroups; t++) a += ldcg(gpart + (long long)t * UP + u);
             G[i + (long long)j * c] = a;
             G[j + (long long)i * c] = a;
         }

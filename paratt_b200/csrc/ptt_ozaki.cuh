@@ -334,8 +334,8 @@ __device__ void combine(const double* acc, bool ok, const double* sa, const doub
 }
 
 // Partial Gram matrix of X (h x c rows of pitch xp, zero beyond c and h up to
-// a multiple of 8) written to P as the 36 upper 8 x 8 tiles (tile q at P + 64
-// q, row-major).  All NT = 256 threads; `sl` = SMEM bytes of shared memory,
+// a multiple of 8) written to P as the 36 upper 8 x 8 tiles in the order and
+// layout of the grid Cholesky QR (ptt_gridqr.cuh: tnum, tix).  All NT = 256 threads; `sl` = SMEM bytes of shared memory,
 // 16-byte aligned; `xtmp` = 64 x 65 doubles of shared memory, may alias X.
 // A non-finite element, a misaligned buffer or a wait that runs out gives a
 // NaN partial.
@@ -356,13 +356,12 @@ __device__ void gram_partial(const double* X, int xp, int h, int c, unsigned cha
     const bool ok = !nonfinite && products<NT, KMAX>(&tm, sl, sl, h > 0 ? (h + 15) / 16 : 1, acc, 0u);
     tm_close(&tm);
     combine<NT>(acc, ok, s_sc, s_sc, xtmp);
-    for (int u = tid; u < 36 * 64; u += NT) {  // tile order (coalesced)
-        int q = u >> 6, ti = 0;
-        while (q >= 8 - ti) {
-            q -= 8 - ti;
-            ti++;
-        }
-        P[u] = xtmp[(ti * 8 + ((u >> 3) & 7)) * 65 + (ti + q) * 8 + (u & 7)];
+    for (int u = tid; u < 36 * 64; u += NT) {  // tile order (coalesced): tile (I, J) is number J (J + 1) / 2 + I
+        const int q = u >> 6, i = (u >> 3) & 7;
+        int tj = 0;
+        while ((tj + 1) * (tj + 2) / 2 <= q) tj++;
+        const int ti = q - tj * (tj + 1) / 2, j = (u & 7) ^ ((i & 2) << 1);  // swizzled columns (gq::tix)
+        P[u] = xtmp[(ti * 8 + i) * 65 + tj * 8 + j];
     }
 }
 

@@ -1266,9 +1266,15 @@ static int set_attrs() {
                                       (int)ring_smem<CT <= 64 ? CT : 64>()));
     PTT_CUDA(cudaFuncSetAttribute(k_svd_replay, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)replay_smem<128>()));
-    PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_stage<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gq::SMEM));
-    PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_stage<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)gq::SMEM_OZ));
+    if constexpr (CT >= 64) {
+        PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_rows<CT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)gq::Cfg<CT>::SM_ROWS));
+        PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_decide<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)gq::Cfg<CT>::SM_DEC));
+    }
+    if constexpr (CT == 64)
+        PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_rows<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)gq::SM_ROWS_OZ));
     PTT_CUDA(cudaFuncSetAttribute(k_gemm_rx_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::SMEM_GEMM));
     PTT_CUDA(cudaFuncSetAttribute(k_gemm_xm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::SMEM_GEMM));
     done.fetch_or(bit);
@@ -1281,18 +1287,24 @@ static int set_attrs() {
 template <int CT>
 static int launch_factor(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, double* ws, gq::GQ* g, long long mcap) {
     ptt_time_begin(c, PTT_TIME_TSQR);
-    if (g) {
-        g->rpb = gq::rows_per_cta(mcap, c->nsm);
-        const int nb = gq::ctas(mcap, g->rpb);
-        pl.gqstate = (const int*)g->rec;
-        for (int s = 0; s < gq::MAXST; s++) {
-            if (c->ozaki)
-                PTT_CUDA(ptt_launch(c, gq::k_gq_stage<true>, dim3(nb), dim3(gq::NT), gq::SMEM_OZ,
+    if constexpr (CT >= 64) {
+        if (g) {
+            using C = gq::Cfg<CT>;
+            g->rpb = gq::rows_per_cta(mcap, c->nsm, C::RPB_MAX);
+            g->nb = gq::ctas(mcap, g->rpb);
+            pl.gqstate = (const int*)g->rec;
+            for (int s = 0; s < gq::MAXST; s++) {
+                if (CT == 64 && c->ozaki)
+                    PTT_CUDA(ptt_launch(c, gq::k_gq_rows<64, true>, dim3(g->nb), dim3(gq::NT), gq::SM_ROWS_OZ,
+                                        (const DevDesc*)x->dd, k, mode, pl, *g, s));
+                else
+                    PTT_CUDA(ptt_launch(c, gq::k_gq_rows<CT, false>, dim3(g->nb), dim3(gq::NT), C::SM_ROWS,
+                                        (const DevDesc*)x->dd, k, mode, pl, *g, s));
+                PTT_LAUNCHED(c);
+                PTT_CUDA(ptt_launch(c, gq::k_gq_decide<CT>, dim3(C::NTI), dim3(gq::NT), C::SM_DEC,
                                     (const DevDesc*)x->dd, k, mode, pl, *g, ws, s, c->d_qrstat));
-            else
-                PTT_CUDA(ptt_launch(c, gq::k_gq_stage<false>, dim3(nb), dim3(gq::NT), gq::SMEM,
-                                    (const DevDesc*)x->dd, k, mode, pl, *g, ws, s, c->d_qrstat));
-            PTT_LAUNCHED(c);
+                PTT_LAUNCHED(c);
+            }
         }
     }
     PTT_CUDA(ptt_launch(c, k_tsqr_factor<CT>, dim3(pl.P), dim3(NT), factor_smem<CT>(), (const DevDesc*)x->dd, k, mode,
@@ -1323,7 +1335,7 @@ static int launch_apply(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, double
 // 4 = QR of the single core `only` (left unfolding; core <- Q, r_{only+1} <- q).
 // rk[k]: upper bound of rank k for the whole call (the capacity, or the
 // actual ranks when they were read back; ranks only shrink while rounding).
-// At CT = 64 every factorisation first runs the grid Cholesky QR
+// At CT = 64 and 128 every factorisation first runs the grid Cholesky QR
 // (ptt_gridqr.cuh) unless the context is set to Householder only.
 template <int CT>
 static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, int phases, int only) {
@@ -1331,7 +1343,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     const int d = x->d;
     int rc = set_attrs<CT>();
     if (rc) return rc;
-    const bool use_gq = (CT == gq::CB) && !c->no_cholqr;
+    const bool use_gq = CT >= 64 && !c->no_cholqr;
     // plan: largest leaf count over all bonds decides the workspace
     const int KC = (CT + KG - 1) / KG * KG;
     int PMAX = 1, KLMAX = 1, NBMAX = 1;
@@ -1344,7 +1356,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         if (t.P > PMAX) PMAX = t.P;
         if (t.KL > KLMAX) KLMAX = t.KL;
         for (long long mm : {ml, mr}) {
-            const int nb = gq::ctas(mm, gq::rows_per_cta(mm, c->nsm));
+            const int nb = gq::ctas(mm, gq::rows_per_cta(mm, c->nsm, gq::Cfg<CT >= 64 ? CT : 64>::RPB_MAX));
             NBMAX = nb > NBMAX ? nb : NBMAX;
         }
         MQMAX = mr > MQMAX ? mr : MQMAX;
@@ -1354,9 +1366,10 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     base.NH = (CT + H - 1) / H;
     long long total = carve(&base, PMAX, KLMAX);
     // grid Cholesky QR: record, partial Gram matrices, Q rows of RIGHT_T bonds
-    const int NGMAX = (NBMAX + gq::GROUP - 1) / gq::GROUP;
+    using GC = gq::Cfg<CT >= 64 ? CT : 64>;
+    const long long gq_rec = (GC::REC + 31) / 32 * 32;
     long long o_gq = (total + 31) / 32 * 32, gq_len = 0;
-    if (use_gq) gq_len = gq::REC + (long long)(NBMAX + NGMAX) * gq::UP + MQMAX * gq::CB + 64;
+    if (use_gq) gq_len = gq_rec + (long long)NBMAX * GC::UP + MQMAX * CT;
     // two slots of the whole region (bond parity): the truncation sweep runs
     // the tail of bond i (V replay, Q V_r, swap of core i) on the side stream
     // while bond i - 1 is factored in the other slot
@@ -1364,7 +1377,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     size_t bytes = (size_t)(2 * SLOT) * sizeof(double) + 256;
     if ((rc = ptt_ws_reserve(c, bytes))) return rc;
     const size_t cnt_tree = (size_t)PMAX * 4 + 64;
-    if ((rc = ptt_counters_reserve(c, cnt_tree + NGMAX + 2))) return rc;
+    if ((rc = ptt_counters_reserve(c, cnt_tree + 1))) return rc;
     double* const ws0 = (double*)c->ws;
     // ints live after the doubles: qn [2P-1], pass [P], Info
     // Tree counters live alone in ctx->d_counters (zero between launches,
@@ -1373,9 +1386,8 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     gq::GQ gqs[2] = {};
     for (int sl = 0; sl < 2 && use_gq; sl++) {
         gqs[sl].rec = wss[sl] + o_gq;
-        gqs[sl].part = gqs[sl].rec + (gq::REC + 31) / 32 * 32;
-        gqs[sl].gpart = gqs[sl].part + (long long)NBMAX * gq::UP;
-        gqs[sl].qscr = gqs[sl].gpart + (long long)NGMAX * gq::UP;
+        gqs[sl].part = gqs[sl].rec + gq_rec;
+        gqs[sl].qscr = gqs[sl].part + (long long)NBMAX * GC::UP;
         gqs[sl].cnt = c->d_counters + cnt_tree;  // main stream only
     }
     double* ws = ws0;
@@ -1479,9 +1491,9 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             int r2 = launch_apply<CT>(c, x, i, RIGHT_T, pl, ws, &info->rank, CT);
             if (r2) return r2;
             if (g) {  // Q V_r for a bond the grid Cholesky QR finished
-                int gx = (int)((mcap + gq::WROWS - 1) / gq::WROWS);
-                gx = gx < 1 ? 1 : (gx > 2 * c->nsm ? 2 * c->nsm : gx);
-                PTT_CUDA(ptt_launch(c, gq::k_gq_write, dim3(gx), dim3(gq::NT), 0, dd, i, pl, *g, ws));
+                int gx = (int)((mcap + GT - 1) / GT);
+                gx = gx < 1 ? 1 : (gx > 4096 ? 4096 : gx);
+                PTT_CUDA(ptt_launch(c, gq::k_gq_write, dim3(gx, (CT + GT - 1) / GT), dim3(gq::NT), 0, dd, i, pl, *g, ws));
                 PTT_LAUNCHED(c);
             }
             return PTT_OK;
@@ -1902,25 +1914,25 @@ extern "C" int ptt_ctx_ozaki(ptt_ctx* c, int on) {
 // cores (the two Gram kernels of the grid Cholesky QR, ptt_gridqr.cuh and
 // ptt_ozaki.cuh).
 extern "C" int ptt_gram(ptt_ctx* c, const double* A, long long m, int cols, long long lda, double* G, int method) {
-    if (!c || !A || !G || m < 1 || cols < 1 || cols > gq::CB || lda < m || (method != 0 && method != 1))
+    if (!c || !A || !G || m < 1 || cols < 1 || cols > 64 || lda < m || (method != 0 && method != 1))
         return ptt_set_error(PTT_ERR_ARG, "ptt_gram: bad arguments");
-    const long long nbl = (m + gq::RPB_MAX - 1) / gq::RPB_MAX;
+    const long long nbl = (m + gq::Cfg<64>::RPB_MAX - 1) / gq::Cfg<64>::RPB_MAX;
     if (nbl > (1ll << 24)) return ptt_set_error(PTT_ERR_CAPACITY, "ptt_gram: %lld rows", m);
     cudaSetDevice(c->device);
     int rc;
     const int nb = (int)nbl, ng = (nb + gq::GROUP - 1) / gq::GROUP;
-    if ((rc = ptt_ws_reserve(c, sizeof(double) * (size_t)(nb + ng) * gq::UP + 256))) return rc;
+    if ((rc = ptt_ws_reserve(c, sizeof(double) * (size_t)(nb + ng) * gq::Cfg<64>::UP + 256))) return rc;
     if ((rc = ptt_counters_reserve(c, (size_t)ng + 1))) return rc;
     double* part = (double*)c->ws;
-    double* gpart = part + (long long)nb * gq::UP;
+    double* gpart = part + (long long)nb * gq::Cfg<64>::UP;
     if (method == 1) {
         PTT_CUDA(cudaFuncSetAttribute(gq::k_gram<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)gq::SMEM_OZ));
-        gq::k_gram<true><<<nb, gq::NT, gq::SMEM_OZ, c->stream>>>(A, m, cols, lda, part, gpart, c->d_counters, G);
+                                      (int)gq::SM_ROWS_OZ));
+        gq::k_gram<true><<<nb, gq::NT, gq::SM_ROWS_OZ, c->stream>>>(A, m, cols, lda, part, gpart, c->d_counters, G);
     } else {
         PTT_CUDA(cudaFuncSetAttribute(gq::k_gram<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(double) * gq::RPB_MAX * gq::XP)));
-        gq::k_gram<false><<<nb, gq::NT, sizeof(double) * gq::RPB_MAX * gq::XP, c->stream>>>(A, m, cols, lda, part,
+                                      (int)gq::SM_GRAM));
+        gq::k_gram<false><<<nb, gq::NT, gq::SM_GRAM, c->stream>>>(A, m, cols, lda, part,
                                                                                           gpart, c->d_counters, G);
     }
     PTT_LAUNCHED(c);
