@@ -26,21 +26,7 @@ using namespace tsqr;
 
 namespace {
 
-constexpr int MAXSW = 40;  // Jacobi sweep limit
-
 __device__ __forceinline__ unsigned group_mask8(int tid) { return 0xFFu << ((tid & 31) & ~7); }
-
-// the same for groups of LP lanes (LP = 2, 4, 8)
-template <int LP>
-__device__ __forceinline__ unsigned group_mask(int tid) {
-    return ((1u << LP) - 1u) << ((tid & 31) & ~(LP - 1));
-}
-template <int LP>
-__device__ __forceinline__ double gsum_g(double v, unsigned mask) {
-#pragma unroll
-    for (int o = LP / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-    return v;
-}
 
 __device__ __forceinline__ double gsum8(double v, unsigned mask) {
     v += __shfl_xor_sync(mask, v, 4);
@@ -254,649 +240,7 @@ __global__ void k_set_identity(Plan pl, double* ws) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// one-sided Jacobi SVD of L = R^T (c x q), R = root factor of the LQ.
-// Column pairs follow the circle (round-robin) order; rotations are recorded
-// so V can be rebuilt row-parallel by k_svd_replay.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int circle_col(int pos, int round, int qq) {
-    return pos == 0 ? 0 : 1 + (pos - 1 + round) % (qq - 1);
-}
-
-// Stationary-ring order, for G = qq / 2 a power of two.  Level l (block size
-// hb = G >> l groups, rounds [2G - 2hb, 2G - hb)): block b of hb consecutive
-// pairs owns columns [2 hb b, 2 hb (b + 1)); pair i of the block keeps column
-// 2 hb b + i and meets 2 hb b + hb + (i + s) mod hb at shift s, so the second
-// columns move one pair along a ring of hb pairs per round while the first
-// ones stay.  Between levels each block splits in two: the first half pairs
-// its first columns among themselves, the second half its second columns
-// (a swap of one column between pairs i and i + hb / 2).  Every pair of
-// columns meets once in 2G - 1 rounds.
-__device__ __forceinline__ void stat_cols(int i, int rd, int G, int* pc, int* qc) {
-    const int x = 2 * G - 1 - rd;  // in [hb, 2 hb - 1]
-    const int hb = 1 << (31 - __clz(x));
-    const int s = rd - (2 * G - 2 * hb);
-    const int b = i / hb, ii = i - b * hb;
-    *pc = 2 * hb * b + ii;
-    *qc = 2 * hb * b + hb + (ii + s) % hb;
-}
-
-// threads of the SVD block: 8 lanes for each of the (CT+2)/2 column pairs
-// of a round, rounded to a power of two (idle threads only slow the barriers)
-template <int CT>
-__host__ __device__ constexpr int svd_nt() {
-    return CT <= 32 ? 128 : (CT <= 64 ? 256 : 512);
-}
-
-// One-sided Jacobi on the columns of L (c rows, q columns).  Each column pair
-// is handled by LP lanes (rows p + LP v), NTH / LP pairs per pass: with the
-// default 8 lanes and svd_nt threads one circle-order round is a single pass
-// for q <= 128.  (A one-warp form, NTH = 32 and LP = 4, measured slower on
-// the benchmark's bonds with q <= 16: 43.6 us against ~40 us, the
-// rotation chain and not the block barrier being the cost.)  Column norms
-// are tracked through the rotations (a_p' = a_p - t a_pq ...) and recomputed
-// at the start of a sweep.
-template <int CT, int NTH = svd_nt<CT>(), int LP = 8>
-__global__ void __launch_bounds__(NTH) k_svd_jacobi(Plan pl, double* ws, double delta, int maxr, int bond,
-                                                    int* status) {
-    PTT_PDL_ENTRY();
-    constexpr int SVD_NT = NTH;
-    extern __shared__ double sm[];
-    constexpr int S = CT + 1;
-    constexpr int NG = CT / LP;
-    double* Lc = sm;                   // (CT+1) columns x S
-    __shared__ double s_nrm[CT + 2];
-    __shared__ double s_sig[CT + 2];
-    __shared__ int s_ord[CT + 2];
-    __shared__ int s_rot;
-    __shared__ double s_thr2;
-    const int tid = threadIdx.x;
-    const int grp = tid / LP, p = tid % LP;  // pair slots x LP lanes
-    const unsigned gm = group_mask<LP>(tid);
-    Info* info = pl.info;
-    if (info->status) return;
-    const int c = info->c, q = info->q;
-    const int qq = q + (q & 1);
-    const double* R = ws + pl.o_Rn;  // root factor, row-major CT x CT; L = R^T
-    constexpr int LPT = (CT * S + SVD_NT - 1) / SVD_NT;  // qq <= CT
-    if constexpr (LPT <= 16) {  // every element requested before the first is stored
-        double v[LPT];
-#pragma unroll
-        for (int u = 0; u < LPT; u++) {
-            const int e = tid + u * SVD_NT;
-            const int j = e / S, t = e - (e / S) * S;
-            v[u] = (e < qq * S && j < q && t < c) ? R[(long long)j * CT + t] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < LPT; u++) {
-            const int e = tid + u * SVD_NT;
-            if (e < qq * S) Lc[e] = v[u];
-        }
-    } else {
-        for (int e = tid; e < qq * S; e += SVD_NT) {
-            const int j = e / S, t = e - (e / S) * S;
-            Lc[e] = (j < q && t < c) ? R[(long long)j * CT + t] : 0.0;
-        }
-    }
-    __syncthreads();
-    double2* rot = (double2*)(ws + pl.o_rot);
-    const int npair = (CT + 2) / 2;
-    const double tol = (double)(c < 16 ? 16 : c) * 2.220446049250313e-16;
-    const double tol2 = tol * tol;  // |ga| > tol sqrt(al be), compared in squares
-    int sweeps = 0;
-    bool conv = (qq < 2);
-    for (int sw = 0; sw < MAXSW && !conv; sw++) {
-        // exact column norms at the start of every sweep
-        for (int j = tid / LP; j < qq; j += SVD_NT / LP) {
-            double s2 = 0.0;
-#pragma unroll
-            for (int v = 0; v < NG; v++) {
-                const double x = Lc[j * S + p + LP * v];
-                s2 += x * x;
-            }
-            s2 = gsum_g<LP>(s2, gm);
-            if (p == 0) s_nrm[j] = s2;
-        }
-        if (tid == 0) s_rot = 0;
-        __syncthreads();
-        // Columns below the numerical-rank threshold (sqrt(q) eps_LAPACK times
-        // the largest column norm) are rounding noise: rotating noise against
-        // noise is a random walk that never meets the relative criterion, and
-        // their values are discarded by the rank rule anyway, so pairs with
-        // such a column are left alone.
-        if (tid == 0) {
-            double mx = 0.0;
-            for (int j = 0; j < qq; j++) mx = fmax(mx, s_nrm[j]);
-            s_thr2 = (double)q * 1.232595164407831e-32 * mx;  // (sqrt(q) * 2^-53)^2 * max |a_j|^2
-        }
-        __syncthreads();
-        const double thr2 = s_thr2;
-        int myrot = 0;
-        for (int rd = 0; rd < qq - 1; rd++) {
-            for (int i = grp; i < qq / 2; i += SVD_NT / LP) {
-                const int pc = circle_col(i, rd, qq), qc = circle_col(qq - 1 - i, rd, qq);
-                double* ap = Lc + pc * S;
-                double* aq = Lc + qc * S;
-                double xa[NG], xb[NG];
-                double g0 = 0.0, g1 = 0.0;
-#pragma unroll
-                for (int v = 0; v < NG; v++) {
-                    xa[v] = ap[p + LP * v];
-                    xb[v] = aq[p + LP * v];
-                }
-#pragma unroll
-                for (int v = 0; v < NG; v += 2) {
-                    g0 = fma(xa[v], xb[v], g0);
-                    g1 = fma(xa[v + 1], xb[v + 1], g1);
-                }
-                const double ga = gsum_g<LP>(g0 + g1, gm);
-                const double al = s_nrm[pc], be = s_nrm[qc];
-                double cs = 1.0, sn = 0.0;
-                if (ga != 0.0 && al > thr2 && be > thr2 && ga * ga > tol2 * (al * be)) {
-                    // the smaller rotation of the pair: with dd = be - al, g2 = 2 ga,
-                    // cos 2theta = |dd| / r, sin 2theta = sign(dd) g2 / r,
-                    // r = sqrt(dd^2 + g2^2); then cos theta = sqrt((1 + cos 2theta) / 2),
-                    // sin theta = sin 2theta / (2 cos theta), t = tan theta -- two
-                    // reciprocal square roots on the chain, no square root or division
-                    const double dd = be - al, g2 = 2.0 * ga;
-                    const double ri = rsqrt(fma(dd, dd, g2 * g2));
-                    const double hc = fma(0.5 * fabs(dd), ri, 0.5);  // (1 + cos 2theta) / 2, in [1/2, 1]
-                    const double ic = rsqrt(hc);                      // 1 / cos theta
-                    cs = hc * ic;
-                    sn = 0.5 * copysign(1.0, dd) * g2 * ri * ic;
-                    const double t = sn * ic;
-#pragma unroll
-                    for (int v = 0; v < NG; v++) {
-                        ap[p + LP * v] = cs * xa[v] - sn * xb[v];
-                        aq[p + LP * v] = sn * xa[v] + cs * xb[v];
-                    }
-                    if (p == 0) {
-                        s_nrm[pc] = al - t * ga;
-                        s_nrm[qc] = be + t * ga;
-                    }
-                    // bit 1: a rotation of a pair whose cosine exceeded 1e-8
-                    myrot |= (ga * ga > 1e-16 * (al * be)) ? 3 : 1;
-                }
-                if (p == 0) rot[((long long)sw * (CT + 1) + rd) * npair + i] = make_double2(cs, sn);
-            }
-            __syncthreads();
-        }
-        if (myrot) atomicOr(&s_rot, myrot);
-        __syncthreads();
-        if (s_rot == 0) {
-            conv = true;
-        } else {
-            sweeps = sw + 1;
-            // cyclic Jacobi converges quadratically at the end: after a sweep
-            // whose cosines all stayed below 1e-8 the next one would only
-            // meet cosines ~1e-16, so it is not run
-            if (!(s_rot & 2)) conv = true;
-        }
-    }
-    if (!conv && tid == 0) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-    // singular values (column norms) and descending order
-    for (int j = tid / LP; j < qq; j += SVD_NT / LP) {
-        double s2 = 0.0;
-#pragma unroll
-        for (int v = 0; v < NG; v++) {
-            const double x = Lc[j * S + p + LP * v];
-            s2 += x * x;
-        }
-        s2 = gsum_g<LP>(s2, gm);
-        // a NaN (corrupt input) would break the strict order below and leave
-        // order slots unset; it sorts last and is reported instead
-        if (p == 0) {
-            const bool nan = !(s2 == s2);
-            if (nan && j < q) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-            s_sig[j] = (j < q && !nan) ? sqrt(s2) : -1.0;
-        }
-    }
-    __syncthreads();
-    for (int j = tid; j < qq; j += SVD_NT) {
-        const double sj = s_sig[j];
-        int pos = 0;
-        for (int i = 0; i < qq; i++) {
-            const double si = s_sig[i];
-            pos += (si > sj) || (si == sj && i < j);
-        }
-        s_ord[pos] = j;
-    }
-    __syncthreads();
-    double* sig_out = ws + pl.o_sig;
-    if (tid == 0) {
-        const double s0 = q > 0 ? s_sig[s_ord[0]] : 0.0;
-        // numerical rank kept by LAPACK dgesvdq(JOBA='A'): sqrt(N)*eps*s0
-        const double thr = sqrt((double)q) * 1.1102230246251565e-16 * s0;
-        int nsv = q > 0 ? 1 : 0;
-        while (nsv < q && s_sig[s_ord[nsv]] >= thr) nsv++;
-        if (!(s0 == s0)) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-        // tail-sum rule, pattac.c:468-481
-        double ssum = 0.0;
-        int rank = nsv;
-        for (int j = nsv - 1; j >= 0; j--) {
-            const double sj = s_sig[s_ord[j]];
-            ssum += sj * sj;
-            if (sqrt(ssum) < delta)
-                rank = j;
-            else
-                break;
-        }
-        if (rank > q) rank = q;
-        if (rank > maxr) rank = maxr;
-        if (rank < 1) rank = 1;
-        info->rank = rank;
-        info->nsv = nsv;
-        info->sweeps = sweeps;
-        info->order = 0;
-        double tail = 0.0;
-        for (int j = rank; j < q; j++) tail += s_sig[s_ord[j]] * s_sig[s_ord[j]];
-        info->tail = tail;
-        if (pl.stats) {
-            double* st = pl.stats + (long long)bond * PTT_STAT_LEN;
-            st[0] = rank;
-            st[1] = nsv;
-            st[2] = sweeps;
-            st[3] = q;
-            st[4] = c;
-            st[5] = tail;
-            st[6] = delta;
-            st[7] = 0.0;
-            for (int j = 0; j < PTT_STAT_NSIG; j++) st[8 + j] = j < q ? s_sig[s_ord[j]] : 0.0;
-        }
-    }
-    for (int j = tid; j < CT; j += SVD_NT) {
-        sig_out[j] = j < q ? s_sig[s_ord[j]] : 0.0;
-        ((int*)(sig_out + CT))[j] = j < qq ? s_ord[j] : 0;
-    }
-    __syncthreads();
-    const int rank = info->rank;
-    double* US = ws + pl.o_US;  // c x rank, column-major ld CT
-    for (int e = tid; e < CT * CT; e += SVD_NT) {
-        const int b = e / CT, t = e - (e / CT) * CT;
-        US[e] = (b < rank && t < c) ? Lc[s_ord[b] * S + t] : 0.0;
-    }
-}
-
-// The same one-sided Jacobi with the columns kept in registers.  Group g of
-// LP lanes holds the two columns of pair g (rows p + LP v), and after each
-// round the columns move as the circle order moves them: pair g's top to
-// pair g - 1 (pair 0's top, column 0, stays; pair 1's top goes to pair 0's
-// bottom), pair g's bottom to pair g + 1 (the last pair's bottom becomes its
-// own top) -- warp shuffles between neighbouring groups, shared memory only
-// across warp boundaries (double-buffered, one block barrier per round).  The
-// tracked column norms travel with the columns.  Rotations are logged for
-// k_svd_replay(_b) exactly as by k_svd_jacobi, and after the last sweep the
-// columns are written to shared memory for the same epilogue (order, rank
-// rule, U S, statistics).
-// LP lanes per column pair (4: a round's rotation math, the same instructions
-// for every group of a warp, serves eight pairs per warp; the SVD is bound by
-// the instructions it issues on its one SM).
-template <int CT, int LP = 4>
-__host__ __device__ constexpr int ring_nt() {
-    return (CT / 2) * LP;
-}
-template <int CT, int LP = 4>
-__global__ void __launch_bounds__(ring_nt<CT, LP>(), 1) k_svd_ring(Plan pl, double* ws, double delta, int maxr, int bond,
-                                                               int* status) {
-    PTT_PDL_ENTRY();
-    constexpr int SVD_NT = ring_nt<CT, LP>();
-    constexpr int GPW = 32 / LP;           // groups per warp
-    constexpr int NG = CT / LP;            // rows per lane
-    constexpr int NW = SVD_NT / 32;        // warps
-    constexpr int S = CT + 1;
-    extern __shared__ double sm[];
-    double* Lc = sm;                                  // (CT + 2) columns x S, written after the sweeps
-    double* xch = sm + (CT + 2) * S;                  // [2 buffers][NW][2 (top, bottom)][LP lanes][NG + 1]
-    __shared__ double s_nrm[CT + 2];
-    __shared__ double s_sig[CT + 2];
-    __shared__ int s_ord[CT + 2];
-    __shared__ int s_rot;
-    __shared__ double s_wmax[NW];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int grp = tid / LP, p = tid % LP;
-    const unsigned gm = group_mask<LP>(tid);
-    Info* info = pl.info;
-    if (info->status) return;
-    const int c = info->c, q = info->q;
-    const int qq = q + (q & 1);
-    const int G = qq / 2;  // pairs of a round
-    const double* R = ws + pl.o_Rn;  // root factor, row-major CT x CT; L = R^T: column j = row j of R
-    // stationary-ring order (one column of each pair moves per round) over G2
-    // pairs, G rounded up to a power of two (the extra columns are zero and
-    // never rotated); circle order for a single pair
-    const bool stat = G >= 2;
-    const int G2 = stat ? 1 << (32 - __clz(G - 1)) : G;
-    const bool act = grp < G2;
-    // round 0: pair g holds columns g (top) and qq - 1 - g (circle) or G2 + g
-    // (stationary ring) (bottom)
-    double top[NG], bot[NG];
-    {
-        const int ct = grp, cb = stat ? G2 + grp : qq - 1 - grp;
-#pragma unroll
-        for (int v = 0; v < NG; v++) {
-            const int t = p + LP * v;
-            top[v] = (act && ct < q && t < c) ? R[(long long)ct * CT + t] : 0.0;
-            bot[v] = (act && cb < q && cb >= 0 && t < c) ? R[(long long)cb * CT + t] : 0.0;
-        }
-    }
-    double2* rot = (double2*)(ws + pl.o_rot);
-    const int npair = (CT + 2) / 2;
-    const double tol = (double)(c < 16 ? 16 : c) * 2.220446049250313e-16;
-    const double tol2 = tol * tol;
-    const int gw = lane / LP;  // group within the warp (0 .. GPW - 1)
-    int sweeps = 0, buf = 0;
-    bool conv = (qq < 2);
-    for (int sw = 0; sw < MAXSW && !conv; sw++) {
-        // exact column norms, and the noise threshold from the largest
-        double al = 0.0, be = 0.0;
-#pragma unroll
-        for (int v = 0; v < NG; v++) {
-            al = fma(top[v], top[v], al);
-            be = fma(bot[v], bot[v], be);
-        }
-        al = gsum_g<LP>(al, gm);
-        be = gsum_g<LP>(be, gm);
-        double mx = act ? fmax(al, be) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) s_wmax[warp] = mx;
-        if (tid == 0) s_rot = 0;
-        __syncthreads();
-        mx = 0.0;
-#pragma unroll
-        for (int w = 0; w < NW; w++) mx = fmax(mx, s_wmax[w]);
-        const double thr2 = (double)q * 1.232595164407831e-32 * mx;  // (sqrt(q) 2^-53)^2 max |a_j|^2
-        int myrot = 0;
-        // rotate the pair (top, bot) of this group; log it as pair grp of round rd
-        auto rotate = [&](int rd) {
-            double cs = 1.0, sn = 0.0;
-            double g0 = 0.0, g1 = 0.0;
-#pragma unroll
-            for (int v = 0; v < NG; v += 2) {
-                g0 = fma(top[v], bot[v], g0);
-                g1 = fma(top[v + 1], bot[v + 1], g1);
-            }
-            const double ga = gsum_g<LP>(g0 + g1, gm);
-            if (ga != 0.0 && al > thr2 && be > thr2 && ga * ga > tol2 * (al * be)) {
-                const double dd = be - al, g2 = 2.0 * ga;
-                const double ri = rsqrt(fma(dd, dd, g2 * g2));
-                const double hc = fma(0.5 * fabs(dd), ri, 0.5);
-                const double ic = rsqrt(hc);
-                cs = hc * ic;
-                sn = 0.5 * copysign(1.0, dd) * g2 * ri * ic;
-                const double t = sn * ic;
-#pragma unroll
-                for (int v = 0; v < NG; v++) {
-                    const double xa = top[v], xb = bot[v];
-                    top[v] = cs * xa - sn * xb;
-                    bot[v] = sn * xa + cs * xb;
-                }
-                al = al - t * ga;
-                be = be + t * ga;
-                myrot |= (ga * ga > 1e-16 * (al * be)) ? 3 : 1;
-            }
-            if (p == 0) rot[((long long)sw * (CT + 1) + rd) * npair + grp] = make_double2(cs, sn);
-        };
-        if (stat) {
-            // levels of block size hb = G2, G2 / 2, ..., 1 (see stat_cols)
-            int rd = 0;
-            for (int hb = G2; hb >= 1; hb >>= 1) {
-                const int i = grp & (hb - 1);
-                const bool cross = hb > GPW;  // the ring of hb pairs spans warps
-                const int wpb = cross ? hb / GPW : 1, wbase = warp - warp % wpb;
-                const int src = cross ? ((lane + LP) & 31) : ((i + 1 == hb) ? lane - (hb - 1) * LP : lane + LP);
-                for (int s = 0; s < hb; s++, rd++) {
-                    if (act) rotate(rd);
-                    if (hb == 1) continue;
-                    // second columns one pair back along the ring: within the
-                    // warp by shuffles, across warps through shared memory
-                    double* xb0 = xch + (long long)buf * NW * 2 * LP * (NG + 1);
-                    if (cross && gw == 0) {
-                        double* d = xb0 + (warp * 2 * LP + p) * (NG + 1);
-#pragma unroll
-                        for (int v = 0; v < NG; v++) d[v] = bot[v];
-                        d[NG] = be;
-                    }
-                    double nb[NG];
-#pragma unroll
-                    for (int v = 0; v < NG; v++) nb[v] = __shfl_sync(0xffffffffu, bot[v], src);
-                    double nbe = __shfl_sync(0xffffffffu, be, src);
-                    if (cross) {
-                        __syncthreads();
-                        if (gw == GPW - 1) {
-                            const int wn = wbase + (warp - wbase + 1) % wpb;
-                            const double* sx = xb0 + (wn * 2 * LP + p) * (NG + 1);
-#pragma unroll
-                            for (int v = 0; v < NG; v++) nb[v] = sx[v];
-                            nbe = sx[NG];
-                        }
-                        buf ^= 1;
-                    }
-#pragma unroll
-                    for (int v = 0; v < NG; v++) bot[v] = nb[v];
-                    be = nbe;
-                }
-                if (hb >= 2) {
-                    // split: pair i < h takes the first column of pair i + h
-                    // as its second, pair i + h the second column of pair i
-                    // as its first (h = hb / 2), through shared memory
-                    const int h = hb >> 1;
-                    const bool lo = i < h;
-                    double* d = Lc + ((long long)grp * LP + p) * (NG + 1);
-                    if (act) {
-#pragma unroll
-                        for (int v = 0; v < NG; v++) d[v] = lo ? bot[v] : top[v];
-                        d[NG] = lo ? be : al;
-                    }
-                    __syncthreads();
-                    if (act) {
-                        const double* sx = Lc + ((long long)(grp ^ h) * LP + p) * (NG + 1);
-                        if (lo) {
-#pragma unroll
-                            for (int v = 0; v < NG; v++) bot[v] = sx[v];
-                            be = sx[NG];
-                        } else {
-#pragma unroll
-                            for (int v = 0; v < NG; v++) top[v] = sx[v];
-                            al = sx[NG];
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            // back to the first arrangement: pair g holds columns 2g, 2g + 1
-            // after the last level; it starts the next sweep with g, G2 + g
-            if (act) {
-#pragma unroll
-                for (int v = 0; v < NG; v++) {
-                    Lc[(2 * grp) * S + p + LP * v] = top[v];
-                    Lc[(2 * grp + 1) * S + p + LP * v] = bot[v];
-                }
-            }
-            __syncthreads();
-            if (act) {
-#pragma unroll
-                for (int v = 0; v < NG; v++) {
-                    top[v] = Lc[grp * S + p + LP * v];
-                    bot[v] = Lc[(G2 + grp) * S + p + LP * v];
-                }
-            }
-        } else {
-            for (int rd = 0; rd < qq - 1; rd++) {
-                if (act) rotate(rd);
-                // move the columns to the next round's pairs
-                double* xb0 = xch + (long long)buf * NW * 2 * LP * (NG + 1);
-                if (gw == 0) {  // this warp's first top: to the previous warp's last group
-                    double* d = xb0 + ((warp * 2 + 0) * LP + p) * (NG + 1);
-#pragma unroll
-                    for (int v = 0; v < NG; v++) d[v] = top[v];
-                    d[NG] = al;
-                }
-                if (gw == GPW - 1) {  // this warp's last bottom: to the next warp's first group
-                    double* d = xb0 + ((warp * 2 + 1) * LP + p) * (NG + 1);
-#pragma unroll
-                    for (int v = 0; v < NG; v++) d[v] = bot[v];
-                    d[NG] = be;
-                }
-                double rt[NG], rb[NG];
-#pragma unroll
-                for (int v = 0; v < NG; v++) {
-                    rt[v] = __shfl_down_sync(0xffffffffu, top[v], LP);  // top of group + 1
-                    rb[v] = __shfl_up_sync(0xffffffffu, bot[v], LP);    // bottom of group - 1
-                }
-                double rta = __shfl_down_sync(0xffffffffu, al, LP);
-                double rbb = __shfl_up_sync(0xffffffffu, be, LP);
-                __syncthreads();
-                if (gw == GPW - 1 && warp + 1 < NW) {
-                    const double* sx = xb0 + (((warp + 1) * 2 + 0) * LP + p) * (NG + 1);
-#pragma unroll
-                    for (int v = 0; v < NG; v++) rt[v] = sx[v];
-                    rta = sx[NG];
-                }
-                if (gw == 0 && warp > 0) {
-                    const double* sx = xb0 + (((warp - 1) * 2 + 1) * LP + p) * (NG + 1);
-#pragma unroll
-                    for (int v = 0; v < NG; v++) rb[v] = sx[v];
-                    rbb = sx[NG];
-                }
-                buf ^= 1;
-                if (G == 1) {
-                    // one pair: both positions are fixed points of the circle order
-                } else if (grp == 0) {  // top fixed, bottom <- top of pair 1
-#pragma unroll
-                    for (int v = 0; v < NG; v++) bot[v] = rt[v];
-                    be = rta;
-                } else if (grp == G - 1) {  // top <- own bottom, bottom <- bottom of pair G - 2
-#pragma unroll
-                    for (int v = 0; v < NG; v++) {
-                        top[v] = bot[v];
-                        bot[v] = rb[v];
-                    }
-                    al = be;
-                    be = rbb;
-                } else if (act) {
-#pragma unroll
-                    for (int v = 0; v < NG; v++) {
-                        top[v] = rt[v];
-                        bot[v] = rb[v];
-                    }
-                    al = rta;
-                    be = rbb;
-                }
-            }
-        }
-        if (myrot) atomicOr(&s_rot, myrot);
-        __syncthreads();
-        if (s_rot == 0) {
-            conv = true;
-        } else {
-            sweeps = sw + 1;
-            if (!(s_rot & 2)) conv = true;
-        }
-        __syncthreads();  // s_rot is reset at the next sweep's start
-    }
-    if (!conv && tid == 0) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-    // the columns back to shared memory: each sweep ends with pair g holding
-    // columns g and qq - 1 - g (circle) or g and G2 + g (stationary ring)
-    if (act) {
-        const int cb = stat ? G2 + grp : qq - 1 - grp;
-#pragma unroll
-        for (int v = 0; v < NG; v++) {
-            Lc[grp * S + p + LP * v] = top[v];
-            Lc[cb * S + p + LP * v] = bot[v];
-        }
-    }
-    __syncthreads();
-    // singular values (column norms) and descending order
-    for (int j = tid / LP; j < qq; j += SVD_NT / LP) {
-        double s2 = 0.0;
-#pragma unroll
-        for (int v = 0; v < NG; v++) {
-            const double x = Lc[j * S + p + LP * v];
-            s2 += x * x;
-        }
-        s2 = gsum_g<LP>(s2, gm);
-        if (p == 0) {
-            const bool nan = !(s2 == s2);
-            if (nan && j < q) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-            s_sig[j] = (j < q && !nan) ? sqrt(s2) : -1.0;
-        }
-    }
-    __syncthreads();
-    for (int j = tid; j < qq; j += SVD_NT) {
-        const double sj = s_sig[j];
-        int pos = 0;
-        for (int i = 0; i < qq; i++) {
-            const double si = s_sig[i];
-            pos += (si > sj) || (si == sj && i < j);
-        }
-        s_ord[pos] = j;
-    }
-    __syncthreads();
-    double* sig_out = ws + pl.o_sig;
-    if (tid == 0) {
-        const double s0 = q > 0 ? s_sig[s_ord[0]] : 0.0;
-        const double thr = sqrt((double)q) * 1.1102230246251565e-16 * s0;
-        int nsv = q > 0 ? 1 : 0;
-        while (nsv < q && s_sig[s_ord[nsv]] >= thr) nsv++;
-        if (!(s0 == s0)) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-        double ssum = 0.0;
-        int rank = nsv;
-        for (int j = nsv - 1; j >= 0; j--) {
-            const double sj = s_sig[s_ord[j]];
-            ssum += sj * sj;
-            if (sqrt(ssum) < delta)
-                rank = j;
-            else
-                break;
-        }
-        if (rank > q) rank = q;
-        if (rank > maxr) rank = maxr;
-        if (rank < 1) rank = 1;
-        info->rank = rank;
-        info->nsv = nsv;
-        info->sweeps = sweeps;
-        info->order = stat ? 1 : 0;
-        double tail = 0.0;
-        for (int j = rank; j < q; j++) tail += s_sig[s_ord[j]] * s_sig[s_ord[j]];
-        info->tail = tail;
-        if (pl.stats) {
-            double* st = pl.stats + (long long)bond * PTT_STAT_LEN;
-            st[0] = rank;
-            st[1] = nsv;
-            st[2] = sweeps;
-            st[3] = q;
-            st[4] = c;
-            st[5] = tail;
-            st[6] = delta;
-            st[7] = 0.0;
-            for (int j = 0; j < PTT_STAT_NSIG; j++) st[8 + j] = j < q ? s_sig[s_ord[j]] : 0.0;
-        }
-    }
-    for (int j = tid; j < CT; j += SVD_NT) {
-        sig_out[j] = j < q ? s_sig[s_ord[j]] : 0.0;
-        ((int*)(sig_out + CT))[j] = j < qq ? s_ord[j] : 0;
-    }
-    __syncthreads();
-    const int rank = info->rank;
-    double* US = ws + pl.o_US;  // c x rank, column-major ld CT
-    for (int e = tid; e < CT * CT; e += SVD_NT) {
-        const int b = e / CT, t = e - (e / CT) * CT;
-        US[e] = (b < rank && t < c) ? Lc[s_ord[b] * S + t] : 0.0;
-    }
-}
-
-// The ring Jacobi is used for bonds of more than SVD_RING_MIN columns; below
-// that the shared-memory Jacobi was faster on one B200 (the reaction-Burgers
-// steps, whose bonds have <= ~40 columns: 105 vs 101 ms per plain step),
-// above it the ring (64 columns: 13.2 vs 21.7 ms for 39 bonds).
-constexpr int SVD_RING_MIN = 48;
-
-template <int CT, int LP = 4>
-static size_t ring_smem() {
-    constexpr int NW = ring_nt<CT, LP>() / 32;
-    return sizeof(double) * ((size_t)(CT + 2) * (CT + 1) + 2ull * NW * 2 * LP * (CT / LP + 1));
-}
+#include "ptt_svd.cuh"
 
 // Rebuild rows of V (q x q, V = product of the recorded rotations) and write
 // V_r = V[:, order[0:rank]] into Bn[root].  One warp per row; each sweep's
@@ -912,23 +256,18 @@ __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = bx * 8 + warp;
     if (info->status) return;
-    const int q = info->q, qq = q + (q & 1), sweeps = info->sweeps, rank = info->rank, order = info->order;
-    // pairs and rounds of a sweep: the stationary ring runs over qq / 2
-    // rounded up to a power of two
-    const int npr = (order == 1 && qq >= 4) ? 1 << (32 - __clz(qq / 2 - 1)) : qq / 2;
-    const int nrd = 2 * npr - 1;
-    // the column pair of every (round, pair) slot, once for all sweeps
+    const int q = info->q, sweeps = info->sweeps, rank = info->rank, order = info->order;
+    // pairs and steps of a sweep: two pairs for each of the G groups
+    const int Gc = (q + 3) >> 2;
+    const int G = order == ORD_RING ? (Gc > 1 ? 1 << (32 - __clz(Gc - 1)) : 1) : Gc;
+    const int npr = 2 * G, nrd = 4 * G - 1;
+    // the column pair of every (step, pair) slot, once for all sweeps
     unsigned char* pcol = (unsigned char*)(tab + (CT + 1) * npair);
     unsigned char* qcol = pcol + (CT + 1) * npair;
     for (int e = threadIdx.x; e < nrd * npr; e += blockDim.x) {
         const int rd = e / npr, i = e - (e / npr) * npr;
         int pc, qc;
-        if (order == 1) {
-            stat_cols(i, rd, npr, &pc, &qc);
-        } else {
-            pc = circle_col(i, rd, qq);
-            qc = circle_col(qq - 1 - i, rd, qq);
-        }
+        svd_pair(i, rd, G, order, &pc, &qc);
         pcol[rd * npair + i] = (unsigned char)pc;
         qcol[rd * npair + i] = (unsigned char)qc;
     }
@@ -947,8 +286,8 @@ __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, in
                     if (r.y != 0.0) {
                         const int pc = pcol[rd * npair + i], qc = qcol[rd * npair + i];
                         const double x = vrow[pc], y = vrow[qc];
-                        vrow[pc] = r.x * x - r.y * y;
-                        vrow[qc] = r.y * x + r.x * y;
+                        vrow[pc] = r.x * fma(-r.y, y, x);  // (cos, tan)
+                        vrow[qc] = r.x * fma(r.y, x, y);
                     }
                 }
                 __syncwarp();
@@ -1235,11 +574,6 @@ static size_t apply_smem() {
     const int VR = CT > H ? CT : H;
     return sizeof(double) * ((size_t)CT * KG + (size_t)VR * (CT + 1));
 }
-template <int CT>
-static size_t svd_smem() {
-    return sizeof(double) * (size_t)(CT + 2) * (CT + 1);
-}
-
 // 8 V rows + one sweep's rotation table ((CT+1) rounds x (CT+2)/2 pairs)
 template <int CT>
 static size_t replay_smem() {
@@ -1259,11 +593,13 @@ static int set_attrs() {
                                   (int)apply_smem<CT>()));
     PTT_CUDA(cudaFuncSetAttribute(k_apply_node<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)apply_smem<CT>()));
-    PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)svd_smem<CT>()));
-    if (CT <= 64)
-        PTT_CUDA(cudaFuncSetAttribute(k_svd_ring<CT <= 64 ? CT : 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)ring_smem<CT <= 64 ? CT : 64>()));
+    PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)svd_smem<64>()));
+    if constexpr (CT == 128) {
+        PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)svd_smem<96>()));
+        PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)svd_smem<128>()));
+    }
     PTT_CUDA(cudaFuncSetAttribute(k_svd_replay, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)replay_smem<128>()));
     if constexpr (CT >= 64) {
@@ -1279,6 +615,22 @@ static int set_attrs() {
     PTT_CUDA(cudaFuncSetAttribute(k_gemm_xm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::SMEM_GEMM));
     done.fetch_or(bit);
     return PTT_OK;
+}
+
+// SVD of a bond's factor (at most rk rows and columns): the kernel for the
+// smallest row bound that holds it, so that a small bond pays for no idle
+// lanes and rows.
+static int launch_svd(ptt_ctx* c, int rk, const Plan& pl, double* ws, double delta, int mr, int bond) {
+    auto go = [&](auto kernel, int nt, size_t smem) -> int {
+        PTT_CUDA(ptt_launch(c, kernel, dim3(1), dim3(nt), smem, pl, ws, delta, mr, bond, c->d_status));
+        return PTT_OK;
+    };
+    if (rk <= 16) return go(k_svd_jacobi<16>, svd_nt<16>(), svd_smem<16>());
+    if (rk <= 32) return go(k_svd_jacobi<32>, svd_nt<32>(), svd_smem<32>());
+    if (rk <= 48) return go(k_svd_jacobi<48>, svd_nt<48>(), svd_smem<48>());
+    if (rk <= 64) return go(k_svd_jacobi<64>, svd_nt<64>(), svd_smem<64>());
+    if (rk <= 96) return go(k_svd_jacobi<96>, svd_nt<96>(), svd_smem<96>());
+    return go(k_svd_jacobi<128>, svd_nt<128>(), svd_smem<128>());
 }
 
 // Factor the unfolding (mode) of core k; R lands at the root slot.  With the
@@ -1476,12 +828,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         if ((rc = launch_factor<CT>(c, x, i, RIGHT_T, pl, ws, g, mcap))) return rc;
         const int mr = maxr ? maxr[i] : rk[i];
         ptt_time_begin(c, PTT_TIME_SVD);
-        if (CT <= 64 && rk[i] > SVD_RING_MIN)  // columns in registers
-            PTT_CUDA(ptt_launch(c, k_svd_ring<CT <= 64 ? CT : 64>, dim3(1), dim3(ring_nt<CT <= 64 ? CT : 64>()),
-                                ring_smem<CT <= 64 ? CT : 64>(), pl, ws, delta, mr, i, c->d_status));
-        else
-            PTT_CUDA(ptt_launch(c, k_svd_jacobi<CT>, dim3(1), dim3(svd_nt<CT>()), svd_smem<CT>(), pl, ws, delta, mr,
-                                i, c->d_status));
+        if ((rc = launch_svd(c, rk[i], pl, ws, delta, mr, i))) return rc;
         ptt_time_end(c, PTT_TIME_SVD);
         PTT_LAUNCHED(c);
         // the tail: V_r, then Q V_r (Householder tree or grid Cholesky QR) into alt[i]
@@ -1815,8 +1162,7 @@ static int round_impl_w(ptt_tt* x, const int* rk, double delta, const int* maxr,
                 Wmax = Wr[i] > Wmax ? Wr[i] : Wmax;
                 const int mr = maxr ? maxr[i] : rk[i];
                 ptt_time_begin(c, PTT_TIME_SVD);
-                PTT_CUDA(ptt_launch(c, k_svd_jacobi<32>, dim3(1), dim3(svd_nt<32>()), svd_smem<32>(), pl, wsb, delta, mr, i,
-                                    c->d_status));
+                if ((rc = launch_svd(c, rk[i], pl, wsb, delta, mr, i))) return rc;
                 ptt_time_end(c, PTT_TIME_SVD);
                 PTT_LAUNCHED(c);
                 const long long mcap = (long long)rk[i - 1] * x->n[i - 1];

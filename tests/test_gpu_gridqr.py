@@ -28,7 +28,7 @@ def make(kind, n, c):
         x = [q * 2.0 ** -np.arange(q.shape[1]) if k < 3 else q for k, q in enumerate(x)]
         return [q.reshape(ranks[k], dims[k], ranks[k + 1], order="F") for k, q in enumerate(x)], 1e-8
     if kind == "repeated":  # x + 2 x at ranks c / 2 + c / 2
-        half = [1] + [(r + 1) // 2 for r in ranks[1:-1]] + [1]
+        half = [1, (min(c, n - 1) + 1) // 2, (c + 1) // 2, (min(c, n - 1) + 1) // 2, 1]
         x = gapped_tt(dims, half, 7, half)
         return O.axpby(1.0, x, 2.0, x), 1e-10
     x = gapped_tt(dims, ranks, 7, keep)
