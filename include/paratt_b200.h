@@ -121,7 +121,7 @@ PTT_API int ptt_ctx_pdl(ptt_ctx* ctx, int on);
  * Cholesky-QR cluster size the device holds and keeps the fastest per
  * (c, m) bucket in the context; roundings then use that table (results
  * differ from the untuned sizes only by rounding order).  Takes well under a
- * second; synchronises.  A size replaces the built-in rule (about 384 rows
+ * second; synchronises.  A size replaces the built-in rule (about 64 rows
  * per CTA) only when it timed at least 15 % faster.  ptt_ctx_autotune_table
  * writes the 18 entries (row-major [c bucket][m bucket]): the chosen size,
  * or 0 where the rule is kept (all 0 if not tuned). */

@@ -1,64 +1,49 @@
-// Cholesky QR of unfoldings with at most 32 columns (included by ptt_round.cu
-// inside its anonymous namespace, after the warp-level TSQR).
+// Cholesky QR of unfoldings with at most 32 columns by one thread-block
+// cluster (included by ptt_round.cu inside its anonymous namespace, after the
+// warp-level TSQR).
 //
 // The Householder TSQR is a chain of c x (tree depth + 1) dependent reflector
 // steps; here the only sequential work is a c-step Cholesky of a c x c Gram
-// matrix per stage.  A = Q R is computed as a sequence of Gram stages: stage
-// s holds the rows of Q_s = A R_1^{-1} ... R_s^{-1} (Q_0 = A; each stage
-// applies its new factor to the rows by a triangular solve), forms their Gram
-// matrix G_s = Q_s^T Q_s, and from it
-//   * s >= 1 and max|G_s - I| <= TAU: Q_s is orthonormal -- done, R = R_s ... R_1;
-//   * s >= 1 and max|G_s - I| <= FIRST: R_{s+1} = I + striu(E) + diag(E)/2 with
-//     E = G_s - I, the Cholesky factor of I + E to first order (Q_s R_{s+1}^{-1}
-//     is then orthonormal to O(c^2 max|E|^2)); when max|E| <= FIRST_DONE that
-//     is below TAU and Q_s R_{s+1}^{-1} is final without another Gram stage;
-//   * otherwise R_{s+1} = chol(G_s), or chol(G_s + sigma I) when a pivot is not
-//     positive or the pivots span more than 12 decades (condition > 1e6) --
-//     two warps form both factors at once and the plain one is kept if valid:
-//     shifted Cholesky QR (Fukaya, Kannan, Nakatsukasa, Yamamoto, Yanagisawa,
-//     SIAM J. Sci. Comput. 42 (2020)) with their shift
-//     sigma = 11 (m c + c (c + 1)) u ||Q_s||_F^2, which cannot break down and
-//     shrinks the condition number by ~sqrt(sigma) / ||Q_s||.
-// An unshifted stage on a matrix of condition kappa < 1e6 leaves an error
-// O(u kappa^2) that the next stages remove (repeated Cholesky QR, Yamamoto,
-// Nakatsukasa, Yanagisawa, Fukaya, ETNA 44 (2015)).  Each stage changes A = Q R
-// by O(u ||A||), so the R handed to the SVD carries the singular values of A to
-// the same absolute accuracy as a Householder R.  Condition numbers up to
-// 1e20 and exactly repeated columns converge within six stages.
+// matrix per stage, in 8 x 8 blocks.  The rules of the stages are those of
+// ptt_gramstage.cuh.
 //
-// One thread-block cluster factors one unfolding: CTA b of the cluster keeps
-// rows [b h, (b+1) h) (h = ceil(m / CS)) in shared memory for all stages, every CTA writes
-// the partial Gram matrix of its rows into its shared memory, and after a
-// cluster barrier every CTA sums all partials (distributed shared memory, CTA
-// order 0..CS-1) and runs the same Cholesky -- identical data and arithmetic,
-// so all CTAs take the same decisions and nothing is broadcast.  The partials
-// alternate between two buffers, so one barrier per stage suffices.  Only the
-// upper TS x TS tiles of the symmetric Gram matrix are formed (36 tiles x 7
-// row groups of threads), and the rows arrive by cp.async.
+// CTA b of the cluster keeps rows [b h, (b+1) h) (h = ceil(m / CS)) in shared
+// memory for all stages and writes the partial Gram matrix of its rows into its
+// shared memory; after a cluster barrier CTA b sums slice b of the entries over
+// all partials (distributed shared memory, CTA order 0..CS-1) and stores it
+// into every CTA's Gram matrix, and after another one every CTA takes the same
+// decision and factor from it -- identical data and arithmetic, so nothing
+// else is broadcast.  (Every CTA summing all partials moves 15 times the
+// matrix out of each SM: 2k cycles a stage at 16 columns, 5k at 32, against
+// ~1.5k with the second barrier.)  Within a CTA every warp takes the decision
+// by itself (lane = column) and warp 0 forms the factor.
+//
+// Bound by the latency of a stage (row solve, products, two barriers, remote
+// sum, decision, factor: ~8k cycles at 16 columns, ~15k at 32).  With one lane
+// per column in the Cholesky (~400 cycles a column, plain and shifted factors
+// in two warps), the decision's column loops in sequence, the row solve's
+// factor entries broadcast from shared memory one by one and 3.8 stages a
+// bond instead of 2.7, a factorisation of a time step took 29 us at 16 columns
+// and 123 us at 32; now 17 and 54.
 //
 // On success Q is written once: LEFT -> alt[k] (m x c, column-major), RIGHT_T
 // -> core[k] in place (row-major rows of c; k_cq_write forms Q V_r from it
-// after the bond's SVD).  A bond that does not converge within MAXST stages or
-// meets a NaN, a zero matrix or an exactly zero column is left untouched and
-// falls back to the Householder TSQR: k_wfactor / k_wapply skip the bonds
+// after the bond's SVD).  A bond that does not converge within MAXST stages,
+// has more columns than rows or meets a NaN or a zero matrix is left untouched
+// and falls back to the Householder TSQR: k_wfactor / k_wapply skip the bonds
 // finished here and k_cq_write skips the others.
 #pragma once
 
 namespace cq {
 
 namespace cg = cooperative_groups;
+using namespace gst;
 
 constexpr int NT = 256;       // threads per CTA
 constexpr int MAXST = 7;      // Gram stages per factorisation
 constexpr int CSMAX = 16;     // CTAs per cluster (non-portable size)
-constexpr int RTARGET = 384;  // rows per CTA the cluster size aims at
-constexpr int NG = 7;         // row groups of the Gram threads (36 tiles x 7 = 252)
-constexpr double TAU = 1e-13;
-constexpr double FIRST = 1e-7;
-constexpr double FIRST_DONE = 1e-8;
-constexpr double U = 1.1102230246251565e-16;  // unit roundoff of double
-
-enum { RUN = 0, DONE = 1, FALLBACK = 2, CHOL = 3, FINISH = 4 };
+constexpr int RTARGET = 64;   // rows per CTA the cluster size aims at: every part but the two barriers shrinks
+                              // with the rows (m = 1280, c = 20: 31 us with 4 CTAs, 27 with 16)
 static_assert(DONE == wt::CQ_DONE, "state code shared with the TSQR kernels");
 
 // Per-bond record at wsb + o_cq (REGION doubles).
@@ -66,136 +51,60 @@ struct State {
     int state;   // RUN, DONE or FALLBACK
     int nst;     // factors applied to Q
     int m, c;    // size of the factored unfolding
-    int nshift;  // shifted stages (diagnostic)
+    int ndrop;   // columns dropped (diagnostic)
     int pad[3];
 };
 constexpr long long REGION = 32;
 
 template <int CB>
 struct Cfg {
-    static constexpr int XP = CB + 2;        // shared row pitch (even)
-    static constexpr int TS = CB / 8;        // Gram tiles are TS x TS, 8 x 8 of them
-    static constexpr int UP = 36 * TS * TS;  // entries of the 36 upper tiles
-    static constexpr int EPT = (UP + NT - 1) / NT;
+    static constexpr int XP = CB + 4;  // shared row pitch: 4 mod 8 doubles, for the fragment loads
+    static constexpr int NB = CB / 8, NTL = NB * (NB + 1) / 2, UP = NTL * 64;  // upper 8 x 8 tiles
 };
 
-// shared memory (doubles): row-group partials, 2 folded partials, Gram, two
-// factors, two accumulated R, scalars, then the CTA's rows
+// shared memory (doubles): 4 warp-pair partials (the factor in the first of
+// them), the folded partial, the Gram matrix, two accumulated R, column
+// scalars, then the CTA's rows
 template <int CB>
 __host__ __device__ constexpr long long fixed_smem() {
-    return (long long)(NG + 2) * Cfg<CB>::UP + 33 * 32 + 2 * (33 * 32 + 32) + 2 * 33 * 32 + 64;
+    return 8LL * Cfg<CB>::UP + 6 * 32;
 }
 template <int CB>
 __host__ __device__ constexpr size_t smem(int rpb) {
-    return sizeof(double) * (size_t)(fixed_smem<CB>() + (long long)rpb * Cfg<CB>::XP);
+    return sizeof(double) * (size_t)(fixed_smem<CB>() + (long long)((rpb + 15) & ~15) * Cfg<CB>::XP);
 }
 constexpr size_t SMEM_MAX = 226 * 1024;  // dynamic; leaves room for the static variables
 template <int CB>
 __host__ __device__ constexpr int rpb_max() {
-    return (int)(((long long)(SMEM_MAX / sizeof(double)) - fixed_smem<CB>()) / Cfg<CB>::XP);
+    return (int)(((long long)(SMEM_MAX / sizeof(double)) - fixed_smem<CB>()) / Cfg<CB>::XP) & ~15;
 }
 
-// upper tile q (0..35) of the 8 x 8 tile grid -> tile row and column
-__device__ __forceinline__ void upper_tile(int q, int* ti, int* tj) {
-    int r = 0;
-    while (q >= 8 - r) {
-        q -= 8 - r;
-        r++;
-    }
-    *ti = r;
-    *tj = r + q;
-}
-
-// x <- x R^{-1} for the rows at x0 and (if two) x1 (R upper triangular c x c
-// in sR, pitch 33, inverse pivots at sR[33 * 32 + j]); each R entry read
-// serves both rows.
+// Cholesky factor of the equilibrated Gram matrix in the tiles at sF (nbc
+// column blocks), in place, by one warp (see gst::chol8); `live`: bits of the
+// columns kept; rinv[j] = 1 / R[j][j].
 template <int CB>
-__device__ __forceinline__ void row_solve2(double* x0s, double* x1s, bool two, const double* sR, int c) {
-    double x0[CB], x1[CB];
-    const double* s1 = two ? x1s : x0s;  // a single row is solved twice, stored once
-#pragma unroll
-    for (int j = 0; j < CB; j++) {
-        x0[j] = x0s[j];
-        x1[j] = s1[j];
-    }
-#pragma unroll
-    for (int j = 0; j < CB; j++) {
-        if (j >= c) continue;
-        const double iv = sR[33 * 32 + j];
-        const double y0 = x0[j] * iv, y1 = x1[j] * iv;
-        x0[j] = y0;
-        x1[j] = y1;
-#pragma unroll
-        for (int l = j + 1; l < CB; l++) {
-            const double r = sR[j * 33 + l];
-            x0[l] = fma(-y0, r, x0[l]);
-            x1[l] = fma(-y1, r, x1[l]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < CB; j++) x0s[j] = x0[j];
-    if (two) {
-#pragma unroll
-        for (int j = 0; j < CB; j++) x1s[j] = x1[j];
-    }
-}
-
-// Cholesky factor of G + shift I (c x c in sG, pitch 33) by one warp, lane =
-// column, into sR (row-major, pitch 33, zero outside c x c; inverse pivots at
-// sR[33 * 32 + j]).  Row j of R is broadcast through sRow.  Returns false
-// when a pivot is not positive; *ratio = min / max pivot.
-template <int CB>
-__device__ bool warp_chol(const double* sG, int c, double shift, double* sR, double* sRow, double* ratio) {
-    const int lane = threadIdx.x & 31;
-    double g[CB];
-#pragma unroll
-    for (int t = 0; t < CB; t++) g[t] = (t < c && lane < c) ? sG[t * 33 + lane] + (t == lane ? shift : 0.0) : 0.0;
-    bool ok = true;
-    double dmin = 1.0 / 0.0, dmax = 0.0;
-#pragma unroll
-    for (int j = 0; j < CB; j++) {
-        if (j >= c) continue;
-        const double d = __shfl_sync(0xffffffffu, g[j], j);
-        ok = ok && (d > 0.0);  // false for NaN
-        dmin = fmin(dmin, d);
-        dmax = fmax(dmax, d);
-        const double dd = d > 0.0 ? d : 1.0;
-        const double inv = rsqrt(dd);
-        const double rj = (lane == j) ? dd * inv : ((lane > j && lane < c) ? g[j] * inv : 0.0);
-        sRow[lane] = rj;
+__device__ __forceinline__ void warp_chol(double* sF, int nbc, unsigned live, double* rinv) {
+    const int lane = threadIdx.x & 31, li = lane >> 2, lk = lane & 3;
+    for (int J = 0; J < nbc; J++) {
+        double r[8][8], inv[8];
+        const int col = 8 * J + 8 + lane;  // this lane's column of the block row
+        const unsigned weak = chol8(sF + tnum(J, J) * 64, (live >> (8 * J)) & 0xffu, r, inv);
         __syncwarp();
-        if (lane > j && lane < c) {
+        if (col < 8 * nbc) solve8(sF + tnum(J, col >> 3) * 64, col & 7, r, inv, weak);
+        if (lane == 31) {
+            double* G = sF + tnum(J, J) * 64;
 #pragma unroll
-            for (int t = j + 1; t < CB; t++) g[t] = fma(-sRow[t], rj, g[t]);
+            for (int i = 0; i < 8; i++) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) G[tix(i, j)] = j >= i ? r[i][j] : 0.0;
+                rinv[8 * J + i] = inv[i];
+            }
         }
-        sR[j * 33 + lane] = rj;
-        if (lane == j) sR[33 * 32 + j] = inv;
+        __syncwarp();
+        for (int K = J + 1; K < nbc; K++)
+            for (int I = J + 1; I <= K; I++) trail8(sF, J, I, K, li, lk);
         __syncwarp();
     }
-    for (int j = c; j < 32; j++) {
-        sR[j * 33 + lane] = 0.0;
-        if (lane == j) sR[33 * 32 + j] = 0.0;
-    }
-    __syncwarp();
-    *ratio = dmax > 0.0 ? dmin / dmax : 0.0;
-    return ok;
-}
-
-// First-order Cholesky factor of G = I + E by one warp (lane = column).
-__device__ __forceinline__ void warp_first_order(const double* sG, int c, double* sR) {
-    const int lane = threadIdx.x & 31;
-    for (int j = 0; j < 32; j++) {
-        double v = 0.0;
-        if (j < c && lane < c) {
-            if (lane > j)
-                v = sG[j * 33 + lane];
-            else if (lane == j)
-                v = 1.0 + 0.5 * (sG[j * 33 + j] - 1.0);
-        }
-        sR[j * 33 + lane] = v;
-    }
-    sR[33 * 32 + lane] = lane < c ? 1.0 / (1.0 + 0.5 * (sG[lane * 33 + lane] - 1.0)) : 0.0;
-    __syncwarp();
 }
 
 // Factor core k's unfolding (mode) by the Cholesky sequence above.  Launched
@@ -205,27 +114,29 @@ template <int CB>
 __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, int mode, Plan pl, wt::WP wp,
                                                   double* wsb, int rpb, long long* qstat) {
     PTT_PDL_ENTRY();
-    constexpr int XP = Cfg<CB>::XP, TS = Cfg<CB>::TS, UP = Cfg<CB>::UP, EPT = Cfg<CB>::EPT;
+    using C = Cfg<CB>;
+    constexpr int XP = C::XP, NB = C::NB, NTL = C::NTL, UP = C::UP;
+    constexpr unsigned FULL = 0xffffffffu;
     cg::cluster_group cl = cg::this_cluster();
     const int CS = (int)cl.num_blocks();
     const int crank = (int)cl.block_rank();
-    extern __shared__ double csm[];
-    double* sScr = csm;                // NG row-group partials (UP each)
-    double* sP = sScr + NG * UP;       // 2 folded partials, read by the other CTAs
-    double* sG = sP + 2 * UP;          // 32 x 33 Gram of the whole unfolding
-    double* sRa = sG + 33 * 32;        // factor (32 x 33) + 32 inverse pivots: plain Cholesky
-    double* sRb = sRa + 33 * 32 + 32;  // the same for the shifted Cholesky
-    double* sT = sRb + 33 * 32 + 32;   // 32 x 33 accumulated R = R_s ... R_1
-    double* sTn = sT + 33 * 32;        // 32 x 33 the other buffer of it
-    double* sRow = sTn + 33 * 32;      // 2 x 32 scalars
-    double* Xs = sRow + 64;            // rpb x XP rows of this CTA
-    double* sR = sRa;                  // factor of the current stage
-    __shared__ int s_dec, s_ok[2];
-    __shared__ double s_ratio[2];
+    extern __shared__ __align__(16) double csm[];
+    double* sScr = csm;             // 4 warp-pair partials
+    double* sF = csm;               // the factor of the stage, once the partials are folded
+    double* sP = sScr + 4 * UP;     // folded partial, read by the other CTAs
+    double* sG = sP + UP;           // Gram matrix of the whole unfolding, written by all CTAs
+    double* sT = sG + UP;           // accumulated R = R_s ... R_1
+    double* sTn = sT + UP;          // the other buffer of it
+    double* s_rinv = sTn + UP;      // inverse pivots of sF
+    double* s_an = s_rinv + 32;     // 1 / |a_j|
+    double* s_d = s_an + 32;        // |q_j| of the columns kept, their inverses
+    double* s_di = s_d + 32;
+    unsigned long long* s_tm = (unsigned long long*)(s_di + 32);  // max_j |T_ij| / |a_j|, two buffers
+    double* Xs = s_di + 96;         // rpb x XP rows of this CTA
     State* st = (State*)(wsb + wp.o_cq);
     const View A = make_view(D, k, mode, false);
     const int m = A.m, c = A.c;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, li = lane >> 2, lk = lane & 3;
     if (c > CB || c < 1 || m < c || (long long)m > (long long)rpb * CS) {  // uniform: Householder TSQR
         if (crank == 0 && tid == 0) {
             st->state = FALLBACK;
@@ -241,217 +152,214 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
     const int rpbd = (m + CS - 1) / CS;  // <= rpb
     const int r0 = crank * rpbd;
     const int h = (m - r0) < rpbd ? ((m - r0) > 0 ? (m - r0) : 0) : rpbd;
-    // this CTA's rows: zero, then every element by cp.async (all in flight)
-    for (int e = tid; e < h * XP; e += NT) Xs[e] = 0.0;
-    for (int e = tid; e < 32 * 33; e += NT) {
-        sT[e] = ((e / 33) == (e % 33) && (e / 33) < c) ? 1.0 : 0.0;
-        sTn[e] = 0.0;
-    }
-    __syncthreads();
+    const int nbc = (c + 7) >> 3, nt = nbc * (nbc + 1) / 2;
+    // this CTA's rows, every element in flight by cp.async; zeros beyond c
     {
-        const int tot = h * c;
         const unsigned xs0 = (unsigned)__cvta_generic_to_shared(Xs);
-        for (int f = tid; f < tot; f += NT) {
-            int row, col;
-            const double* g;
-            if (mode == LEFT) {  // column-major: a column's rows are contiguous
-                col = f / h;
-                row = f - col * h;
-                g = A.p + (long long)(r0 + row) + (long long)col * m;
-            } else {  // RIGHT_T: this CTA's rows are one contiguous range
-                row = f / c;
-                col = f - row * c;
-                g = A.p + (long long)r0 * c + f;
+        if (mode == LEFT) {  // column-major: a warp copies a column's contiguous rows
+            for (int col = warp; col < c; col += NT / 32) {
+                const double* g = A.p + (long long)r0 + (long long)col * m;
+                for (int row = lane; row < h; row += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(xs0 + 8u * (unsigned)(row * XP + col)),
+                                 "l"(g + row)
+                                 : "memory");
             }
-            const unsigned sa = xs0 + 8u * (unsigned)(row * XP + col);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(g) : "memory");
+        } else {  // RIGHT_T: this CTA's rows are one contiguous range, stepped without divisions
+            const int dq = NT / c, dr = NT - dq * c, tot = h * c;
+            int row = tid / c, col = tid - row * c;
+            const double* g = A.p + (long long)r0 * c;
+            for (int f = tid; f < tot; f += NT) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(xs0 + 8u * (unsigned)(row * XP + col)),
+                             "l"(g + f)
+                             : "memory");
+                row += dq;
+                col += dr;
+                if (col >= c) {
+                    col -= c;
+                    row++;
+                }
+            }
         }
+        const int cz = CB - c, h16 = (h + 15) & ~15;
+        for (int col = warp; col < cz; col += NT / 32)
+            for (int row = lane; row < h; row += 32) Xs[row * XP + c + col] = 0.0;
+        for (int e = tid; e < (h16 - h) * XP; e += NT) Xs[h * XP + e] = 0.0;
         asm volatile("cp.async.wait_all;\n" ::: "memory");
     }
     __syncthreads();
     // Gram warps: rows [4 ks0, 4 ks1) of this CTA, every 8 x 8 tile of the
-    // NB column blocks (mma.m8n8k4: four rows a step, the block's fragment
-    // serves as A and as B)
-    constexpr int NB = CB / 8, NTL = NB * (NB + 1) / 2;
-    static_assert(4 * NTL * 64 <= NG * UP, "the warp tiles fit the Gram scratch");
-    const int warp = tid >> 5, lane = tid & 31, li = lane >> 2, lk = lane & 3;
+    // column blocks (mma.m8n8k4: four rows a step, a block's fragment serves
+    // as A and as B)
     const int nks = (h + 3) / 4;
     const int ks0 = (nks * warp) / (NT / 32), ks1 = (nks * (warp + 1)) / (NT / 32);
-    int dec = RUN, nst = 0, nshift = 0, stage = 0;
+    const double dropc = DROP * sqrt((double)c);
+    int dec = RUN, nst = 0, stage = 0, ndrop = 0;
+    unsigned live = 0;
     for (stage = 0; stage < MAXST; stage++) {
         if (stage > 0) {  // Q_stage = Q_{stage-1} R_stage^{-1}
-            for (int r = tid; r < h; r += 2 * NT) row_solve2<CB>(Xs + r * XP, Xs + (r + NT) * XP, r + NT < h, sR, c);
+            tile_solve<XP, NT / 32>(Xs, h, sF, s_rinv, nbc);
             __syncthreads();
         }
         // partial Gram of this CTA's rows on the FP64 tensor cores: each warp
         // its rows, all tiles; warps w and w + 4 are added in shared memory,
-        // then the four sums in warp order into the grid layout of myP
+        // then the four sums in warp order
         {
             double c0[NTL], c1[NTL];
 #pragma unroll
-            for (int t = 0; t < NTL; t++) {
-                c0[t] = 0.0;
-                c1[t] = 0.0;
-            }
+            for (int t = 0; t < NTL; t++) c0[t] = c1[t] = 0.0;
             for (int ks = ks0; ks < ks1; ks++) {
-                const int row = 4 * ks + lk;
+                const double* xr = Xs + (4 * ks + lk) * XP + li;
                 double f[NB];
 #pragma unroll
-                for (int bb = 0; bb < NB; bb++) f[bb] = row < h ? Xs[row * XP + 8 * bb + li] : 0.0;
+                for (int bb = 0; bb < NB; bb++) f[bb] = xr[8 * bb];
                 int t = 0;
 #pragma unroll
-                for (int I = 0; I < NB; I++)
+                for (int J = 0; J < NB; J++)
 #pragma unroll
-                    for (int J = I; J < NB; J++, t++)
-                        asm volatile(
-                            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                            : "+d"(c0[t]), "+d"(c1[t])
-                            : "d"(f[I]), "d"(f[J]));
+                    for (int I = 0; I <= J; I++, t++) mma884(c0[t], c1[t], f[I], f[J]);
             }
-            double* slot = sScr + (warp & 3) * NTL * 64 + li * 8 + 2 * lk;
+            double* slot = sScr + (warp & 3) * UP + tix(li, 2 * lk);
             if (warp < 4) {
 #pragma unroll
-                for (int t = 0; t < NTL; t++) {
-                    slot[t * 64] = c0[t];
-                    slot[t * 64 + 1] = c1[t];
-                }
+                for (int t = 0; t < NTL; t++) *(double2*)(slot + t * 64) = make_double2(c0[t], c1[t]);
             }
             __syncthreads();
             if (warp >= 4) {
 #pragma unroll
                 for (int t = 0; t < NTL; t++) {
-                    slot[t * 64] += c0[t];
-                    slot[t * 64 + 1] += c1[t];
+                    const double2 v = *(const double2*)(slot + t * 64);
+                    *(double2*)(slot + t * 64) = make_double2(v.x + c0[t], v.y + c1[t]);
                 }
             }
             __syncthreads();
         }
-        double* myP = sP + (stage & 1) * UP;
-        for (int u = tid; u < UP; u += NT) {
-            // entry (gi, gj) of upper grid tile qq, from the 8 x 8 tile of its
-            // column blocks (the symmetric entry when gi's block is the later)
-            const int qq = u / (TS * TS), w = u - qq * (TS * TS);
-            int a0, b0;
-            upper_tile(qq, &a0, &b0);
-            int gi = a0 * TS + w / TS, gj = b0 * TS + w % TS;
-            if ((gi >> 3) > (gj >> 3)) {
-                const int tmp = gi;
-                gi = gj;
-                gj = tmp;
-            }
-            const int I = gi >> 3, J = gj >> 3;
-            const int e = (I * NB - (I * (I - 1)) / 2 + (J - I)) * 64 + (gi & 7) * 8 + (gj & 7);
-            myP[u] = ((sScr[e] + sScr[NTL * 64 + e]) + sScr[2 * NTL * 64 + e]) + sScr[3 * NTL * 64 + e];
-        }
+        for (int u = tid; u < nt * 64; u += NT)
+            sP[u] = ((sScr[u] + sScr[UP + u]) + sScr[2 * UP + u]) + sScr[3 * UP + u];
         cl.sync();  // every CTA's partial is complete and visible
-        // sum the CTAs' partials in CTA order (distributed shared memory),
-        // every load issued before the sums
+        // this CTA's slice of the entries, summed in CTA order (every load
+        // issued before the sums), into every CTA's Gram matrix
         {
-            double v[EPT][CSMAX];
+            const int per = (nt * 64 + CS - 1) / CS, u0 = crank * per;
+            for (int e = tid; e < per; e += NT) {
+                const int u = u0 + e;
+                if (u < nt * 64) {
+                    double v[CSMAX];
 #pragma unroll
-            for (int i = 0; i < EPT; i++) {
-                const int u = tid + i * NT;
-#pragma unroll
-                for (int b = 0; b < CSMAX; b++) v[i][b] = (u < UP && b < CS) ? cl.map_shared_rank(myP, b)[u] : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < EPT; i++) {
-                const int u = tid + i * NT;
-                if (u < UP) {
+                    for (int b = 0; b < CSMAX; b++) v[b] = b < CS ? cl.map_shared_rank(sP, b)[u] : 0.0;
                     double s2 = 0.0;
 #pragma unroll
-                    for (int b = 0; b < CSMAX; b++) s2 += v[i][b];  // zeros beyond CS leave the sum unchanged
-                    const int qq = u / (TS * TS), w = u - qq * (TS * TS);
-                    int a0, b0;
-                    upper_tile(qq, &a0, &b0);
-                    const int gi = a0 * TS + w / TS, gj = b0 * TS + w % TS;
-                    sG[gi * 33 + gj] = s2;
-                    sG[gj * 33 + gi] = s2;
-                }
-            }
-        }
-        __syncthreads();
-        // decision; when a Cholesky factor is needed warp 0 forms the plain
-        // and warp 1 the shifted one at the same time
-        if (tid < 64) {
-            const int lane = tid & 31, wq = tid >> 5;
-            double tr = (lane < c) ? sG[lane * 33 + lane] : 0.0;
-            double e = 0.0;
-            bool nan = false;
-            for (int t = 0; t < c; t++) {
-                const double v2 = (lane < c) ? sG[t * 33 + lane] - (t == lane ? 1.0 : 0.0) : 0.0;
-                nan = nan || !(v2 == v2);
-                e = fmax(e, fabs(v2));
-            }
+                    for (int b = 0; b < CSMAX; b++) s2 += v[b];  // zeros beyond CS leave the sum unchanged
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                tr += __shfl_xor_sync(0xffffffffu, tr, o);
-                e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
-            }
-            nan = __any_sync(0xffffffffu, nan);
-            // an exactly zero column stays zero under every stage: leave the
-            // bond to the Householder TSQR at once
-            const bool zcol = __any_sync(0xffffffffu, lane < c && sG[lane * 33 + lane] == 0.0);
-            int d;
-            if (nan || !(tr > 0.0) || !(tr < 1.0 / 0.0) || (stage == 0 && zcol)) {
-                d = FALLBACK;
-            } else if (stage >= 1 && e <= TAU) {
-                d = DONE;
-            } else if (stage >= 1 && e <= FIRST) {
-                if (wq == 0) warp_first_order(sG, c, sRa);
-                d = e <= FIRST_DONE ? FINISH : RUN;
-            } else if (stage == MAXST - 1) {
-                d = FALLBACK;
-            } else {
-                const double sigma = wq ? 11.0 * ((double)m * c + (double)c * (c + 1)) * U * tr : 0.0;
-                double ratio;
-                const bool ok = warp_chol<CB>(sG, c, sigma, wq ? sRb : sRa, sRow + 32 * wq, &ratio);
-                if (lane == 0) {
-                    s_ok[wq] = ok;
-                    s_ratio[wq] = ratio;
+                    for (int b = 0; b < CSMAX; b++)
+                        if (b < CS) cl.map_shared_rank(sG, b)[u] = s2;
                 }
-                d = CHOL;
             }
-            if (tid == 0) s_dec = d;
         }
-        __syncthreads();
-        dec = s_dec;
-        sR = sRa;
-        if (dec == CHOL) {
-            if (s_ok[0] && s_ratio[0] >= 1e-12) {
-                dec = RUN;
-            } else if (s_ok[1]) {
-                dec = RUN;
-                sR = sRb;
-                nshift++;
-            } else {
-                dec = FALLBACK;
+        cl.sync();  // the Gram matrix is complete in every CTA
+        // the decision, by every warp from the same data: lane = column
+        double dj;
+        float emaxf = 0.f;
+        {
+            const double gjj = lane < c ? sG[telem(lane, lane)] : 0.0;
+            dj = gjj > 0.0 ? sqrt(gjj) : 0.0;
+            bool on = gjj > 0.0;
+            if (stage > 0)
+                on = on && dj * __longlong_as_double((long long)s_tm[32 * (stage & 1) + lane]) > dropc;
+            bool bad = lane < c && (!(gjj >= 0.0 && gjj < LARGE) || (gjj != 0.0 && gjj < SMALL));
+            live = __ballot_sync(FULL, on);
+            const unsigned l0 = live >> li, l1 = live >> (2 * lk);
+#pragma unroll
+            for (int J = 0; J < NB; J++) {
+                if (8 * J < c) {  // uniform
+#pragma unroll
+                    for (int I = 0; I <= J; I++) {  // two entries a lane of every tile
+                        const double2 v = *(const double2*)(sG + tnum(I, J) * 64 + tix(li, 2 * lk));
+                        const bool d0 = I == J && li == 2 * lk, d1 = I == J && li == 2 * lk + 1;
+                        bad = bad || !(v.x - v.x == 0.0) || !(v.y - v.y == 0.0);
+                        const float e0 = fabsf((float)(v.x - (d0 ? 1.0 : 0.0))), e1 = fabsf((float)(v.y - (d1 ? 1.0 : 0.0)));
+                        const bool oi = (l0 >> (8 * I)) & 1u;
+                        if (oi && ((l1 >> (8 * J)) & 1u)) emaxf = fmaxf(emaxf, e0);
+                        if (oi && ((l1 >> (8 * J + 1)) & 1u)) emaxf = fmaxf(emaxf, e1);
+                    }
+                }
             }
+            // non-negative values order as their bits; the thresholds lie decades
+            // apart, so single precision decides
+            emaxf = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(emaxf)));
+            if (__any_sync(FULL, bad)) live = 0u;
+        }
+        const double emax = (double)emaxf;
+        ndrop = c - __popc(live);
+        if (live == 0u) {
+            dec = FALLBACK;
+        } else if (stage >= 1 && emax <= TAU) {
+            dec = DONE;
+        } else if (stage == MAXST - 1) {
+            dec = FALLBACK;
+        } else if (stage >= 1 && emax <= FIRST) {
+            dec = emax <= FIRST_DONE ? FINISH : RUN;
+        } else {
+            dec = RUN;
         }
         if (dec == DONE || dec == FALLBACK) break;
+        const bool first = stage >= 1 && emax <= FIRST;
         nst = stage + 1;
-        // R <- R_{stage+1} R (both upper triangular, zero beyond c) into the
-        // other buffer on the FP64 tensor cores: warp w forms 8 x 8 tiles w and
-        // w + 8 of the 10 upper tiles, k over the tile's triangle band; the
-        // tiles below the diagonal of sTn stay zero from the start, the lower
-        // halves of the diagonal tiles come out as exact zeros
-        for (int t = warp; t < 10; t += NT / 32) {
-            int I = 0, J = t;
-            while (J >= 4 - I) {
-                J -= 4 - I;
-                I++;
+        // H (or the first-order factor) into sF by all warps; the column
+        // scalars by each warp (the same values)
+        {
+            const bool on = (live >> lane) & 1u;
+            const double di = on ? 1.0 / dj : 0.0;
+            s_d[lane] = on ? dj : 0.0;
+            s_di[lane] = di;
+            if (stage == 0) s_an[lane] = di;
+            if (warp == 0) s_tm[32 * ((stage + 1) & 1) + lane] = 0ull;
+            __syncwarp();
+        }
+        for (int t = warp; t < nt; t += NT / 32) {
+            int I, J;
+            tile_of(t, &I, &J);
+            const int at = t * 64 + tix(li, 2 * lk);
+            const double2 v = *(const double2*)(sG + at);
+            const int i = 8 * I + li, j = 8 * J + 2 * lk;
+            double2 w;
+            if (first) {
+                const bool oi = (live >> i) & 1u, o0 = (live >> j) & 1u, o1 = (live >> (j + 1)) & 1u;
+                w.x = !(oi && o0) || j < i ? 0.0 : (i == j ? 1.0 + 0.5 * (v.x - 1.0) : v.x);
+                w.y = !(oi && o1) || j + 1 < i ? 0.0 : (i == j + 1 ? 1.0 + 0.5 * (v.y - 1.0) : v.y);
+                if (i == j) s_rinv[i] = w.x != 0.0 ? 1.0 / w.x : 0.0;
+                if (i == j + 1) s_rinv[i] = w.y != 0.0 ? 1.0 / w.y : 0.0;
+            } else {
+                w.x = v.x * s_di[i] * s_di[j];
+                w.y = v.y * s_di[i] * s_di[j + 1];
             }
-            J += I;
-            double d0 = 0.0, d1 = 0.0;
-            for (int k0 = 8 * I; k0 < 8 * J + 8; k0 += 4) {
-                const double av = sR[(8 * I + li) * 33 + k0 + lk];
-                const double bv = sT[(k0 + lk) * 33 + 8 * J + li];
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                             : "+d"(d0), "+d"(d1)
-                             : "d"(av), "d"(bv));
+            *(double2*)(sF + at) = w;
+        }
+        __syncthreads();
+        if (!first) {
+            if (warp == 0) {
+                warp_chol<CB>(sF, nbc, live, s_rinv);
+                if (lane < 8 * nbc) s_rinv[lane] *= s_di[lane];
             }
-            sTn[(8 * I + li) * 33 + 8 * J + 2 * lk] = d0;
-            sTn[(8 * I + li) * 33 + 8 * J + 2 * lk + 1] = d1;
+            __syncthreads();
+            for (int t = warp; t < nt; t += NT / 32) {  // R = chol(H) D
+                int I, J;
+                tile_of(t, &I, &J);
+                double2* pv = (double2*)(sF + t * 64 + tix(li, 2 * lk));
+                const double2 v = *pv;
+                *pv = make_double2(v.x * s_d[8 * J + 2 * lk], v.y * s_d[8 * J + 2 * lk + 1]);
+            }
+            __syncthreads();
+        }
+        // R <- R_{stage+1} R into the other buffer, and max_j |R_ij| / |a_j|
+        for (int t = warp; t < nt; t += NT / 32) {
+            int I, J;
+            tile_of(t, &I, &J);
+            const int at = t * 64 + tix(li, 2 * lk);
+            const double2 v = stage == 0 ? *(const double2*)(sF + at) : tile_product(sF, sT, I, J, li, lk);
+            *(double2*)(sTn + at) = v;
+            const int j = 8 * J + 2 * lk;
+            const double w = fmax(fabs(v.x) * s_an[j], fabs(v.y) * s_an[j + 1]);
+            atomicMax(&s_tm[32 * ((stage + 1) & 1) + 8 * I + li], (unsigned long long)__double_as_longlong(w));
         }
         {
             double* t2 = sT;
@@ -459,9 +367,10 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
             sTn = t2;
         }
         if (dec == FINISH) {  // apply the first-order factor; Q is final
-            for (int r = tid; r < h; r += 2 * NT) row_solve2<CB>(Xs + r * XP, Xs + (r + NT) * XP, r + NT < h, sR, c);
+            tile_solve<XP, NT / 32>(Xs, h, sF, s_rinv, nbc);
             __syncthreads();
             dec = DONE;
+            live = FULL;  // R carries the dropped columns' zero rows
             break;
         }
         __syncthreads();
@@ -470,22 +379,30 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
     if (dec == DONE) {
         if (mode == LEFT) {
             double* out = D->alt[k];
-            for (int e = tid; e < h * c; e += NT) {
-                const int col = e / h, row = e - col * h;
-                out[(long long)(r0 + row) + (long long)col * m] = Xs[row * XP + col];
+            for (int col = warp; col < c; col += NT / 32) {
+                double* g = out + (long long)r0 + (long long)col * m;
+                for (int row = lane; row < h; row += 32) g[row] = Xs[row * XP + col];
             }
         } else {
             double* out = A.p + (long long)r0 * c;  // in place over A: this CTA's rows only
-            for (int e = tid; e < h * c; e += NT) {
-                const int row = e / c, col = e - row * c;
-                out[e] = Xs[row * XP + col];
+            const int dq = NT / c, dr = NT - dq * c, tot = h * c;
+            int row = tid / c, col = tid - row * c;
+            for (int f = tid; f < tot; f += NT) {
+                out[f] = Xs[row * XP + col];
+                row += dq;
+                col += dr;
+                if (col >= c) {
+                    col -= c;
+                    row++;
+                }
             }
         }
         if (crank == 0) {
             double* Rs = wsb + wp.o_R;  // root slot, row-major 32 x 32
             for (int e = tid; e < 1024; e += NT) {
                 const int i = e >> 5, j = e & 31;
-                Rs[e] = (i < c && j < c && j >= i) ? sT[i * 33 + j] : 0.0;
+                // a column dropped by the deciding stage takes its row of R with it
+                Rs[e] = (i < c && j < c && j >= i && ((live >> i) & 1u)) ? sT[telem(i, j)] : 0.0;
             }
             if (tid == 0) {
                 Info* info = (Info*)(wsb + pl.o_info_d);
@@ -506,7 +423,7 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
         st->nst = nst;
         st->m = m;
         st->c = c;
-        st->nshift = nshift;
+        st->ndrop = ndrop;
         if (dec == FALLBACK && qstat) atomicAdd((unsigned long long*)(qstat + 1), 1ull);
     }
 }

@@ -5,7 +5,7 @@
 // rank 64: 8.4 MB) does not fit one cluster's shared memory, and the
 // Householder TSQR costs one block barrier per reflector and tree level.
 // Here the rows are spread over all SMs and A = Q R is a sequence of Gram
-// stages (the decisions are those of gq::decide below), two launches each:
+// stages, two launches each:
 //
 //   k_gq_rows    CTA b loads its rows of Q_{s-1} (A for s <= 1), applies the
 //                factor of the previous stage by a row-wise triangular solve
@@ -19,30 +19,7 @@
 // longer than everything else it had to do (the partials are 18 KB each at 64
 // columns and 70 KB at 128; a single SM reads them at ~64 bytes a cycle).
 //
-// A stage with Gram matrix G = Q_s^T Q_s, accumulated R = T (A = Q_s T):
-//   * columns whose part of A is below the rounding of A are dropped: column
-//     j of Q_s adds q_j T_j: to A, at most |q_j| max_i |T_ji| / |a_i| of each
-//     column a_i; where that is below 0.5 sqrt(c) u it is rounding noise of A,
-//     and q_j and T_j: are set to zero (exactly zero columns of A likewise).
-//     Unfoldings of sums are numerically rank-deficient: without this the
-//     noise directions kept the sequence busy for up to eight stages, and 11
-//     of the 78 factorisations of a rank-64 rounding with d = 40 fell back;
-//   * s >= 1 and max|G - I| <= TAU over the other columns: done, R = T;
-//   * s >= 1 and max|G - I| <= FIRST: R_{s+1} = I + striu(E) + diag(E)/2, the
-//     Cholesky factor of I + E to first order; when max|E| <= FIRST_DONE that
-//     finishes without another Gram stage;
-//   * otherwise R_{s+1} = chol(H) D with D = diag(|q_j|) and H = D^-1 G D^-1
-//     (unit diagonal, so the scale of a column does not matter).  A pivot
-//     below PIV is set to PIV and the rest of its row of R to zero: the column
-//     is only rescaled and is orthogonalised against the others in the next
-//     stage, where it has unit norm again.  So every stage resolves another
-//     seven decades of the spectrum, whatever the condition: condition 1e25
-//     and exactly repeated columns take four or five stages.  (Shifted
-//     Cholesky QR -- Fukaya, Kannan, Nakatsukasa, Yamamoto, Yanagisawa, SIAM
-//     J. Sci. Comput. 42 (2020) -- resolves five decades a stage at this size
-//     and perturbs the columns that need no shift.)
-// The row-wise triangular solve changes A = Q R by O(u |a_j|) per column and
-// stage, so R carries the singular values to the accuracy of a Householder R.
+// The rules of a stage are those of ptt_gramstage.cuh.
 // The host launches MAXST stages; a launch finds the state left by the
 // previous one and returns at once when the factorisation is finished.
 //
@@ -56,24 +33,12 @@
 
 namespace gq {
 
+using namespace gst;
+
 constexpr int NT = 256;
 constexpr int RPB_MIN = 16;
 constexpr int MAXST = 6;               // Gram stages per factorisation
 constexpr int GROUP = 8;               // k_gram: CTAs summed by the first level
-constexpr double TAU = 1e-13;
-constexpr double FIRST = 1e-7;
-constexpr double FIRST_DONE = 1e-8;
-constexpr double U = 1.1102230246251565e-16;
-constexpr double PIV = 1e-13;          // smallest pivot of the equilibrated Gram matrix that is trusted: its
-                                       // relative error is ~1e-15 / PIV, so the next stage sees max|E| ~ 1e-2
-constexpr double DROP = 0.5 * U;       // times sqrt(c): a column's part of A that is rounding noise
-constexpr double SMALL = 1e-280;       // squared norms below this lose digits to underflow: fall back
-
-// A symmetric or upper triangular CB x CB matrix is kept as its upper 8 x 8
-// tiles: tile (I, J), I <= J, is number J (J + 1) / 2 + I (independent of CB,
-// so c columns use the first tiles), entry (i, j) of a tile at tix(i, j).
-// The swizzle puts the four rows of an mma fragment load, and the four
-// columns of a transposed one, in different banks.
 template <int CB>
 struct Cfg {
     static constexpr int NB = CB / 8;
@@ -90,28 +55,12 @@ struct Cfg {
     static constexpr long long O_FAC = 8, O_T = O_FAC + FL, O_AN = O_T + UP, O_TM = O_AN + CB, O_G = O_TM + CB;
     static constexpr long long REC = O_G + UP;
 };
-__device__ __forceinline__ int tix(int i, int j) { return i * 8 + (j ^ ((i & 2) << 1)); }
-__device__ __forceinline__ int tnum(int I, int J) { return (J * (J + 1)) / 2 + I; }
-__device__ __forceinline__ void tile_of(int t, int* I, int* J) {
-    int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-    while ((j + 1) * (j + 2) / 2 <= t) j++;
-    while (j * (j + 1) / 2 > t) j--;
-    *J = j;
-    *I = t - j * (j + 1) / 2;
-}
-__device__ __forceinline__ void mma884(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
 // the Ozaki Gram (ptt_ozaki.cuh): the digit slices take the factor's region
 // and beyond once the rows are solved; its 64 x 65 sum buffer the rows' region
 constexpr size_t SM_ROWS_OZ = sizeof(double) * (size_t)Cfg<64>::RPB_MAX * Cfg<64>::XP + oz::SMEM;
 static_assert(Cfg<64>::RPB_MAX == oz::KMAX, "one CTA's rows are one exact FP32 accumulation");
 static_assert(SM_ROWS_OZ >= Cfg<64>::SM_ROWS && Cfg<64>::RPB_MAX * Cfg<64>::XP >= 64 * 65, "Ozaki buffers");
 static_assert(Cfg<128>::SM_ROWS <= 227 * 1024 && Cfg<128>::SM_DEC <= 227 * 1024, "shared memory");
-
-enum { RUN = 0, DONE = 1, FALLBACK = 2, FINISH = 4, CHOL = 8 };
 
 __host__ __device__ __forceinline__ bool finished(int s) { return s == DONE || s == FINISH; }
 
@@ -153,67 +102,6 @@ __device__ __forceinline__ int rows_taken(int m, int nb) {
 }
 __device__ __forceinline__ bool shape_ok(int m, int c, int cb, const GQ& g) {
     return c <= cb && c >= 1 && m >= c && (long long)m <= (long long)g.rpb * g.nb;
-}
-
-// x <- x R^{-1} for the CTA's rows (h of them, zero rows up to a multiple of
-// 16), one warp per 16 rows, by 8-column blocks in order: the update of block
-// J by the solved blocks, X_J - Y_{<J} R_{<J,J}, on the FP64 tensor cores
-// (two accumulators a tile, so the chain is J products long), then forward
-// substitution in the 8 x 8 diagonal block with one lane per row, the block
-// passed through shared memory: 8 dependent multiply-add pairs, where passing
-// each solved entry between the row's four lanes by shuffles took ~65 cycles
-// an entry.  Rows are independent, so a warp needs no block barrier.  R upper
-// triangular in tiles, iv = inverse pivots, zero beyond c and for a dropped
-// column.
-template <int CB>
-__device__ __forceinline__ void tile_solve(double* Xs, int h, const double* R, const double* iv, int nbc) {
-    constexpr int XP = Cfg<CB>::XP;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int li = lane >> 2, lk = lane & 3;
-    for (int u = warp; u * 16 < h; u += NT / 32) {
-        double* xa = Xs + (u * 16 + li) * XP;  // this lane's fragment rows
-        double* xb = xa + 8 * XP;
-        double* xr = Xs + (u * 16 + (lane & 15)) * XP;
-        for (int J = 0; J < nbc; J++) {
-            const double2 ca = *(const double2*)(xa + 8 * J + 2 * lk);
-            const double2 cb = *(const double2*)(xb + 8 * J + 2 * lk);
-            double a0 = ca.x, a1 = ca.y, b0 = cb.x, b1 = cb.y;
-            double e0 = 0.0, e1 = 0.0, f0 = 0.0, f1 = 0.0;
-            if (J > 0) {
-                for (int I = 0; I < J; I++) {
-                    const double* Rt = R + tnum(I, J) * 64;
-                    const double r0 = Rt[tix(lk, li)], r1 = Rt[tix(lk + 4, li)];
-                    mma884(a0, a1, -xa[8 * I + lk], r0);
-                    mma884(b0, b1, -xb[8 * I + lk], r0);
-                    mma884(e0, e1, -xa[8 * I + 4 + lk], r1);
-                    mma884(f0, f1, -xb[8 * I + 4 + lk], r1);
-                }
-                *(double2*)(xa + 8 * J + 2 * lk) = make_double2(a0 + e0, a1 + e1);
-                *(double2*)(xb + 8 * J + 2 * lk) = make_double2(b0 + f0, b1 + f1);
-                __syncwarp();
-            }
-            if (lane < 16) {
-                const double* Rd = R + tnum(J, J) * 64;
-                double x[8];
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const double2 v = *(const double2*)(xr + 8 * J + j);
-                    x[j] = v.x;
-                    x[j + 1] = v.y;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const double y = x[j] * iv[8 * J + j];
-                    x[j] = y;
-#pragma unroll
-                    for (int l = j + 1; l < 8; l++) x[l] = fma(-y, Rd[tix(j, l)], x[l]);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) *(double2*)(xr + 8 * J + j) = make_double2(x[j], x[j + 1]);
-            }
-            __syncwarp();
-        }
-    }
 }
 
 // Partial Gram matrix of the CTA's rows on the FP64 tensor cores
@@ -425,7 +313,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_rows(const DevDesc* D, int k, int 
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     if (stage > 0) {
-        tile_solve<CB>(Xs, h, sF, sF + C::UP, nbc);
+        tile_solve<XP, NT / 32>(Xs, h, sF, sF + C::UP, nbc);
         __syncthreads();
         if (Qv.rs == 1) {  // column-major, in the load's 4 x 8 warp tiles
             const int nrb = (h + 3) / 4, ncb = (c + 7) / 8;
@@ -474,46 +362,9 @@ __device__ void chol_tiles(double* sG, int nbc, int c, const unsigned char* aliv
     for (int J = 0; J < nbc; J++) {
         double r[8][8], inv[8];
         const int col = 8 * J + 8 + tid;  // this thread's column of the block row
-        const unsigned live = alive[J];
         if (tid < CB) {
-            const double* G = sG + tnum(J, J) * 64;
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = i; j < 8; j++) r[i][j] = G[tix(i, j)];
-            unsigned weak = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const bool on = (live >> j) & 1u;
-                const double p = r[j][j];
-                const bool good = p > PIV;  // false for NaN
-                const double pp = good ? p : PIV;
-                const double iv = on ? rsqrt(pp) : 0.0;
-                const double io = good ? iv : 0.0;
-                r[j][j] = on ? pp * iv : 0.0;
-                inv[j] = iv;
-                if (!(on && good)) weak |= 1u << j;
-#pragma unroll
-                for (int l = j + 1; l < 8; l++) r[j][l] *= io;
-#pragma unroll
-                for (int i = j + 1; i < 8; i++)
-#pragma unroll
-                    for (int l = i; l < 8; l++) r[i][l] = fma(-r[j][i], r[j][l], r[i][l]);
-            }
-            if (col < 8 * nbc) {
-                double* Gc = sG + tnum(J, col >> 3) * 64;
-                double y[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) y[i] = Gc[tix(i, col & 7)];
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    y[i] = ((weak >> i) & 1u) ? 0.0 : y[i] * inv[i];
-#pragma unroll
-                    for (int l = i + 1; l < 8; l++) y[l] = fma(-r[i][l], y[i], y[l]);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i++) Gc[tix(i, col & 7)] = y[i];
-            }
+            const unsigned weak = chol8(sG + tnum(J, J) * 64, alive[J], r, inv);
+            if (col < 8 * nbc) solve8(sG + tnum(J, col >> 3) * 64, col & 7, r, inv, weak);
         }
         __syncthreads();
         if (tid == 0) {  // the diagonal block, read by every panel thread until the barrier
@@ -529,15 +380,7 @@ __device__ void chol_tiles(double* sG, int nbc, int c, const unsigned char* aliv
         for (int t = warp; t < n * (n + 1) / 2; t += NT / 32) {
             int I, K;
             tile_of(t, &I, &K);
-            I += J + 1;
-            K += J + 1;
-            const double* Ra = sG + tnum(J, I) * 64;
-            const double* Rb = sG + tnum(J, K) * 64;
-            double2* Ct = (double2*)(sG + tnum(I, K) * 64 + tix(li, 2 * lk));
-            double2 v = *Ct;
-            mma884(v.x, v.y, -Ra[tix(lk, li)], Rb[tix(lk, li)]);
-            mma884(v.x, v.y, -Ra[tix(lk + 4, li)], Rb[tix(lk + 4, li)]);
-            *Ct = v;
+            trail8(sG, J, I + J + 1, K + J + 1, li, lk);
         }
         __syncthreads();
     }
@@ -642,7 +485,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
         s_d[j] = on ? dj : 0.0;
         s_di[j] = on ? 1.0 / dj : 0.0;
         s_tm[j] = 0ull;
-        if (j < c && !(gjj >= 0.0 && gjj < 1e300)) atomicOr(&s_flags, 1);      // NaN, Inf or near overflow
+        if (j < c && !(gjj >= 0.0 && gjj < LARGE)) atomicOr(&s_flags, 1);      // NaN, Inf or near overflow
         if (j < c && gjj != 0.0 && gjj < SMALL) atomicOr(&s_flags, 1);
         const unsigned bits = __ballot_sync(0xffffffffu, on);
         if ((lane & 7) == 0) s_alive[j >> 3] = (unsigned char)((bits >> lane) & 0xffu);
@@ -729,14 +572,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
             if (stage == 0) {
                 v = *(const double2*)(sG + t * 64 + tix(li, 2 * lk));
             } else {
-                double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-                for (int K = I; K <= J; K++) {
-                    const double* Fk = sG + tnum(I, K) * 64;
-                    const double* Tk = sT + tnum(K, J) * 64;
-                    mma884(a0, a1, Fk[tix(li, lk)], Tk[tix(lk, li)]);
-                    mma884(b0, b1, Fk[tix(li, lk + 4)], Tk[tix(lk + 4, li)]);
-                }
-                v = make_double2(a0 + b0, a1 + b1);
+                v = tile_product(sG, sT, I, J, li, lk);
             }
             *(double2*)(T + t * 64 + tix(li, 2 * lk)) = v;
             const int i = 8 * I + li, j = 8 * J + 2 * lk;

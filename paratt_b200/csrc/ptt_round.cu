@@ -505,6 +505,7 @@ __global__ void k_bond_finalize(DevDesc* D, int kq, int ka, int kb, const int* v
 }
 
 #include "ptt_wtsqr.cuh"
+#include "ptt_gramstage.cuh"
 #include "ptt_cholqr.cuh"
 #include "ptt_gridqr.cuh"
 
