@@ -66,6 +66,22 @@ __device__ __forceinline__ FiberIter fiber_iter(int R) {
     return it;
 }
 
+// Walk of a core by runs of JRUN consecutive fibers of one slab l, one warp
+// per run: one division per run instead of one per fiber, and the next
+// fiber's addresses by addition.
+constexpr int JRUN = 16;
+struct RunIter {
+    int t, step, runs, total;  // run t of `runs` per slab
+};
+__device__ __forceinline__ RunIter run_iter(int n, int slabs) {
+    RunIter it;
+    it.t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    it.step = (int)(((long long)gridDim.x * blockDim.x) >> 5);
+    it.runs = (n + JRUN - 1) / JRUN;
+    it.total = it.runs * slabs;
+    return it;
+}
+
 // Blocks per core of a fiber launch over d cores (grid y = core): enough for
 // the largest core's fibers at 8 per block (one per warp of 256 threads),
 // capped at 32 blocks per SM over the whole grid.
@@ -242,6 +258,30 @@ __global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* 
     const double* xc = X->core[k];
     const double* yc = Y->core[k];
     double* zc = Z->alt[k];
+    if ((rz & 1) == 0 && rz >= 32) {
+        // A warp walks runs of fibers (j, lz), lz = ly + ry1 jx; lane: rows iz =
+        // 2 lane + 64 b and the next, iz = ky + ry ix, so the row's factors are
+        // found once and every store is 16 bytes.  Bound by the writes (8 bytes
+        // per element; x and y come from L1/L2): d = 40, n = 256, ranks 8 x 8, 336
+        // MB: 144 us with a division and an 8-byte store per element, 58 now.
+        const RunIter it = run_iter(n, rz1);
+        const int lane = threadIdx.x & 31;
+        for (int b = 2 * lane; b < rz; b += 64) {
+            const int i0 = b / ry, k0 = b - i0 * ry, i1 = (b + 1) / ry, k1 = (b + 1) - i1 * ry;
+            for (int t = it.t; t < it.total; t += it.step) {
+                const int lz = t / it.runs, j0 = (t - lz * it.runs) * JRUN, h = min(JRUN, n - j0);
+                const int jx = lz / ry1, ly = lz - jx * ry1;
+                const double* xf = xc + (long long)rx * (j0 + (long long)n * jx);
+                const double* yf = yc + (long long)ry * (j0 + (long long)n * ly);
+                double2* zf = (double2*)(zc + (long long)rz * (j0 + (long long)n * lz) + b);
+#pragma unroll 4
+                for (int j = 0; j < h; j++)
+                    __stcs(zf + (long long)(rz / 2) * j, make_double2(xf[rx * j + i0] * yf[ry * j + k0],
+                                                                      xf[rx * j + i1] * yf[ry * j + k1]));
+            }
+        }
+        return;
+    }
     // fiber (j, lz), lz = ly + ry1 jx: rows iz = ky + ry ix
     const int NF = n * rz1;
     const FiberIter it = fiber_iter(rz);
@@ -481,6 +521,42 @@ __global__ void k_opsum(const DevDesc* X, DevDesc* Y, Stencil st, double shift, 
     }
     const double* xc = X->core[k];
     double* yc = Y->alt[k];
+    if (d > 1 && k > 0 && k < d - 1 && (r & 1) == 0 && r >= 32 && st.len == 3) {
+        // A middle core: a warp walks runs of fibers (j, l') of x and writes both
+        // of y's fibers that come from each, [x; 0] and [S x; x]; the three-point
+        // stencil slides along the run in registers, so every fiber of x is read
+        // once (plus two per run) and all accesses are 16 bytes.  Bound by HBM,
+        // four bytes written per byte read: d = 40, n = 256, r = 64, 1.68 GB: 504
+        // us with 8-byte accesses, a division per fiber and the stencil's
+        // neighbours re-read, 280 now (6.0 TB/s).
+        const RunIter it = run_iter(n, r1);
+        const int lane = threadIdx.x & 31;
+        const double s0 = st.s[0], s1 = st.s[1], s2 = st.s[2];
+        for (int b = 2 * lane; b < r; b += 64) {
+            for (int t = it.t; t < it.total; t += it.step) {
+                const int l = t / it.runs, j0 = (t - l * it.runs) * JRUN, h = min(JRUN, n - j0);
+                const double2* xs = (const double2*)(xc + (long long)r * n * l + b);  // fiber j at xs[j r / 2]
+                const int r2 = r >> 1;
+                double2* ya = (double2*)(yc + (long long)ry * (j0 + (long long)n * l) + b);
+                double2* yb = ya + (long long)r * n * r1;  // the fiber l + r1
+                double2 xm = __ldg(xs + (long long)r2 * (j0 > 0 ? j0 - 1 : n - 1)), x0 = __ldg(xs + (long long)r2 * j0);
+#pragma unroll 4
+                for (int j = 0; j < h; j++) {
+                    const int jn = j0 + j + 1 < n ? j0 + j + 1 : 0;
+                    const double2 xp = __ldg(xs + (long long)r2 * jn);
+                    const double2 sx = make_double2(fma(s2, xp.x, fma(s1, x0.x, fma(s0, xm.x, 0.0))),
+                                                    fma(s2, xp.y, fma(s1, x0.y, fma(s0, xm.y, 0.0))));
+                    __stcs(ya + (long long)r * j, x0);
+                    __stcs(ya + (long long)r * j + r2, make_double2(0.0, 0.0));
+                    __stcs(yb + (long long)r * j, sx);
+                    __stcs(yb + (long long)r * j + r2, x0);
+                    xm = x0;
+                    x0 = xp;
+                }
+            }
+        }
+        return;
+    }
     // fiber (j, l) of y; l' = l - r1 for the second block column
     const int NF = n * ry1;
     const FiberIter it = fiber_iter(ry);
