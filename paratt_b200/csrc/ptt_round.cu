@@ -258,9 +258,10 @@ __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, in
     if (info->status) return;
     const int q = info->q, sweeps = info->sweeps, rank = info->rank, order = info->order;
     // pairs and steps of a sweep: two pairs for each of the G groups
-    const int Gc = (q + 3) >> 2;
+    const int qa = info->qa, Gc = qa > 4 ? (qa + 3) >> 2 : 1;
     const int G = order == ORD_RING ? (Gc > 1 ? 1 << (32 - __clz(Gc - 1)) : 1) : Gc;
     const int npr = 2 * G, nrd = 4 * G - 1;
+    const int* perm = (const int*)(ws + pl.o_sig + CT) + CT;
     // the column pair of every (step, pair) slot, once for all sweeps
     unsigned char* pcol = (unsigned char*)(tab + (CT + 1) * npair);
     unsigned char* qcol = pcol + (CT + 1) * npair;
@@ -268,8 +269,9 @@ __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, in
         const int rd = e / npr, i = e - (e / npr) * npr;
         int pc, qc;
         svd_pair(i, rd, G, order, &pc, &qc);
-        pcol[rd * npair + i] = (unsigned char)pc;
-        qcol[rd * npair + i] = (unsigned char)qc;
+        // slots of the log to columns of V; beyond qa (never rotated): CT
+        pcol[rd * npair + i] = (unsigned char)(pc < qa ? perm[pc] : CT);
+        qcol[rd * npair + i] = (unsigned char)(qc < qa ? perm[qc] : CT);
     }
     for (int j = lane; j < SR; j += 32) vrow[j] = (j == row) ? 1.0 : 0.0;
     const double2* rot = (const double2*)(ws + pl.o_rot);

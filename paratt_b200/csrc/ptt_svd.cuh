@@ -31,6 +31,12 @@
 //     largest column norm of about one, so the single-precision values do not
 //     overflow;
 //   * a warp whose pairs are all orthogonal already skips the application.
+//
+// The figures of a bond's SVD against the kernels before (columns in shared
+// memory, or one column per group moved by shuffles, FP64 reciprocal square
+// roots on the chain): 20 columns 81 -> 50 us, 64 columns of a rank-32 sum 283 ->
+// 133 us (99 where half of them are noise), 95 columns with a spectrum of 2^-j
+// 531 -> 130 us, 14 columns of a time step 31 -> 20.
 #pragma once
 
 constexpr int MAXSW = 40;  // Jacobi sweep limit
@@ -169,7 +175,6 @@ __device__ __forceinline__ double dot_rows(const double (&x)[NR], const double (
 }
 
 // RB bounds c and q (a multiple of 16; RB / 4 groups).
-// One step at 20 / 64 / 95 columns: see the figures at launch_svd.
 template <int RB>
 __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double* ws, double delta, int maxr, int bond,
                                                                 int* status) {
@@ -182,7 +187,8 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
     double2* xch = (double2*)sm;
     __shared__ double2 s_xn[NBUF][NBLK];  // norms of the moving blocks
     __shared__ double s_sig[RB], s_srt[RB], s_suf[RB];
-    __shared__ int s_ord[RB];
+    __shared__ double s_nrm[RB];
+    __shared__ int s_ord[RB], s_perm[RB], s_slot[RB];
     __shared__ int s_rot, s_rank;
     __shared__ double s_wmax[NW > 0 ? NW : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -194,27 +200,8 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
         if (tid == 0) PTT_STATUS_SET(status, PTT_ERR_CAPACITY);
         return;
     }
-    // the stationary ring where its power-of-two block count costs at most 15 %
-    // more steps than the circle: it takes one sweep in eight less (8.5 against
-    // 9.7 at 64 columns, 6.3 against 6.7 at 32) and moves half as many blocks
-    const int Gc = (q + 3) >> 2;                                // groups of the circle order
-    const int Gr = Gc > 1 ? 1 << (32 - __clz(Gc - 1)) : 1;      // of the ring order
-    const bool ring = 4 * Gr <= RB && 20 * (4 * Gr - 1) <= 23 * (4 * Gc - 1);
-    const int G = ring ? Gr : Gc, ns = 2 * G - 1;
-    const bool act = grp < G;
-    // columns of this group: blocks grp and G + grp (ring) or 2 G - 1 - grp (circle)
-    const int ja = 2 * grp, jb = 2 * (ring ? G + grp : 2 * G - 1 - grp);
     const double* R = ws + pl.o_Rn;  // root factor, row-major CT x CT; L = R^T: column j of L = row j of R
     double A0[NR], A1[NR], B0[NR], B1[NR];
-#pragma unroll
-    for (int v = 0; v < NR; v++) {
-        const int t = p + LP * v;
-        const bool in = act && t < c;
-        A0[v] = (in && ja < q) ? R[(long long)ja * CT + t] : 0.0;
-        A1[v] = (in && ja + 1 < q) ? R[(long long)(ja + 1) * CT + t] : 0.0;
-        B0[v] = (in && jb < q) ? R[(long long)jb * CT + t] : 0.0;
-        B1[v] = (in && jb + 1 < q) ? R[(long long)(jb + 1) * CT + t] : 0.0;
-    }
     auto gsum = [&](double v) {
 #pragma unroll
         for (int o = LP / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
@@ -227,6 +214,84 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
             __syncwarp();
     };
     double a0, a1, b0, b1;  // squared norms of the group's columns
+    // The columns as they come (group g: 4 g .. 4 g + 3), their norms, and from
+    // them the columns that take part.  Columns below the numerical-rank
+    // threshold (sqrt(q) eps_LAPACK times the largest column norm) are
+    // rounding noise: rotating noise against noise is a random walk that never
+    // meets the relative criterion, and their values are discarded by the rank
+    // rule anyway, so they are left alone -- and, since the largest norm only
+    // grows, for good: the sweeps run over the qa others alone (half of 64 in
+    // the truncation of a rank-32 sum, 50 of 95 in a spectrum of 2^-j).
+#pragma unroll
+    for (int v = 0; v < NR; v++) {
+        const int t = p + LP * v, j = 4 * grp;
+        A0[v] = (t < c && j < q) ? R[(long long)j * CT + t] : 0.0;
+        A1[v] = (t < c && j + 1 < q) ? R[(long long)(j + 1) * CT + t] : 0.0;
+        B0[v] = (t < c && j + 2 < q) ? R[(long long)(j + 2) * CT + t] : 0.0;
+        B1[v] = (t < c && j + 3 < q) ? R[(long long)(j + 3) * CT + t] : 0.0;
+    }
+    a0 = gsum(dot_rows(A0, A0));
+    a1 = gsum(dot_rows(A1, A1));
+    b0 = gsum(dot_rows(B0, B0));
+    b1 = gsum(dot_rows(B1, B1));
+    if (p < 4) s_nrm[4 * grp + p] = p == 0 ? a0 : (p == 1 ? a1 : (p == 2 ? b0 : b1));
+#pragma unroll
+    for (int v = 0; v < NR; v++) {
+        const int t = p + LP * v, j = 4 * grp;
+        Lc[j * S + t] = A0[v];
+        Lc[(j + 1) * S + t] = A1[v];
+        Lc[(j + 2) * S + t] = B0[v];
+        Lc[(j + 3) * S + t] = B1[v];
+    }
+    if (tid == 0) s_rot = 0;
+    sync();
+    double mx = 0.0;
+    int qa = 0;
+    {
+        for (int j = lane; j < RB; j += 32) mx = fmax(mx, s_nrm[j]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
+        const int thr = __double2hiint((double)q * 1.232595164407831e-32 * mx);  // (sqrt(q) * 2^-53)^2 * max |a_j|^2
+        for (int j0 = 0; j0 < RB; j0 += 32) {
+            const int j = j0 + lane;
+            const bool in = j < RB && j < q && s_nrm[j < RB ? j : 0] > 0.0 && __double2hiint(s_nrm[j < RB ? j : 0]) > thr;
+            const unsigned m = __ballot_sync(FULL, in);
+            const int at = qa + __popc(m & ((1u << lane) - 1u));
+            if (warp == 0 && j < RB) {
+                s_slot[j] = in ? at : -1;
+                if (in) s_perm[at] = j;
+            }
+            qa += __popc(m);
+        }
+    }
+    // the stationary ring where its power-of-two block count costs at most 15 %
+    // more steps than the circle: it takes one sweep in eight less (8.5 against
+    // 9.7 at 64 columns, 6.3 against 6.7 at 32) and moves half as many blocks
+    const int Gc = qa > 4 ? (qa + 3) >> 2 : 1;                  // groups of the circle order
+    const int Gr = Gc > 1 ? 1 << (32 - __clz(Gc - 1)) : 1;      // of the ring order
+    const bool ring = 4 * Gr <= RB && 20 * (4 * Gr - 1) <= 23 * (4 * Gc - 1);
+    const int G = ring ? Gr : Gc, ns = 2 * G - 1;
+    const bool act = grp < G;
+    // slots of this group: blocks grp and G + grp (ring) or 2 G - 1 - grp (circle)
+    const int ja = 2 * grp, jb = 2 * (ring ? G + grp : 2 * G - 1 - grp);
+    int sh = 0;  // L is held as 2^-sh L
+    if (mx > 0.0 && mx < 1.0 / 0.0) sh = ilogb(mx) >> 1;
+    const double down = scalbn(1.0, -sh);
+    sync();
+    if (act) {
+        auto fetch = [&](int slot, double(&x)[NR]) {
+            const double* col = Lc + s_perm[slot < qa ? slot : 0] * S;
+#pragma unroll
+            for (int v = 0; v < NR; v++) x[v] = slot < qa ? col[p + LP * v] * down : 0.0;
+        };
+        if (qa > 0) {
+            fetch(ja, A0);
+            fetch(ja + 1, A1);
+            fetch(jb, B0);
+            fetch(jb + 1, B1);
+        }
+    }
+    sync();  // the moving blocks take the columns' place
     // exact norms of all columns; returns the largest
     auto norms = [&]() {
         a0 = gsum(dot_rows(A0, A0));
@@ -248,32 +313,9 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
     const int npair = (CT + 2) / 2;
     const double tol = (double)(c < 16 ? 16 : c) * 2.220446049250313e-16;
     const double tol2 = tol * tol;  // |ga| > tol sqrt(al be), compared in squares
-    int sh = 0;                     // L is held as 2^-sh L
     int sweeps = 0;
-    bool conv = q < 2;
-    double mx = 0.0;
-    if (!conv) {
-        mx = norms();
-        if (mx > 0.0 && mx < 1.0 / 0.0) sh = ilogb(mx) >> 1;
-        if (sh != 0) {
-            const double f = scalbn(1.0, -sh);
-#pragma unroll
-            for (int v = 0; v < NR; v++) {
-                A0[v] *= f;
-                A1[v] *= f;
-                B0[v] *= f;
-                B1[v] *= f;
-            }
-        }
-        if (tid == 0) s_rot = 0;
-        if (NW > 1) __syncthreads();
-    }
+    bool conv = qa < 2;
     for (int sw = 0; sw < MAXSW && !conv; sw++) {
-        // Columns below the numerical-rank threshold (sqrt(q) eps_LAPACK times
-        // the largest column norm) are rounding noise: rotating noise against
-        // noise is a random walk that never meets the relative criterion, and
-        // their values are discarded by the rank rule anyway, so pairs with
-        // such a column are left alone.
         mx = norms();
         // (sqrt(q) * 2^-53)^2 * max |a_j|^2, compared by the high words
         const int thr = __double2hiint((double)q * 1.232595164407831e-32 * mx);
@@ -441,23 +483,34 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
     b0 = gsum(dot_rows(B0, B0));
     b1 = gsum(dot_rows(B1, B1));
     if (act) {
+        auto store = [&](int slot, const double(&x)[NR]) {
+            if (slot >= qa) return;
+            double* col = Lc + s_perm[slot] * S;
 #pragma unroll
-        for (int v = 0; v < NR; v++) {
-            const int t = p + LP * v;
-            Lc[ja * S + t] = A0[v];
-            Lc[(ja + 1) * S + t] = A1[v];
-            Lc[jb * S + t] = B0[v];
-            Lc[(jb + 1) * S + t] = B1[v];
-        }
+            for (int v = 0; v < NR; v++) col[p + LP * v] = x[v];
+        };
+        store(ja, A0);
+        store(ja + 1, A1);
+        store(jb, B0);
+        store(jb + 1, B1);
         if (p < 4) {  // lane p: one of the four columns
-            const int j = (p & 2 ? jb : ja) + (p & 1);
+            const int slot = (p & 2 ? jb : ja) + (p & 1);
             const double s2 = p == 0 ? a0 : (p == 1 ? a1 : (p == 2 ? b0 : b1));
-            // a NaN (corrupt input) would break the strict order below and leave
-            // order slots unset; it sorts last and is reported instead
-            const bool nan = !(s2 == s2);
-            if (nan && j < q) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
-            s_sig[j] = (j < q && !nan) ? sqrt(s2) * back : -1.0;
+            if (slot < qa) s_nrm[s_perm[slot]] = s2;
         }
+    }
+    for (int j = warp; j < q; j += NW) {  // the columns that took no part
+        if (s_slot[j] < 0)
+            for (int t = lane; t < c; t += 32) Lc[j * S + t] = R[(long long)j * CT + t] * down;
+    }
+    __syncthreads();
+    for (int j = tid; j < q; j += NTH) {
+        const double s2 = s_nrm[j];
+        // a NaN (corrupt input) would break the strict order below and leave
+        // order slots unset; it sorts last and is reported instead
+        const bool nan = !(s2 == s2);
+        if (nan) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
+        s_sig[j] = nan ? -1.0 : sqrt(s2) * (s_slot[j] < 0 ? 1.0 : back);
     }
     __syncthreads();
     for (int j = tid; j < q; j += NTH) {  // descending order
@@ -514,6 +567,7 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
             info->nsv = nsv;
             info->sweeps = sweeps;
             info->order = ring ? ORD_RING : ORD_CIRCLE;
+            info->qa = qa;
             info->tail = tail;
             if (pl.stats) {
                 double* st = pl.stats + (long long)bond * PTT_STAT_LEN;
@@ -532,7 +586,9 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
     }
     for (int j = tid; j < CT; j += NTH) {
         sig_out[j] = j < q ? s_srt[j] : 0.0;
-        ((int*)(sig_out + CT))[j] = j < q ? s_ord[j] : 0;
+        int* ord = (int*)(sig_out + CT);
+        ord[j] = j < q ? s_ord[j] : 0;
+        ord[CT + j] = j < qa ? s_perm[j] : CT;  // slot of the rotation log -> column (CT: none)
     }
     __syncthreads();
     const int rank = s_rank;

@@ -63,6 +63,7 @@ struct Info {
     int status;
     int order;        // Jacobi pair order of the recorded rotations (ORD_*, ptt_svd.cuh)
     double tail;      // retained tail sum (diagnostic)
+    int qa;           // columns the Jacobi rotated (slots of the rotation log)
 };
 
 // Workspace layout, computed on the host (identical formula in kernels).
