@@ -42,6 +42,8 @@ using namespace gst;
 constexpr int NT = 256;       // threads per CTA
 constexpr int MAXST = 7;      // Gram stages per factorisation
 constexpr int CSMAX = 16;     // CTAs per cluster (non-portable size)
+constexpr double TAUC = 1e-15;  // as gst::TAU: a cluster's first-order finish costs one more row solve (~1 us), so
+                                // it is taken down to the rounding of G itself
 constexpr int RTARGET = 64;   // rows per CTA the cluster size aims at: every part but the two barriers shrinks
                               // with the rows (m = 1280, c = 20: 31 us with 4 CTAs, 27 with 16)
 static_assert(DONE == wt::CQ_DONE, "state code shared with the TSQR kernels");
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
         ndrop = c - __popc(live);
         if (live == 0u) {
             dec = FALLBACK;
-        } else if (stage >= 1 && emax <= TAU) {
+        } else if (stage >= 1 && emax <= TAUC) {
             dec = DONE;
         } else if (stage == MAXST - 1) {
             dec = FALLBACK;

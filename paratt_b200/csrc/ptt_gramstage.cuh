@@ -32,7 +32,7 @@
 
 namespace gst {
 
-constexpr double TAU = 1e-13;
+constexpr double TAU = 1e-14;
 constexpr double FIRST = 1e-7;
 constexpr double FIRST_DONE = 1e-8;
 constexpr double U = 1.1102230246251565e-16;

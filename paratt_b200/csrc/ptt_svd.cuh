@@ -136,7 +136,7 @@ __device__ __forceinline__ double widen(float f, bool on) {
 // theta = sqrt((1 + cos 2theta) / 2), tan theta = sin 2theta / (1 + cos
 // 2theta) -- dd and ga scaled by the exponent of max(al, be).
 struct Pre {
-    double lim, lim8;  // squares of tol and of 1e-8, times al be
+    double lim, lim9;  // squares of tol and of 1e-9, times al be
     float ds;          // dd, scaled
     int E;             // exponent field of max(al, be)
     bool big;
@@ -149,7 +149,7 @@ __device__ __forceinline__ Pre svd_pre(double al, double be, int thr, double tol
     r.ds = scaled_float(be - al, r.E);
     const double ab = al * be;
     r.lim = tol2 * ab;
-    r.lim8 = 1e-16 * ab;
+    r.lim9 = 1e-18 * ab;
     return r;
 }
 __device__ __forceinline__ void svd_angle(const Pre& r, double ga, bool on, double* t, double* cs) {
@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
                 ny0 = fma(t0, g0, ny0);
                 nx1 = fma(-t1, g1, nx1);
                 ny1 = fma(t1, g1, ny1);
-                // bit 1: a rotation of a pair whose cosine exceeded 1e-8
-                myrot |= (on0 ? (q0 > r0.lim8 ? 3 : 1) : 0) | (on1 ? (q1 > r1.lim8 ? 3 : 1) : 0);
+                // bit 1: a rotation of a pair whose cosine exceeded 1e-9
+                myrot |= (on0 ? (q0 > r0.lim9 ? 3 : 1) : 0) | (on1 ? (q1 > r1.lim9 ? 3 : 1) : 0);
             }
             if (p == 0 && act) {
                 lg[0] = make_double2(c0, t0);
@@ -469,8 +469,8 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
         } else {
             sweeps = sw + 1;
             // cyclic Jacobi converges quadratically at the end: after a sweep
-            // whose cosines all stayed below 1e-8 the next one would only
-            // meet cosines ~1e-15 (the single-precision angles leave 1e-7 of
+            // whose cosines all stayed below 1e-9 the next one would only
+            // meet cosines ~1e-16 (the single-precision angles leave 1e-7 of
             // each), so it is not run
             if (!(any & 2)) conv = true;
         }
