@@ -85,79 +85,28 @@ __device__ void replay_geqrt(double* Rp, const double* Vb, const double* taus, i
     }
 }
 
+// out = Q B for the Householder tree: block (p, y) takes leaf p and 32 columns
+// of B and walks from the root down to its leaf, replaying the reflectors of
+// each node on its own copy of the node's rows in shared memory (the left
+// child takes the triangle's rows, the right child the eliminated ones), then
+// those of its leaf.  B is V_r at the root slot (RIGHT_T) or the identity
+// (LEFT).  The depth of the chain is that of one launch per level; the upper
+// nodes are replayed once per leaf below them, on SMs the level launches left
+// idle.  One launch instead of one for B, one per level and one for the
+// leaves: behind the grid Cholesky QR it is nearly always skipped, and then
+// its launches are all it costs (at 16384 x 64 seven of 1.0 us each, and 2 to
+// 5 us each of a lane's time in a batch; 64 trains of ranks to 96: 64.1 ms
+// with them, 58.1 without).
+// LEFT: out(row, col) at alt[row + m*col];  RIGHT_T: alt[row*k + col]
 template <int CT>
-__global__ void __launch_bounds__(NT) k_apply_node(Plan pl, double* ws, int first, const int* kptr) {
-    PTT_PDL_ENTRY();
-    if (gq_finished(pl)) return;
-    extern __shared__ double sm[];
-    constexpr int S = CT + 1;
-    double* Rp = sm;             // CT x KG
-    double* Vs = Rp + CT * KG;   // H x S
-    const int node = first + blockIdx.x;
-    const int kg0 = blockIdx.y * KG;
-    const int kk = *kptr;
-    if (pl.info->status || kg0 >= kk) return;
-    const int q = pl.qn[node];
-    if (q == 0) return;
-    const int tid = threadIdx.x, col = tid >> 3, part = tid & 7;
-    const int c = pl.info->c;
-    const int KC = pl.KC;
-    double* Bn = ws + pl.o_Bn;
-    const double* Bi = Bn + (long long)node * CT * KC;
-    const int cl = 2 * node + 1, cr = 2 * node + 2;
-    const int ps = pl.pass[node];
-    if (ps == 1 || ps == 2) {
-        double* Bo = Bn + (long long)(ps == 1 ? cl : cr) * CT * KC;
-        for (int e = tid; e < CT * KG; e += NT) {
-            const int a = e / KG, b = e - (e / KG) * KG;
-            Bo[(long long)a * KC + kg0 + b] = Bi[(long long)a * KC + kg0 + b];
-        }
-        return;
-    }
-    if (ps != 0) return;
-    for (int e = tid; e < CT * KG; e += NT) {
-        const int a = e / KG, b = e - (e / KG) * KG;
-        Rp[e] = Bi[(long long)a * KC + kg0 + b];
-    }
-    const double* RR = ws + pl.o_Rn + (long long)cr * CT * CT;
-    double* Bcr = Bn + (long long)cr * CT * KC;
-    for (int half = pl.NH - 1; half >= 0; half--) {
-        const int h0 = half * H;
-        if (h0 >= c) continue;
-        __syncthreads();
-        for (int e = tid; e < H * CT; e += NT) {
-            const int t = e / CT, l = e - (e / CT) * CT;
-            Vs[t * S + l] = (h0 + t < c) ? RR[(long long)(h0 + t) * CT + l] : 0.0;
-        }
-        __syncthreads();
-        double out[H / 8];
-#pragma unroll
-        for (int v = 0; v < H / 8; v++) out[v] = 0.0;
-        const double* taus = ws + pl.o_tau_node + ((long long)node * pl.NH + half) * CT;
-        replay_tsqrt<CT>(Rp, Vs, taus, c, out, col, part);
-#pragma unroll
-        for (int v = 0; v < H / 8; v++) {
-            const int t = h0 + part + 8 * v;
-            if (t < CT) Bcr[(long long)t * KC + kg0 + col] = out[v];
-        }
-    }
-    __syncthreads();
-    double* Bcl = Bn + (long long)cl * CT * KC;
-    for (int e = tid; e < CT * KG; e += NT) {
-        const int a = e / KG, b = e - (e / KG) * KG;
-        Bcl[(long long)a * KC + kg0 + b] = Rp[e];
-    }
-}
-
-// out_mode LEFT: out(row, col) at alt[row + m*col];  RIGHT_T: alt[row*k + col]
-template <int CT>
-__global__ void __launch_bounds__(NT) k_apply_leaf(const DevDesc* D, int kcore, int mode, Plan pl, double* ws,
-                                                   const int* kptr) {
+__global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int mode, Plan pl, double* ws,
+                                              const int* kptr) {
     PTT_PDL_ENTRY();
     if (gq_finished(pl)) return;
     extern __shared__ double sm[];
     constexpr int S = CT + 1;
     constexpr int VR = CT > H ? CT : H;
+    constexpr int NHC = (CT + H - 1) / H;  // chunks of a node
     double* Rp = sm;             // CT x KG
     double* Vs = Rp + CT * KG;   // VR x S
     const int p = blockIdx.x;
@@ -165,7 +114,7 @@ __global__ void __launch_bounds__(NT) k_apply_leaf(const DevDesc* D, int kcore, 
     const int kk = *kptr;
     if (pl.info->status || kg0 >= kk) return;
     const int tid = threadIdx.x, col = tid >> 3, part = tid & 7;
-    const int m = pl.info->m, c = pl.info->c;
+    const int m = pl.info->m, c = pl.info->c, q = pl.info->q;
     // the unfolding the factorisation recorded (m x c), not the descriptor's
     // ranks: in the truncation sweep this runs on the side stream while the
     // main stream has already published the bond's new rank
@@ -184,13 +133,44 @@ __global__ void __launch_bounds__(NT) k_apply_leaf(const DevDesc* D, int kcore, 
     if (rows <= 0) return;
     const int rb = rows < c ? rows : c;
     const int slot = pl.P - 1 + p;
-    const int KC = pl.KC;
-    const double* Bi = ws + pl.o_Bn + (long long)slot * CT * KC;
-    const double* tau_leaf = ws + pl.o_tau_leaf + (long long)p * pl.KL * CT;
+    const double* B = ws + pl.o_Bn;  // V_r, CT x KC
     for (int e = tid; e < CT * KG; e += NT) {
-        const int a = e / KG, b = e - (e / KG) * KG;
-        Rp[e] = Bi[(long long)a * KC + kg0 + b];
+        const int a = e / KG, b = kg0 + e - a * KG;
+        Rp[e] = mode == LEFT ? (a == b && a < q ? 1.0 : 0.0) : B[(long long)a * pl.KC + b];
     }
+    for (int l = 31 - __clz(pl.P); l > 0; l--) {
+        const int node = ((slot + 1) >> l) - 1;                       // ancestor l levels up
+        const bool right = ((((slot + 1) >> (l - 1)) - 1) & 1) == 0;  // its child on the path
+        if (pl.pass[node] != 0) continue;                             // one child without rows: nothing was eliminated
+        const double* RR = ws + pl.o_Rn + (long long)(2 * node + 2) * CT * CT;
+        double out[NHC][H / 8];
+#pragma unroll
+        for (int half = NHC - 1; half >= 0; half--) {
+            const int h0 = half * H;
+#pragma unroll
+            for (int v = 0; v < H / 8; v++) out[half][v] = 0.0;
+            if (h0 >= c) continue;
+            __syncthreads();
+            for (int e = tid; e < H * CT; e += NT) {
+                const int t = e / CT, j = e - (e / CT) * CT;
+                Vs[t * S + j] = (h0 + t < c) ? RR[(long long)(h0 + t) * CT + j] : 0.0;
+            }
+            __syncthreads();
+            replay_tsqrt<CT>(Rp, Vs, ws + pl.o_tau_node + ((long long)node * pl.NH + half) * CT, c, out[half], col,
+                             part);
+        }
+        __syncthreads();
+        if (right) {
+#pragma unroll
+            for (int half = 0; half < NHC; half++)
+#pragma unroll
+                for (int v = 0; v < H / 8; v++) {
+                    const int t = half * H + part + 8 * v;
+                    if (t < CT) Rp[t * KG + col] = out[half][v];
+                }
+        }
+    }
+    const double* tau_leaf = ws + pl.o_tau_leaf + (long long)p * pl.KL * CT;
     const int ocol = kg0 + col;
     const bool colok = ocol < kk;
     const int nch = (rows - rb + H - 1) / H;
@@ -224,19 +204,6 @@ __global__ void __launch_bounds__(NT) k_apply_leaf(const DevDesc* D, int kcore, 
     for (int e = tid; e < CT * KG; e += NT) {
         const int t = e / KG, b = e - (e / KG) * KG;
         if (t < rb && kg0 + b < kk) outp[(long long)(r0 + t) * ors + (long long)(kg0 + b) * ocs] = Rp[e];
-    }
-}
-
-// B = I_q at the root, zero-padded to CT x KC.
-__global__ void k_set_identity(Plan pl, double* ws) {
-    PTT_PDL_ENTRY();
-    if (pl.info->status || gq_finished(pl)) return;
-    const int CT = pl.CT, KC = pl.KC;
-    const int q = pl.info->q;
-    double* B = ws + pl.o_Bn;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < CT * KC; e += gridDim.x * blockDim.x) {
-        const int a = e / KC, b = e - (e / KC) * KC;
-        B[e] = (a == b && a < q) ? 1.0 : 0.0;
     }
 }
 
@@ -394,14 +361,15 @@ __device__ void gemm_tile(GV A, GV B, double* C, long long crs, long long ccs, i
 }
 
 // The bookkeeping that follows a bond's contraction: publish the bond's new
-// rank (D->r[kq] = *val) and swap core[ka] with the buffer just written.
-// With a ticket (a zero-initialised counter) the last block of the
-// contraction does it, so it needs no launch of its own; without one the
-// caller launches k_bond_finalize.
+// rank (D->r[kq] = *val; kq < 0: none) and swap core[ka], and core[kb] unless
+// kb < 0, with the buffers just written.  With a ticket (a zero-initialised
+// counter) the last block of the contraction does it, so it needs no launch of
+// its own; without one the caller launches k_bond_finalize.
 struct Fin {
     int* ticket;
     int kq, ka;
     const int* val;
+    int kb = -1;
 };
 
 __device__ __forceinline__ void fin_last_block(DevDesc* D, const Fin& f, const Info* info) {
@@ -415,10 +383,15 @@ __device__ __forceinline__ void fin_last_block(DevDesc* D, const Fin& f, const I
         *f.ticket = 0;
         __threadfence();
         if (info->status == 0) {
-            D->r[f.kq] = *f.val;
+            if (f.kq >= 0) D->r[f.kq] = *f.val;
             double* t = D->core[f.ka];
             D->core[f.ka] = D->alt[f.ka];
             D->alt[f.ka] = t;
+            if (f.kb >= 0) {
+                t = D->core[f.kb];
+                D->core[f.kb] = D->alt[f.kb];
+                D->alt[f.kb] = t;
+            }
         }
     }
 }
@@ -490,11 +463,11 @@ __global__ void __launch_bounds__(256, 1) k_gemm_xm_oz(DevDesc* D, int im1, Plan
     oz::gemm_tiles<256>(ws + pl.o_US, pl.CT, 1, D->core[im1], M, 1, D->alt[im1], M, rank, M, c, osm, true);
 }
 
-// publish a bond's new rank and swap the two rewritten cores
+// publish a bond's new rank (kq < 0: none) and swap the rewritten cores (kb < 0: one)
 __global__ void k_bond_finalize(DevDesc* D, int kq, int ka, int kb, const int* val, const Info* info) {
     PTT_PDL_ENTRY();
     if (threadIdx.x == 0 && info->status == 0) {
-        D->r[kq] = *val;
+        if (kq >= 0) D->r[kq] = *val;
         double* t = D->core[ka];
         D->core[ka] = D->alt[ka];
         D->alt[ka] = t;
@@ -525,10 +498,9 @@ struct Layout {
     long long bytes;
 };
 
-// pmax bounds the leaves (and so the tree levels, one apply launch each):
-// the Householder TSQR behind the grid Cholesky QR only runs for a bond that
-// falls back, so there it takes few, long leaves and its skipped launches
-// stay few.
+// pmax bounds the leaves (and so the tree levels): the Householder TSQR behind
+// the grid Cholesky QR only runs for a bond that falls back, so there it takes
+// few, long leaves and its skipped launches stay small.
 static void plan_bond(int CT, long long mcap, int KC, Plan* pl, int pmax = 512) {
     int L = 2 * CT;
     if (L < 128) L = 128;
@@ -558,7 +530,7 @@ static long long carve(Plan* pl, int PMAX, int LMAXKL) {
     pl->o_tau_leaf = take((long long)PMAX * LMAXKL * CT);
     pl->o_Rn = take((long long)(2 * PMAX - 1) * CT * CT);
     pl->o_tau_node = take((long long)PMAX * pl->NH * CT);
-    pl->o_Bn = take((long long)(2 * PMAX - 1) * CT * KC);
+    pl->o_Bn = take((long long)CT * KC);
     pl->o_US = take((long long)CT * CT);
     pl->o_rot = take((long long)MAXSW * (CT + 1) * ((CT + 2) / 2) * 2);
     pl->o_sig = take(2LL * CT + 64);
@@ -592,10 +564,7 @@ static int set_attrs() {
     if (ptt_device_done(done, &bit)) return PTT_OK;
     PTT_CUDA(cudaFuncSetAttribute(k_tsqr_factor<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)factor_smem<CT>()));
-    PTT_CUDA(cudaFuncSetAttribute(k_apply_leaf<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)apply_smem<CT>()));
-    PTT_CUDA(cudaFuncSetAttribute(k_apply_node<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)apply_smem<CT>()));
+    PTT_CUDA(cudaFuncSetAttribute(k_apply<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apply_smem<CT>()));
     PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)svd_smem<64>()));
     if constexpr (CT == 128) {
         PTT_CUDA(cudaFuncSetAttribute(k_svd_jacobi<96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -669,19 +638,11 @@ static int launch_factor(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, doubl
     return PTT_OK;
 }
 
-// out = Q * Bn[root]; k columns read from *kptr, at most kcap.
+// out = Q B (k_apply); k columns read from *kptr, at most kcap.
 template <int CT>
 static int launch_apply(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, double* ws, const int* kptr, int kcap) {
-    const int kgroups = (kcap + KG - 1) / KG;
-    int first = 0, cnt = 1;
-    while (first + cnt <= pl.P - 1) {  // internal levels: nodes [first, first+cnt)
-        PTT_CUDA(ptt_launch(c, k_apply_node<CT>, dim3(cnt, kgroups), dim3(NT), apply_smem<CT>(), pl, ws, first, kptr));
-        PTT_LAUNCHED(c);
-        first += cnt;
-        cnt *= 2;
-    }
-    PTT_CUDA(ptt_launch(c, k_apply_leaf<CT>, dim3(pl.P, kgroups), dim3(NT), apply_smem<CT>(), (const DevDesc*)x->dd, k,
-                        mode, pl, ws, kptr));
+    PTT_CUDA(ptt_launch(c, k_apply<CT>, dim3(pl.P, (kcap + KG - 1) / KG), dim3(NT), apply_smem<CT>(),
+                        (const DevDesc*)x->dd, k, mode, pl, ws, kptr));
     PTT_LAUNCHED(c);
     return PTT_OK;
 }
@@ -732,7 +693,9 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     size_t bytes = (size_t)(2 * SLOT) * sizeof(double) + 256;
     if ((rc = ptt_ws_reserve(c, bytes))) return rc;
     const size_t cnt_tree = (size_t)PMAX * 4 + 64;
-    if ((rc = ptt_counters_reserve(c, cnt_tree + 1))) return rc;
+    if ((rc = ptt_counters_reserve(c, cnt_tree + 3))) return rc;
+    int* const tick_main = c->d_counters + cnt_tree + 1;  // Fin tickets: the contractions of the main stream,
+    int* const tick_tail = c->d_counters + cnt_tree + 2;  // and the tails' (one stream each)
     double* const ws0 = (double*)c->ws;
     // ints live after the doubles: qn [2P-1], pass [P], Info
     // Tree counters live alone in ctx->d_counters (zero between launches,
@@ -772,37 +735,47 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         const long long mcap = (long long)rk[i] * x->n[i];
         Plan pl = mkplan(mcap);
         if ((rc = launch_factor<CT>(c, x, i, LEFT, pl, ws, g, mcap))) return rc;
-        PTT_CUDA(ptt_launch(c, k_set_identity, dim3(32), dim3(256), 0, pl, ws));
-        PTT_LAUNCHED(c);
         if ((rc = launch_apply<CT>(c, x, i, LEFT, pl, ws, &info->q, CT))) return rc;
         PTT_CUDA(ptt_launch(c, k_bond_finalize, dim3(1), dim3(32), 0, x->dd, i + 1, i, -1, (const int*)&info->q,
                             (const Info*)info));
         PTT_LAUNCHED(c);
         return PTT_OK;
     }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PTT_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+    const bool ovl = cap == cudaStreamCaptureStatusNone && !c->capturing && !c->lane;
+    // The rank update and swaps ride in the contraction's last block where
+    // launches are plain (a batch's lanes, a capture): one launch less a bond
+    // is 2 to 5 us there.  With programmatic launches a separate
+    // k_bond_finalize costs 1.2 us, the tickets of 256 blocks 1.7.
+    int* const tmain = ovl ? nullptr : tick_main;
+    int* const ttail = ovl ? nullptr : tick_tail;
+    auto finalize = [&](int kq, int ka, int kb, const int* val, const Info* inf) -> int {
+        PTT_CUDA(ptt_launch(c, k_bond_finalize, dim3(1), dim3(32), 0, x->dd, kq, ka, kb, val, inf));
+        PTT_LAUNCHED(c);
+        return PTT_OK;
+    };
     // left-to-right orthogonalisation
     for (int i = 0; i < d - 1 && (phases & 1); i++) {
         const long long mcap = (long long)rk[i] * x->n[i];
         Plan pl = mkplan(mcap);
         if ((rc = launch_factor<CT>(c, x, i, LEFT, pl, ws, g, mcap))) return rc;
-        {
-            const long long ncap = (long long)x->n[i + 1] * rk[i + 2];
-            int gy = (int)((ncap + GT - 1) / GT);
-            if (gy > 4096) gy = 4096;
-            if (c->ozaki && CT <= oz::KG)  // one wave, R split once per CTA
-                PTT_CUDA(ptt_launch(c, k_gemm_rx_oz, dim3(1, gy < c->nsm ? gy : c->nsm), dim3(256), oz::SMEM_GEMM,
-                                    x->dd, i + 1, pl, ws));
-            else
-                PTT_CUDA(ptt_launch(c, k_gemm_rx, dim3((CT + GT - 1) / GT, gy), dim3(256), 0, x->dd, i + 1, pl, ws,
-                                    Fin{}));
-            PTT_LAUNCHED(c);
-        }
-        PTT_CUDA(ptt_launch(c, k_set_identity, dim3(32), dim3(256), 0, pl, ws));
-        PTT_LAUNCHED(c);
         if ((rc = launch_apply<CT>(c, x, i, LEFT, pl, ws, &info->q, CT))) return rc;
-        PTT_CUDA(ptt_launch(c, k_bond_finalize, dim3(1), dim3(32), 0, x->dd, i + 1, i, i + 1, (const int*)&info->q,
-                            (const Info*)info));
-        PTT_LAUNCHED(c);
+        const long long ncap = (long long)x->n[i + 1] * rk[i + 2];
+        int gy = (int)((ncap + GT - 1) / GT);
+        if (gy > 4096) gy = 4096;
+        // then the rank q and the swap of both rewritten cores
+        if (c->ozaki && CT <= oz::KG) {  // one wave, R split once per CTA
+            PTT_CUDA(ptt_launch(c, k_gemm_rx_oz, dim3(1, gy < c->nsm ? gy : c->nsm), dim3(256), oz::SMEM_GEMM,
+                                x->dd, i + 1, pl, ws));
+            PTT_LAUNCHED(c);
+            if ((rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
+        } else {
+            PTT_CUDA(ptt_launch(c, k_gemm_rx, dim3((CT + GT - 1) / GT, gy), dim3(256), 0, x->dd, i + 1, pl, ws,
+                                Fin{tmain, i + 1, i + 1, &info->q, i}));
+            PTT_LAUNCHED(c);
+            if (!tmain && (rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
+        }
     }
     // right-to-left truncation.  The tail of bond i (V replay, Q V_r into
     // core i, swap of core i) is not needed by bond i - 1, which only reads
@@ -813,9 +786,6 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     // contexts of a batch (which overlap whole roundings already: measured
     // 1.22 s against 0.98 s for 64 trains with the side stream), the sweep
     // stays serial.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    PTT_CUDA(cudaStreamIsCapturing(c->stream, &cap));
-    const bool ovl = cap == cudaStreamCaptureStatusNone && !c->capturing && !c->lane;
     bool pending[2] = {false, false};
     for (int i = d - 1; i >= 1 && (phases & 2); i--) {
         const int sl = ovl ? (i & 1) : 0;
@@ -834,7 +804,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         if ((rc = launch_svd(c, rk[i], pl, ws, delta, mr, i))) return rc;
         ptt_time_end(c, PTT_TIME_SVD);
         PTT_LAUNCHED(c);
-        // the tail: V_r, then Q V_r (Householder tree or grid Cholesky QR) into alt[i]
+        // the tail: V_r, then Q V_r (Householder tree or grid Cholesky QR) into alt[i], the swap of core i
         auto tail = [&]() -> int {
             PTT_CUDA(ptt_launch(c, k_svd_replay, dim3((CT + 7) / 8), dim3(256), replay_smem<CT>(), pl, ws));
             PTT_LAUNCHED(c);
@@ -843,10 +813,12 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             if (g) {  // Q V_r for a bond the grid Cholesky QR finished
                 int gx = (int)((mcap + GT - 1) / GT);
                 gx = gx < 1 ? 1 : (gx > 4096 ? 4096 : gx);
-                PTT_CUDA(ptt_launch(c, gq::k_gq_write, dim3(gx, (CT + GT - 1) / GT), dim3(gq::NT), 0, dd, i, pl, *g, ws));
+                PTT_CUDA(ptt_launch(c, gq::k_gq_write, dim3(gx, (CT + GT - 1) / GT), dim3(gq::NT), 0, x->dd, i, pl, *g,
+                                    ws, Fin{ttail, -1, i, &info->rank}));
                 PTT_LAUNCHED(c);
+                if (ttail) return PTT_OK;
             }
-            return PTT_OK;
+            return finalize(-1, i, -1, &info->rank, info);
         };
         if (ovl) {
             PTT_CUDA(cudaEventRecord(c->ev_svd[sl], c->stream));
@@ -860,12 +832,6 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             c->no_pdl = 1;
             rc = tail();
             if (!rc) {
-                const cudaError_t e = ptt_launch(c, k_bond_finalize, dim3(1), dim3(32), 0, x->dd, i, i, -1,
-                                                 (const int*)&info->rank, (const Info*)info);
-                rc = e == cudaSuccess ? PTT_OK : ptt_set_error(PTT_ERR_CUDA, "CUDA: %s", cudaGetErrorString(e));
-                PTT_LAUNCHED(c);
-            }
-            if (!rc) {
                 const cudaError_t e = cudaEventRecord(c->ev_tail[sl], c->side);
                 rc = e == cudaSuccess ? PTT_OK : ptt_set_error(PTT_ERR_CUDA, "CUDA: %s", cudaGetErrorString(e));
             }
@@ -876,22 +842,21 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         } else if ((rc = tail())) {
             return rc;
         }
-        {
-            const long long mcap2 = (long long)rk[i - 1] * x->n[i - 1];
-            int gx = (int)((mcap2 + GT - 1) / GT);
-            if (gx > 4096) gx = 4096;
-            if (c->ozaki && CT <= oz::KG)  // one wave, U_r S_r split once per CTA
-                PTT_CUDA(ptt_launch(c, k_gemm_xm_oz, dim3(1, gx < c->nsm ? gx : c->nsm), dim3(256), oz::SMEM_GEMM,
-                                    x->dd, i - 1, pl, ws));
-            else
-                PTT_CUDA(ptt_launch(c, k_gemm_xm, dim3(gx, (CT + GT - 1) / GT), dim3(256), 0, x->dd, i - 1, pl, ws,
-                                    Fin{}));
+        // core i - 1 times U_r S_r, then the new rank r_i and the swap of core i - 1
+        const long long mcap2 = (long long)rk[i - 1] * x->n[i - 1];
+        int gx = (int)((mcap2 + GT - 1) / GT);
+        if (gx > 4096) gx = 4096;
+        if (c->ozaki && CT <= oz::KG) {  // one wave, U_r S_r split once per CTA
+            PTT_CUDA(ptt_launch(c, k_gemm_xm_oz, dim3(1, gx < c->nsm ? gx : c->nsm), dim3(256), oz::SMEM_GEMM, x->dd,
+                                i - 1, pl, ws));
             PTT_LAUNCHED(c);
+            if ((rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
+        } else {
+            PTT_CUDA(ptt_launch(c, k_gemm_xm, dim3(gx, (CT + GT - 1) / GT), dim3(256), 0, x->dd, i - 1, pl, ws,
+                                Fin{tmain, i, i - 1, &info->rank}));
+            PTT_LAUNCHED(c);
+            if (!tmain && (rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
         }
-        // the new rank r_i and core i - 1 (core i too when the tail ran here)
-        PTT_CUDA(ptt_launch(c, k_bond_finalize, dim3(1), dim3(32), 0, x->dd, i, ovl ? i - 1 : i, ovl ? -1 : i - 1,
-                            (const int*)&info->rank, (const Info*)info));
-        PTT_LAUNCHED(c);
     }
     for (int sl = 0; sl < 2; sl++)
         if (pending[sl]) PTT_CUDA(cudaStreamWaitEvent(c->stream, c->ev_tail[sl], 0));
