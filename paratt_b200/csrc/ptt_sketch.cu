@@ -431,6 +431,473 @@ __global__ void k_gauss_all(double* G, GaussOff o, int k0, int k1, unsigned long
     }
 }
 
+// ---------------------------------------------------------------------------
+// Small ranks: the contractions of one core fused per mode index.
+//
+// With ranks of a few tens a core's contractions are some 10 kFLOP for each of
+// its n mode indices: as batched products they are 3 or 4 launches of mostly
+// padded tiles, bound by launches and latency.  256 modes, ranks 18, sketch
+// rank 12: 19 us a core right-to-left as batched products, 4.7 here; 19.5
+// left-to-right without the QR, 5.4 and 2.9 for M' here.  An RK2 step of the
+// 40-dimensional problem: 12.3 ms in these contractions before, 4.3 now.  The
+// floor of a core is its read, 0.1 us; what is left is one launch, the chain of
+// some 50 tensor-core steps of a warp and the sum of the partials.  Here one
+// warp takes a mode index j through the whole chain on the FP64 tensor
+// cores, with no intermediate in memory: the accumulator of one product is the
+// operand of the next (a lane's accumulators hold the columns 2 q and 2 q + 1
+// of its row, q = lane & 3, so with the contraction index of the next product
+// taken in the order 2 q + s, s = 0, 1, they are its fragments as they are).
+// Cores are read once, straight into fragments.
+//
+// Sums over the modes (W_k) or over the rows (M' = Q^T Z) leave one partial per
+// CTA, at most 32 up to 256 modes; the kernel that reads W_k or M' next adds
+// them in CTA order while it loads them, so no launch does only that: 32
+// partials of 18 x 12 cost each reader about 1 us, a launch of its own 2.3.
+// Deterministic: every order is fixed.
+// ---------------------------------------------------------------------------
+constexpr int SK_NT = 256, SK_NW = SK_NT / 32;
+constexpr int SK_SMAX = 64;    // most partials of a sum
+constexpr int SK_NMAX = 2048;  // largest mode size: beyond it 64 CTAs leave too much of the GPU idle
+constexpr int SK_YR = 8;       // product with y: largest rank of x and of y
+constexpr int SK_YL = 16;      // and largest sketch rank
+
+__device__ __forceinline__ void sk_mma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// A matrix stored as ns partials (ns = 0: as it is), element e summed in order.
+struct SkSum {
+    const double* p;
+    int ns;
+    long long stride;
+};
+__device__ __forceinline__ double sk_sum(const SkSum& m, long long e) {
+    if (m.ns == 0) return m.p[e];
+    double a = 0.0;
+    for (int s0 = 0; s0 < m.ns; s0 += 32) {
+        double v[32];
+#pragma unroll
+        for (int u = 0; u < 32; u++) v[u] = s0 + u < m.ns ? m.p[(long long)(s0 + u) * m.stride + e] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 32; u++) a += v[u];
+    }
+    return a;
+}
+
+// sm(row, col) = the rows x cols matrix m (column-major), zero up to nr x nc;
+// at(row, col) gives the address.  The valid elements are dealt out densely,
+// so that as many threads as there are elements wait for one batch of loads.
+template <typename At>
+__device__ __forceinline__ void sk_fill(const SkSum& m, int rows, int cols, int nr, int nc, At at, double* wout) {
+    for (int e = threadIdx.x; e < nr * nc; e += SK_NT) {
+        const int b = e / nr, a = e - b * nr;
+        if (a >= rows || b >= cols) *at(a, b) = 0.0;
+    }
+    for (int e = threadIdx.x; e < rows * cols; e += SK_NT) {
+        const int b = e / rows, a = e - b * rows;
+        const double v = sk_sum(m, e);
+        *at(a, b) = v;
+        if (wout) wout[e] = v;
+    }
+}
+
+// The warps' accumulators (T tiles of 8 x 8 each) added in a fixed order
+// ((w, w + 4), then w = 0..3) and handed to put(tile, row, column, value).
+template <int T, typename Put>
+__device__ __forceinline__ void sk_reduce(double (&acc)[T][2], double* red, Put put) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2* slot = (double2*)red + (warp & 3) * T * 32;
+    __syncthreads();
+    if (warp >= 4) {
+#pragma unroll
+        for (int t = 0; t < T; t++) slot[t * 32 + lane] = make_double2(acc[t][0], acc[t][1]);
+    }
+    __syncthreads();
+    if (warp < 4) {
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            const double2 v = slot[t * 32 + lane];
+            slot[t * 32 + lane] = make_double2(acc[t][0] + v.x, acc[t][1] + v.y);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < T * 32; e += SK_NT) {
+        const double2* r2 = (const double2*)red + e;
+        const double2 a = r2[0], b = r2[T * 32], c = r2[2 * T * 32], d = r2[3 * T * 32];
+        const int t = e >> 5, l = e & 31;
+        put(t, l >> 2, 2 * (l & 3), ((a.x + b.x) + c.x) + d.x);
+        put(t, l >> 2, 2 * (l & 3) + 1, ((a.y + b.y) + c.y) + d.y);
+    }
+}
+
+// x core (rx x n x rxp), G core (Lk x n x Lp), W = W_{k+1} (rxp x Lp): partial
+// b of W_k (rx x Lk) over the modes of CTA b.  All ranks <= 8 NT.  CTA 0
+// writes the summed W to wout for the left-to-right sweep.
+template <int NT>
+__global__ void __launch_bounds__(SK_NT, 1) k_sketch_rl(const double* x, int rx, int n, int rxp, const double* G, int Lk,
+                                                        int Lp, SkSum W, double* wout, double* part,
+                                                        long long pstride) {
+    PTT_PDL_ENTRY();
+    constexpr int D = 8 * NT, LD = D + (NT % 2 ? 0 : 8);  // LD = 8 mod 16: no bank conflicts
+    __shared__ double Ws[D * LD];
+    __shared__ __align__(16) double red[4 * NT * NT * 64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, q = lane & 3;
+    // the first mode's fragments are in flight while W is summed
+    double xf[NT][NT][2], gf[NT][2 * NT];
+    auto load = [&](int j) {
+        const double* xj = x + (long long)rx * j;
+        const double* Gj = G + (long long)Lk * j;
+#pragma unroll
+        for (int it = 0; it < NT; it++)
+#pragma unroll
+            for (int rt = 0; rt < NT; rt++)
+#pragma unroll
+                for (int s = 0; s < 2; s++) {
+                    const int i = 8 * it + lr, k = 8 * rt + 2 * q + s;
+                    xf[it][rt][s] = (i < rx && k < rxp) ? xj[i + (long long)rx * n * k] : 0.0;
+                }
+#pragma unroll
+        for (int ct = 0; ct < NT; ct++)
+#pragma unroll
+            for (int kp = 0; kp < 2 * NT; kp++) {
+                const int cc = 8 * ct + lr, p = 4 * kp + q;
+                gf[ct][kp] = (cc < Lk && p < Lp) ? Gj[cc + (long long)Lk * n * p] : 0.0;
+            }
+    };
+    const int j0 = blockIdx.x * SK_NW + warp, js = gridDim.x * SK_NW;
+    if (j0 < n) load(j0);
+    sk_fill(W, rxp, Lp, D, D, [&](int i, int p) { return Ws + p * LD + i; }, blockIdx.x == 0 ? wout : nullptr);
+    __syncthreads();
+    double acc[NT * NT][2];
+#pragma unroll
+    for (int t = 0; t < NT * NT; t++) acc[t][0] = acc[t][1] = 0.0;
+    for (int j = j0; j < n; j += js) {
+        if (j != j0) load(j);
+#pragma unroll
+        for (int ct = 0; ct < NT; ct++) {
+            if (8 * ct >= Lk) continue;
+            double at[NT][2];  // (G_j W^T), rows c, columns jx
+#pragma unroll
+            for (int rt = 0; rt < NT; rt++) at[rt][0] = at[rt][1] = 0.0;
+#pragma unroll
+            for (int kp = 0; kp < 2 * NT; kp++) {
+                if (4 * kp >= Lp) continue;
+#pragma unroll
+                for (int rt = 0; rt < NT; rt++) sk_mma(at[rt], gf[ct][kp], Ws[(4 * kp + q) * LD + 8 * rt + lr]);
+            }
+#pragma unroll
+            for (int rt = 0; rt < NT; rt++) {
+                if (8 * rt >= rxp) continue;
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+#pragma unroll
+                    for (int it = 0; it < NT; it++) sk_mma(acc[it * NT + ct], xf[it][rt][s], at[rt][s]);
+            }
+        }
+    }
+    double* out = part + (long long)blockIdx.x * pstride;
+    sk_reduce<NT * NT>(acc, red, [&](int t, int r, int cc, double v) {
+        const int i = 8 * (t / NT) + r, c = 8 * (t % NT) + cc;
+        if (i < rx && c < Lk) out[i + (long long)rx * c] = v;
+    });
+}
+
+// M (r x rx), x core (rx x n x rxp), W = W_{k+1} (rxp x Lp): Z = M x (r n x
+// rxp) and, unless Y is null, Y = Z W (r n x Lp).  All ranks <= 8 NT.
+// rset: the train's ranks that this launch publishes (see GemmB).
+template <int NT>
+__global__ void __launch_bounds__(SK_NT, 1) k_sketch_lr(SkSum M, int r, const double* x, int rx, int n, int rxp, SkSum W,
+                                                        int Lp, double* Z, double* Y, int* rset, int rk0) {
+    PTT_PDL_ENTRY();
+    constexpr int D = 8 * NT, LD = D + (NT % 2 ? 0 : 8), LT = D + 4;
+    __shared__ double Ms[D * LD];  // M(c, i) at i LD + c
+    __shared__ double Ws[D * LT];  // W(i, l) at i LT + l
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, q = lane & 3;
+    if (rset && blockIdx.x == 0 && tid == 0) {
+        rset[rk0] = r;
+        rset[rk0 + 1] = Lp;
+    }
+    double xf[2 * NT][NT];
+    auto load = [&](int j) {
+        const double* xj = x + (long long)rx * j;
+#pragma unroll
+        for (int ks = 0; ks < 2 * NT; ks++)
+#pragma unroll
+            for (int jt = 0; jt < NT; jt++) {
+                const int i = 4 * ks + q, k = 8 * jt + lr;
+                xf[ks][jt] = (i < rx && k < rxp) ? xj[i + (long long)rx * n * k] : 0.0;
+            }
+    };
+    const int j0 = blockIdx.x * SK_NW + warp, js = gridDim.x * SK_NW;
+    if (j0 < n) load(j0);
+    if (Y) sk_fill(W, rxp, Lp, D, D, [&](int i, int l) { return Ws + i * LT + l; }, nullptr);
+    sk_fill(M, r, rx, D, D, [&](int c, int i) { return Ms + i * LD + c; }, nullptr);
+    __syncthreads();
+    const long long zld = (long long)r * n;
+    for (int j = j0; j < n; j += js) {
+        if (j != j0) load(j);
+#pragma unroll
+        for (int ct = 0; ct < NT; ct++) {
+            if (8 * ct >= r) continue;
+            const int c = 8 * ct + lr;
+            double z[NT][2];
+#pragma unroll
+            for (int jt = 0; jt < NT; jt++) z[jt][0] = z[jt][1] = 0.0;
+#pragma unroll
+            for (int ks = 0; ks < 2 * NT; ks++) {
+                if (4 * ks >= rx) continue;
+                const double a = Ms[(4 * ks + q) * LD + c];
+#pragma unroll
+                for (int jt = 0; jt < NT; jt++) sk_mma(z[jt], a, xf[ks][jt]);
+            }
+#pragma unroll
+            for (int jt = 0; jt < NT; jt++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int k = 8 * jt + 2 * q + h;
+                    if (c < r && k < rxp) Z[c + (long long)r * j + zld * k] = z[jt][h];
+                }
+            if (!Y) continue;
+            double y[NT][2];
+#pragma unroll
+            for (int lt = 0; lt < NT; lt++) y[lt][0] = y[lt][1] = 0.0;
+#pragma unroll
+            for (int jt = 0; jt < NT; jt++) {
+                if (8 * jt >= rxp) continue;
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+#pragma unroll
+                    for (int lt = 0; lt < NT; lt++) sk_mma(y[lt], z[jt][s], Ws[(8 * jt + 2 * q + s) * LT + 8 * lt + lr]);
+            }
+#pragma unroll
+            for (int lt = 0; lt < NT; lt++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int l = 8 * lt + 2 * q + h;
+                    if (c < r && l < Lp) Y[c + (long long)r * j + zld * l] = y[lt][h];
+                }
+        }
+    }
+}
+
+// The same two for the product x (.) y, ranks of x and y <= 8, sketch ranks
+// <= 16.  Row ky + ry ix of W_k belongs to the pair (ix, ky).  The rank index
+// of one factor is the tensor-core dimension, the other's is a loop whose
+// factor is a scalar per mode: with it the sum over y's rank is 256 FMAs of a
+// lane's own accumulators.
+__global__ void __launch_bounds__(SK_NT, 1) k_sketch_rl_xy(const double* x, int rx, int rxp, const double* y, int ry,
+                                                           int ryp, int n, const double* G, int Lk, int Lp, SkSum W,
+                                                           double* wout, double* part, long long pstride) {
+    PTT_PDL_ENTRY();
+    constexpr int LD = SK_YR * SK_YR + 8;
+    __shared__ double Ws[SK_YL * LD];  // W(ly + ryp jx, p) at p LD + 8 ly + jx
+    __shared__ __align__(16) double red[4 * 16 * 64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, q = lane & 3;
+    const int Rp = rxp * ryp, R = rx * ry;
+    double xf[2], gf[2][4], yv[2];
+    auto load = [&](int j) {
+        const double* Gj = G + (long long)Lk * j;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const int k = 2 * q + s;
+            xf[s] = (lr < rx && k < rxp) ? x[lr + (long long)rx * (j + (long long)n * k)] : 0.0;
+            yv[s] = (lr < ry && k < ryp) ? y[lr + (long long)ry * (j + (long long)n * k)] : 0.0;  // y(lr, 2 q + s)
+        }
+#pragma unroll
+        for (int ct = 0; ct < 2; ct++)
+#pragma unroll
+            for (int kp = 0; kp < 4; kp++) {
+                const int c = 8 * ct + lr, p = 4 * kp + q;
+                gf[ct][kp] = (c < Lk && p < Lp) ? Gj[c + (long long)Lk * n * p] : 0.0;
+            }
+    };
+    const int j0 = blockIdx.x * SK_NW + warp, js = gridDim.x * SK_NW;
+    if (j0 < n) load(j0);
+    for (int e = tid; e < SK_YL * LD; e += SK_NT) Ws[e] = 0.0;
+    __syncthreads();
+    sk_fill(W, Rp, Lp, Rp, Lp, [&](int i, int p) { return Ws + p * LD + 8 * (i % ryp) + i / ryp; },
+            blockIdx.x == 0 ? wout : nullptr);
+    __syncthreads();
+    double acc[16][2];  // tile 2 ky + ct: rows ix, columns c
+#pragma unroll
+    for (int t = 0; t < 16; t++) acc[t][0] = acc[t][1] = 0.0;
+    for (int j = j0; j < n; j += js) {
+        if (j != j0) load(j);
+#pragma unroll
+        for (int ly = 0; ly < SK_YR; ly++) {
+            if (ly >= ryp) continue;
+            double at[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, b[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+            for (int kp = 0; kp < 4; kp++) {
+                if (4 * kp >= Lp) continue;
+                const double w = Ws[(4 * kp + q) * LD + 8 * ly + lr];
+                sk_mma(at[0], gf[0][kp], w);
+                sk_mma(at[1], gf[1][kp], w);
+            }
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+                sk_mma(b[0], xf[s], at[0][s]);
+                sk_mma(b[1], xf[s], at[1][s]);
+            }
+#pragma unroll
+            for (int ky = 0; ky < SK_YR; ky++) {
+                const double f = __shfl_sync(0xffffffffu, yv[ly & 1], 4 * ky + (ly >> 1));
+#pragma unroll
+                for (int ct = 0; ct < 2; ct++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) acc[2 * ky + ct][h] = fma(f, b[ct][h], acc[2 * ky + ct][h]);
+            }
+        }
+    }
+    double* out = part + (long long)blockIdx.x * pstride;
+    sk_reduce<16>(acc, red, [&](int t, int r, int cc, double v) {
+        const int ky = t >> 1, c = 8 * (t & 1) + cc;
+        if (r < rx && ky < ry && c < Lk) out[ky + ry * r + (long long)R * c] = v;
+    });
+}
+
+__global__ void __launch_bounds__(SK_NT, 1) k_sketch_lr_xy(SkSum M, int r, const double* x, int rx, int rxp,
+                                                           const double* y, int ry, int ryp, int n, SkSum W, int Lp,
+                                                           double* Z, double* Y, int* rset, int rk0) {
+    PTT_PDL_ENTRY();
+    constexpr int LD = SK_YL + 8, LT = SK_YL + 4;
+    __shared__ double Ms[64 * LD];  // M(c, ky + ry ix) at (8 ix + ky) LD + c
+    __shared__ double Ws[64 * LT];  // W(ly + ryp jx, l) at (8 jx + ly) LT + l
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, q = lane & 3;
+    const int Rp = rxp * ryp;
+    if (rset && blockIdx.x == 0 && tid == 0) {
+        rset[rk0] = r;
+        rset[rk0 + 1] = Lp;
+    }
+    double xv[2], yf[2];
+    auto load = [&](int j) {
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const int k = 2 * q + s, ky = 4 * s + q;
+            xv[s] = (lr < rx && k < rxp) ? x[lr + (long long)rx * (j + (long long)n * k)] : 0.0;  // x(lr, 2 q + s)
+            yf[s] = (ky < ry && lr < ryp) ? y[ky + (long long)ry * (j + (long long)n * lr)] : 0.0;
+        }
+    };
+    const int j0 = blockIdx.x * SK_NW + warp, js = gridDim.x * SK_NW;
+    if (j0 < n) load(j0);
+    for (int e = tid; e < 64 * LD; e += SK_NT) Ms[e] = 0.0;
+    for (int e = tid; e < 64 * LT; e += SK_NT) Ws[e] = 0.0;
+    __syncthreads();
+    if (Y) sk_fill(W, Rp, Lp, Rp, Lp, [&](int i, int l) { return Ws + (8 * (i / ryp) + i % ryp) * LT + l; }, nullptr);
+    sk_fill(M, r, rx * ry, r, rx * ry, [&](int c, int i) { return Ms + (8 * (i / ry) + i % ry) * LD + c; }, nullptr);
+    __syncthreads();
+    const long long zld = (long long)r * n;
+    for (int j = j0; j < n; j += js) {
+        if (j != j0) load(j);
+#pragma unroll
+        for (int ct = 0; ct < 2; ct++) {
+            if (8 * ct >= r) continue;
+            const int c = 8 * ct + lr;
+            double z[SK_YR][2];  // z[jx]: rows c, columns ly
+#pragma unroll
+            for (int jx = 0; jx < SK_YR; jx++) z[jx][0] = z[jx][1] = 0.0;
+#pragma unroll
+            for (int ix = 0; ix < SK_YR; ix++) {
+                if (ix >= rx) continue;
+                double pt[2] = {0.0, 0.0};  // P(c, ly) = sum_ky M(c, ky + ry ix) y(ky, ly)
+#pragma unroll
+                for (int s = 0; s < 2; s++) sk_mma(pt, Ms[(8 * ix + 4 * s + q) * LD + c], yf[s]);
+#pragma unroll
+                for (int jx = 0; jx < SK_YR; jx++) {
+                    const double f = __shfl_sync(0xffffffffu, xv[jx & 1], 4 * ix + (jx >> 1));
+                    z[jx][0] = fma(f, pt[0], z[jx][0]);
+                    z[jx][1] = fma(f, pt[1], z[jx][1]);
+                }
+            }
+            double yo[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+            for (int jx = 0; jx < SK_YR; jx++) {
+                if (jx >= rxp) continue;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int ly = 2 * q + h;
+                    if (c < r && ly < ryp) Z[c + (long long)r * j + zld * (ly + ryp * jx)] = z[jx][h];
+                }
+                if (Y) {
+#pragma unroll
+                    for (int s = 0; s < 2; s++)
+#pragma unroll
+                        for (int lt = 0; lt < 2; lt++)
+                            sk_mma(yo[lt], z[jx][s], Ws[(8 * jx + 2 * q + s) * LT + 8 * lt + lr]);
+                }
+            }
+            if (!Y) continue;
+#pragma unroll
+            for (int lt = 0; lt < 2; lt++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int l = 8 * lt + 2 * q + h;
+                    if (c < r && l < Lp) Y[c + (long long)r * j + zld * l] = yo[lt][h];
+                }
+        }
+    }
+}
+
+// Partial b of M' = Q^T Z (q x N) over the rows [b rows, (b + 1) rows) of the
+// K: Q is K x q, Z K x N, both column-major with leading dimension K.  q <= 8
+// TQ, N <= 8 TN.  Warp w takes an eighth of the rows, fragments straight from
+// memory (a group of four lanes reads 32 contiguous bytes), four steps in
+// flight.  rows is a multiple of 32.
+template <int TQ, int TN>
+__global__ void __launch_bounds__(SK_NT, 1) k_sketch_m(const double* Q, const double* Z, int K, int q, int N, int rows,
+                                                       double* part, long long pstride) {
+    PTT_PDL_ENTRY();
+    __shared__ __align__(16) double red[4 * TQ * TN * 64];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    double acc[TQ * TN][2];
+#pragma unroll
+    for (int t = 0; t < TQ * TN; t++) acc[t][0] = acc[t][1] = 0.0;
+    const int per = rows / SK_NW;
+    const int k0 = blockIdx.x * rows + warp * per;
+    const int k1 = k0 + per < K ? k0 + per : K;
+    constexpr int U = TQ + TN > 8 ? 2 : 4;
+    for (int k = k0; k < k1; k += 4 * U) {
+        double a[U][TQ], b[U][TN];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int row = k + 4 * u + lk;
+#pragma unroll
+            for (int t = 0; t < TQ; t++)
+                a[u][t] = (row < k1 && 8 * t + lr < q) ? Q[row + (long long)K * (8 * t + lr)] : 0.0;
+#pragma unroll
+            for (int t = 0; t < TN; t++)
+                b[u][t] = (row < k1 && 8 * t + lr < N) ? Z[row + (long long)K * (8 * t + lr)] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int t = 0; t < TQ; t++) {
+                if (8 * t >= q) continue;
+#pragma unroll
+                for (int v = 0; v < TN; v++) sk_mma(acc[t * TN + v], a[u][t], b[u][v]);
+            }
+    }
+    double* out = part + (long long)blockIdx.x * pstride;
+    sk_reduce<TQ * TN>(acc, red, [&](int t, int r, int cc, double v) {
+        const int i = 8 * (t / TN) + r, c = 8 * (t % TN) + cc;
+        if (i < q && c < N) out[i + (long long)q * c] = v;
+    });
+}
+
+// CTAs of a per-mode launch and rows of an M' slice (a multiple of 32)
+static int sk_ctas(int n) {
+    const int one = (n + SK_NW - 1) / SK_NW;  // one mode a warp
+    if (one <= 32) return one;
+    const int four = (n + 4 * SK_NW - 1) / (4 * SK_NW);
+    return four > 32 ? (four < SK_SMAX ? four : SK_SMAX) : 32;
+}
+static int sk_rows(int K) {
+    const int r = ((K + 31) / 32 + 31) / 32 * 32;  // at most 32 slices
+    return r < 64 ? 64 : r;
+}
+
 __global__ void k_fill(double* p, long long cnt, double v) {
     PTT_PDL_ENTRY();
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < cnt;
@@ -476,6 +943,19 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
         if (l < 1) l = 1;
         L[k] = (int)l;
     }
+    // every core fused per mode (the kernels above): the ranks and sketch ranks
+    // within their tiles, the mode sizes within what 64 CTAs keep up with.  All
+    // cores or none: the two paths hand W and M over in different forms.
+    // A rounding of 10 modes, general / fused, ms: ranks 8 and sketch 8 at n = 8
+    // 0.75 / 0.67, at 2048 1.24 / 0.83; ranks 24, sketch 16 at n = 256 1.17 /
+    // 0.96, at 2048 3.17 / 2.77; ranks 32, sketch 32 at n = 256 1.93 / 1.86, at
+    // 1024 5.26 / 5.31; products of ranks 8 and 8, sketch 16 at n = 8 0.89 /
+    // 0.85, at 256 1.60 / 1.11, at 2048 5.97 / 3.03.
+    bool fuse = true;
+    for (int k = 0; k <= d; k++) {
+        if (y ? (rx[k] > SK_YR || ry[k] > SK_YR || L[k] > SK_YL) : rx[k] > 32) fuse = false;
+        if (k < d && n[k] > SK_NMAX) fuse = false;
+    }
     // z capacity: ranks <= L
     {
         int cap[PTT_MAX_DIM + 1];
@@ -501,8 +981,17 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
         szZ = (long long)L[k] * n[k] * Rp > szZ ? (long long)L[k] * n[k] * Rp : szZ;
         szM = (long long)L[k] * R[k] > szM ? (long long)L[k] * R[k] : szM;
     }
-    const long long oA = off, oB = oA + szA, oP = oB + szB, oZ = oP + szP, oM0 = oZ + szZ, oM1 = oM0 + szM;
-    const long long total = oM1 + szM + 64;
+    long long szW = 1;  // partials of W_k (two buffers); those of M' share the size
+    if (fuse) {
+        szA = szB = szP = 0;
+        for (int k = 1; k < d; k++) {  // M' has at most 32 partials
+            const long long ns = sk_ctas(n[k]) > 32 ? sk_ctas(n[k]) : 32;
+            szW = ns * L[k] * R[k] > szW ? ns * L[k] * R[k] : szW;
+        }
+    }
+    const long long oA = off, oB = oA + szA, oP = oB + szB, oZ = oP + szP, oM0 = oZ + szZ, oM1 = oM0 + szM,
+                    oW0 = oM1 + szM, oW1 = oW0 + szW, oMp = oW1 + szW;
+    const long long total = oMp + szW + 64;
     if ((rc = ptt_ws2_reserve(c, (size_t)total * sizeof(double)))) return rc;
     double* ws = (double*)c->ws2;
     // input core pointers (the ones train points every core at one ones vector)
@@ -532,11 +1021,43 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
     PTT_CUDA(ptt_launch(c, k_fill, dim3(1), dim3(32), 0, ws + oW[d], 1, 1.0));
     PTT_LAUNCHED(c);
 
+    auto tiles_of = [](int a, int b, int e, int f) {  // 16, 24 or 32-wide tiles: 2, 3 or 4
+        const int m = (a > b ? a : b) > (e > f ? e : f) ? (a > b ? a : b) : (e > f ? e : f);
+        return m <= 16 ? 2 : (m <= 24 ? 3 : 4);
+    };
+    auto work = [&](double flop) {
+        if (c->tkind == PTT_TIME_GEMM) c->hwork[PTT_TIME_GEMM] += flop;
+    };
+
     // ---- right-to-left sketch contractions -------------------------------
+    SkSum Wk{ws + oW[d], 0, 0};  // W_{k+1}
     for (int k = d - 1; k >= 1; k--) {
         const long long Rp = R[k + 1];
         const int Lk = L[k], Lp = L[k + 1], nk = n[k];
         const int rxk = rx[k], ryk = ry[k], rxp = rx[k + 1], ryp = ry[k + 1];
+        if (fuse) {
+            double* part = ws + ((k & 1) ? oW0 : oW1);
+            const long long ps = R[k] * Lk;
+            const int ns = sk_ctas(nk);
+            double* wout = Wk.ns ? ws + oW[k + 1] : nullptr;
+            const double* G = ws + oG[k];
+            ptt_time_begin(c, PTT_TIME_GEMM);
+            if (y) {
+                work(2.0 * nk * Lk * ((double)Rp * Lp + (double)rxk * rxp * ryp + (double)R[k] * ryp));
+                PTT_CUDA(ptt_launch(c, k_sketch_rl_xy, dim3(ns), dim3(SK_NT), 0, xc[k], rxk, rxp, yc[k], ryk, ryp, nk, G,
+                                    Lk, Lp, Wk, wout, part, ps));
+            } else {
+                work(2.0 * nk * Lk * ((double)Rp * Lp + (double)rxk * rxp));
+                const int nt = tiles_of(rxk, rxp, Lk, Lp);
+                auto kern = nt == 2 ? k_sketch_rl<2> : (nt == 3 ? k_sketch_rl<3> : k_sketch_rl<4>);
+                PTT_CUDA(ptt_launch(c, kern, dim3(ns), dim3(SK_NT), 0, xc[k], rxk, nk, rxp, G, Lk, Lp, Wk, wout, part,
+                                    ps));
+            }
+            PTT_LAUNCHED(c);
+            ptt_time_end(c, PTT_TIME_GEMM);
+            Wk = SkSum{part, ns, ps};
+            continue;
+        }
         GemmB g;
         if (!y) {
             // x alone (the partner is the ones train): A_j = W_{k+1} G_j^T
@@ -578,6 +1099,7 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
     // ---- left-to-right orthogonalisation against the sketch ----------------
     double* M = ws + oM0;
     double* Mn = ws + oM1;
+    SkSum Mk{M, 0, 0};
     PTT_CUDA(ptt_launch(c, k_fill, dim3(1), dim3(32), 0, M, 1, 1.0));
     PTT_LAUNCHED(c);
     int r = 1;
@@ -589,7 +1111,29 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
         const int nk = n[k], rxk = rx[k], ryk = ry[k], rxp = rx[k + 1], ryp = ry[k + 1];
         GemmB g;
         double* Zp = (k == d - 1) ? z->hd.core[k] : ws + oZ;
-        if (!y) {
+        int* const dr = (int*)((char*)z->dd + offsetof(DevDesc, r));
+        if (fuse) {
+            // Z, and Y = Z W_{k+1} into z core k, whose ranks it sets for the QR
+            const bool last = k == d - 1;
+            const int Lp = L[k + 1];
+            const SkSum W = k == 0 ? Wk : SkSum{ws + oW[k + 1], 0, 0};  // W_2 .. were summed by their first reader
+            double* Y = last ? nullptr : z->hd.core[k];
+            int* rset = last ? nullptr : dr;
+            ptt_time_begin(c, PTT_TIME_GEMM);
+            if (y) {
+                work(2.0 * nk * r * ((double)ryp * R[k] + (double)rxp * rxk * ryp + (last ? 0.0 : (double)Lp * Rp)));
+                PTT_CUDA(ptt_launch(c, k_sketch_lr_xy, dim3(sk_ctas(nk)), dim3(SK_NT), 0, Mk, r, xc[k], rxk, rxp, yc[k],
+                                    ryk, ryp, nk, W, Lp, Zp, Y, rset, k));
+            } else {
+                work(2.0 * nk * r * ((double)Rp * rxk + (last ? 0.0 : (double)Lp * Rp)));
+                const int nt = tiles_of(rxk, rxp, r, Lp);
+                auto kern = nt == 2 ? k_sketch_lr<2> : (nt == 3 ? k_sketch_lr<3> : k_sketch_lr<4>);
+                PTT_CUDA(ptt_launch(c, kern, dim3(sk_ctas(nk)), dim3(SK_NT), 0, Mk, r, xc[k], rxk, nk, rxp, W, Lp, Zp, Y,
+                                    rset, k));
+            }
+            PTT_LAUNCHED(c);
+            ptt_time_end(c, PTT_TIME_GEMM);
+        } else if (!y) {
             // x alone: Z = M x_k, (r x r_k) times the core's right unfolding
             g = GemmB{M, 1, r, 0, 0,
                       xc[k], 1, rxk, 0, 0,
@@ -618,12 +1162,14 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
         const int Lp = L[k + 1];
         // Y = Z W_{k+1} into z core k, then QR in place (core k <- Q)
         // its first kernel also sets z's ranks r_k = r, r_{k+1} = Lp for the QR
-        g = GemmB{ws + oZ, 1, (long long)r * nk, 0, 0,
-                  ws + oW[k + 1], 1, Rp, 0, 0,
-                  z->hd.core[k], 1, (long long)r * nk, 0, 0,
-                  r * nk, Lp, (int)Rp, 1, 1, 1.0, 0.0,
-                  (int*)((char*)z->dd + offsetof(DevDesc, r)), k, r, Lp};
-        if ((rc = gemm(c, g))) return rc;
+        if (!fuse) {
+            g = GemmB{ws + oZ, 1, (long long)r * nk, 0, 0,
+                      ws + oW[k + 1], 1, Rp, 0, 0,
+                      z->hd.core[k], 1, (long long)r * nk, 0, 0,
+                      r * nk, Lp, (int)Rp, 1, 1, 1.0, 0.0,
+                      dr, k, r, Lp};
+            if ((rc = gemm(c, g))) return rc;
+        }
         {
             // QR of core k: ranks known here (no read-back); the QR swaps
             // core k with its second buffer, mirrored in the host shadow
@@ -638,6 +1184,22 @@ static int sketch_round(const ptt_tt* x, const ptt_tt* y, ptt_tt* z, const int* 
         }
         const int q = r * nk < Lp ? r * nk : Lp;
         // M' = Q^T Z   (q x Rp)
+        if (fuse) {
+            const int K = r * nk, rows = sk_rows(K), ns = (K + rows - 1) / rows;
+            const long long ps = (long long)q * Rp;
+            work(2.0 * K * (double)ps);
+            const int nt = tiles_of(q, rxp, 0, 0);
+            auto kern = y ? k_sketch_m<2, 8> : (nt == 2 ? k_sketch_m<2, 2> : (nt == 3 ? k_sketch_m<3, 3> : k_sketch_m<4, 4>));
+            ptt_time_begin(c, PTT_TIME_GEMM);
+            PTT_CUDA(ptt_launch(c, kern, dim3(ns), dim3(SK_NT), 0, (const double*)z->hd.core[k], (const double*)(ws + oZ), K,
+                                q, (int)Rp, rows, ws + oMp, ps));
+            PTT_LAUNCHED(c);
+            ptt_time_end(c, PTT_TIME_GEMM);
+            Mk = SkSum{ws + oMp, ns, ps};
+            zr[k] = r;
+            r = q;
+            continue;
+        }
         g = GemmB{z->hd.core[k], (long long)r * nk, 1, 0, 0,
                   ws + oZ, 1, (long long)r * nk, 0, 0,
                   Mn, 1, q, 0, 0,
