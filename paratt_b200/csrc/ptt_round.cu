@@ -432,6 +432,140 @@ __global__ void __launch_bounds__(256) k_gemm_xm(DevDesc* D, int im1, Plan pl, d
     fin_last_block(D, fin, pl.info);
 }
 
+// The same two contractions for a train whose ranks stay <= 8 NT <= 32, with
+// the rank update and the swap (kq, core i).  Latency bounds them: 2560 x 10
+// columns are 0.4 us of DMMAs and of memory, a launch 0.8 us, the pointer chase
+// (record, descriptor, data) 0.35 us a step and the ticket 0.7.  So the record
+// and the descriptor are read together, every warp takes 8 columns (rows) with
+// both operands' fragments straight from memory -- all its loads in flight at
+// once, no shared memory, no barrier before the ticket -- and only the tiles
+// that exist are multiplied.  The k order is gemm_tile's: the same bits.  A
+// launch of a 40-dimensional step (n = 256, ranks to 16) in its chain: 5.3 us
+// with 64 x 64 tiles, 2.6 here; 5120 x 20 columns 7.1 and 3.8.
+struct WGemm {
+    int status, c, q, rank, nk, r0, r1;
+    double *core, *alt;
+};
+__device__ __forceinline__ WGemm wgemm_sizes(const DevDesc* D, int i, const Info* info) {
+    WGemm g;
+    g.status = info->status;
+    g.c = info->c;
+    g.q = info->q;
+    g.rank = info->rank;
+    g.nk = D->n[i];
+    g.r0 = D->r[i];
+    g.r1 = D->r[i + 1];
+    g.core = D->core[i];
+    g.alt = D->alt[i];
+    return g;
+}
+__device__ __forceinline__ void wgemm_finish(DevDesc* D, int* ticket, int kq, int i, const WGemm& g, int val) {
+    __threadfence();  // this block's output is visible before its ticket
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(ticket, 1) == (int)gridDim.x - 1) {
+        *ticket = 0;
+        if (g.status == 0) {
+            D->r[kq] = val;
+            D->core[i] = g.alt;
+            D->alt[i] = g.core;
+        }
+    }
+}
+
+// core i <- R core i (R = root factor, q x c, row-major CT), r_i <- q
+template <int NT8>
+__global__ void __launch_bounds__(256) k_wgemm_rx(DevDesc* D, int i, Plan pl, const double* ws, int* ticket) {
+    PTT_PDL_ENTRY();
+    const WGemm g = wgemm_sizes(D, i, pl.info);
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    const int N = g.nk * g.r1, q = g.q, c = g.c;
+    const double* R = ws + pl.o_Rn;
+    const int t0 = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (g.status == 0 && 8 * t0 < N) {
+        double a[NT8][2 * NT8], b[2 * NT8];
+        auto load_b = [&](int t) {
+#pragma unroll
+            for (int k4 = 0; k4 < 2 * NT8; k4++) {
+                const int kk = 4 * k4 + lk, col = 8 * t + lr;
+                b[k4] = (kk < c && col < N) ? g.core[kk + (long long)c * col] : 0.0;
+            }
+        };
+        load_b(t0);
+#pragma unroll
+        for (int r = 0; r < NT8; r++)
+#pragma unroll
+            for (int k4 = 0; k4 < 2 * NT8; k4++) {
+                const int row = 8 * r + lr, kk = 4 * k4 + lk;
+                a[r][k4] = (row < q && kk < c) ? R[row * pl.CT + kk] : 0.0;
+            }
+        for (int t = t0; 8 * t < N; t += 8 * gridDim.x) {
+            if (t != t0) load_b(t);
+#pragma unroll
+            for (int r = 0; r < NT8; r++) {
+                if (8 * r >= q) continue;
+                double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+                for (int k4 = 0; k4 < 2 * NT8; k4++)
+                    if (4 * k4 < c)
+                        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                                     : "+d"(d0), "+d"(d1)
+                                     : "d"(a[r][k4]), "d"(b[k4]));
+                const int row = 8 * r + lr, col = 8 * t + 2 * lk;
+                if (row < q && col < N) g.alt[row + (long long)q * col] = d0;
+                if (row < q && col + 1 < N) g.alt[row + (long long)q * (col + 1)] = d1;
+            }
+        }
+    }
+    wgemm_finish(D, ticket, i, i, g, q);
+}
+
+// core i <- core i US (US = c x rank, column-major, leading dimension CT), r_{i+1} <- rank
+template <int NT8>
+__global__ void __launch_bounds__(256) k_wgemm_xm(DevDesc* D, int i, Plan pl, const double* ws, int* ticket) {
+    PTT_PDL_ENTRY();
+    const WGemm g = wgemm_sizes(D, i, pl.info);
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    const int M = g.r0 * g.nk, c = g.c, rank = g.rank;
+    const double* US = ws + pl.o_US;
+    const int t0 = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (g.status == 0 && 8 * t0 < M) {
+        double a[2 * NT8], b[NT8][2 * NT8];
+        auto load_a = [&](int t) {
+#pragma unroll
+            for (int k4 = 0; k4 < 2 * NT8; k4++) {
+                const int row = 8 * t + lr, kk = 4 * k4 + lk;
+                a[k4] = (row < M && kk < c) ? g.core[row + (long long)M * kk] : 0.0;
+            }
+        };
+        load_a(t0);
+#pragma unroll
+        for (int v = 0; v < NT8; v++)
+#pragma unroll
+            for (int k4 = 0; k4 < 2 * NT8; k4++) {
+                const int col = 8 * v + lr, kk = 4 * k4 + lk;
+                b[v][k4] = (col < rank && kk < c) ? US[kk + pl.CT * col] : 0.0;
+            }
+        for (int t = t0; 8 * t < M; t += 8 * gridDim.x) {
+            if (t != t0) load_a(t);
+#pragma unroll
+            for (int v = 0; v < NT8; v++) {
+                if (8 * v >= rank) continue;
+                double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+                for (int k4 = 0; k4 < 2 * NT8; k4++)
+                    if (4 * k4 < c)
+                        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                                     : "+d"(d0), "+d"(d1)
+                                     : "d"(a[k4]), "d"(b[v][k4]));
+                const int row = 8 * t + lr, col = 8 * v + 2 * lk;
+                if (row < M && col < rank) g.alt[row + (long long)M * col] = d0;
+                if (row < M && col + 1 < rank) g.alt[row + (long long)M * (col + 1)] = d1;
+            }
+        }
+    }
+    wgemm_finish(D, ticket, i + 1, i, g, rank);
+}
+
 #include "ptt_ozaki.cuh"
 
 // k_gemm_rx of the block-level path with the product as an Ozaki
@@ -1110,8 +1244,9 @@ static int round_impl_w(ptt_tt* x, const int* rk, double delta, const int* maxr,
                 int gy = (int)((ncap + GT - 1) / GT);
                 if (gy > 4096) gy = 4096;
                 // the contraction's last block publishes the rank and swaps the core
-                PTT_CUDA(ptt_launch(c, k_gemm_rx, dim3(dim3(1, gy)), dim3(256), 0, x->dd, i + 1, pl, wsb,
-                                    Fin{fin_ticket, i + 1, i + 1, &pl.info->q}));
+                const int cb = cbound(rk[i + 1]);
+                auto kern = cb == 16 ? k_wgemm_rx<2> : (cb == 24 ? k_wgemm_rx<3> : k_wgemm_rx<4>);
+                PTT_CUDA(ptt_launch(c, kern, dim3(gy), dim3(256), 0, x->dd, i + 1, pl, (const double*)wsb, fin_ticket));
                 PTT_LAUNCHED(c);
             }
             if (d > 1) {
@@ -1136,8 +1271,9 @@ static int round_impl_w(ptt_tt* x, const int* rk, double delta, const int* maxr,
                 const long long mcap = (long long)rk[i - 1] * x->n[i - 1];
                 int gx = (int)((mcap + GT - 1) / GT);
                 if (gx > 4096) gx = 4096;
-                PTT_CUDA(ptt_launch(c, k_gemm_xm, dim3(dim3(gx, 1)), dim3(256), 0, x->dd, i - 1, pl, wsb,
-                                    Fin{fin_ticket, i, i - 1, &pl.info->rank}));
+                const int cb = cbound(rk[i]);
+                auto kern = cb == 16 ? k_wgemm_xm<2> : (cb == 24 ? k_wgemm_xm<3> : k_wgemm_xm<4>);
+                PTT_CUDA(ptt_launch(c, kern, dim3(gx), dim3(256), 0, x->dd, i - 1, pl, (const double*)wsb, fin_ticket));
                 PTT_LAUNCHED(c);
             }
             if (d > 1) {
