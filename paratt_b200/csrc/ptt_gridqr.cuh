@@ -631,18 +631,17 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
 
 // alt[k] = Q V_r (m x rank, row-major) for a RIGHT_T bond this path finished:
 // Q rows in g.qscr (row-major, pitch c), V_r at the root B slot (row-major CT
-// x KC).  64 x 64 tiles on the FP64 tensor cores.
-__global__ void __launch_bounds__(NT) k_gq_write(DevDesc* D, int k, Plan pl, GQ g, double* ws, Fin fin) {
+// x KC).  With a ticket the last block swaps the core, also for a bond the
+// Householder tree wrote.
+template <int CB>
+__global__ void __launch_bounds__(256, Slab<CB>::PER_SM) k_gq_write(DevDesc* D, int k, Plan pl, GQ g, double* ws,
+                                                                    Fin fin) {
     PTT_PDL_ENTRY();
+    extern __shared__ __align__(128) double gsm[];
     const Info* info = pl.info;
     if (finished(ldcg((const int*)g.rec)) && info->status == 0) {
         const int m = info->m, c = info->c, rank = info->rank;
-        if ((int)blockIdx.y * GT < rank) {
-            GV Q{g.qscr, c, 1};
-            GV V{ws + pl.o_Bn, pl.KC, 1};
-            for (int t = blockIdx.x; t * GT < m; t += gridDim.x)
-                gemm_tile(Q, V, D->alt[k], rank, 1, m, rank, c, t, blockIdx.y);
-        }
+        slab_mul<CB>(ws + pl.o_Bn, 1, pl.KC, rank, c, g.qscr, 1, c, m, D->alt[k], 1, rank, blockIdx.x, gridDim.x, gsm);
     }
     fin_last_block(D, fin, info);
 }

@@ -283,81 +283,96 @@ __global__ void __launch_bounds__(256) k_svd_replay_b(Plan pl, double* ws, long 
 }
 
 // ---------------------------------------------------------------------------
-// FP64 GEMM tiles: C[M x N] = A[M x K] * B[K x N], views with strides.
+// A small matrix times a long one on the FP64 tensor cores: C(row, n) =
+// sum_k S(row, k) B(k, n), S s x c with s, c <= CB (R, U_r S_r or V_r of a
+// bond), n < N in the tens of thousands (a core's columns or rows).
+//
+// Memory is the bound at CB = 64 (16384 columns: 16 MB, 2.5 us, against 3.6 of
+// DMMAs at their peak).  S is laid out once per CTA in fragment order (one
+// conflict-free read per product); a warp takes 8 columns of B at a time,
+// fragments straight from memory, all of a tile's loads in flight and the next
+// tile's issued as the products use up this one's.  k runs in the order 8 b + 2 q
+// + s (lane q of four, step s), so a group of four lanes reads 64 contiguous
+// bytes whichever index of B is contiguous.  64 x 64 x 16 tiles staged through
+// shared memory took 18.2 us (R x core), 14.5 (core x U_r S_r) and 12.1 (Q V_r)
+// at 16384 x 64.
 // ---------------------------------------------------------------------------
-struct GV {
-    const double* p;
-    long long rs, cs;
+template <int CB>
+struct Slab {
+    static constexpr int T = CB / 8;                                // tile rows of S, blocks of 8 of k
+    static constexpr size_t SMEM = sizeof(double) * T * T * 64;
+    static constexpr int PER_SM = CB <= 64 ? 2 : 1;                 // CTAs
 };
 
-constexpr int GT = 64, GK = 16;
-
-__device__ void gemm_tile(GV A, GV B, double* C, long long crs, long long ccs, int M, int N, int K, int tm, int tn) {
-    __shared__ double sA[GK][GT + 1];
-    __shared__ double sB[GK][GT + 1];
-    const int tid = threadIdx.x;
-    const int m0 = tm * GT, n0 = tn * GT;
-    // the tile product on the FP64 tensor cores: warp w owns the eight 8 x 8
-    // output tiles of tile row w (mma.m8n8k4, four k a step)
-    const int warp = tid >> 5, lane = tid & 31, li = lane >> 2, lk = lane & 3;
-    double d0[8], d1[8];
+template <int CB>
+__device__ __forceinline__ void slab_mul(const double* S, int srs, int scs, int s, int c, const double* B, long long brs,
+                                         long long bcs, long long N, double* C, long long crs, long long ccs, int blk,
+                                         int nblk, double* Ss) {
+    constexpr int T = Slab<CB>::T;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, q = lane & 3;
+    const int st = (s + 7) >> 3, kt = (c + 7) >> 3;
+    double b[T][2];
+    const double* bp = B + 2 * q * brs + lr * bcs;
+    auto load = [&](long long n0, int kb) {
 #pragma unroll
-    for (int t = 0; t < 8; t++) {
-        d0[t] = 0.0;
-        d1[t] = 0.0;
-    }
-    // every element of a K chunk requested before the first is stored, and the
-    // next chunk's loads in flight during this chunk's products
-    constexpr int PT = GT * GK / 256;
-    double va[PT], vb[PT];
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int u = 0; u < PT; u++) {
-            const int e = tid + 256 * u;
-            {
-                const int r = e % GT, kk = e / GT;
-                const int gr = m0 + r, gk = k0 + kk;
-                va[u] = (gr < M && gk < K) ? A.p[(long long)gr * A.rs + (long long)gk * A.cs] : 0.0;
-            }
-            {
-                const int kk = e % GK, cn = e / GK;
-                const int gk = k0 + kk, gc = n0 + cn;
-                vb[u] = (gk < K && gc < N) ? B.p[(long long)gk * B.rs + (long long)gc * B.cs] : 0.0;
-            }
-        }
+        for (int h = 0; h < 2; h++)
+            b[kb][h] = (8 * kb + 2 * q + h < c && n0 + lr < N) ? bp[(8 * kb + h) * brs + n0 * bcs] : 0.0;
     };
-    if (K > 0) load(0);
-    for (int k0 = 0; k0 < K; k0 += GK) {
+    long long n0 = 8LL * (8 * blk + warp);
+    const long long step = 64LL * nblk;
+    if (n0 < N) {
 #pragma unroll
-        for (int u = 0; u < PT; u++) {
-            const int e = tid + 256 * u;
-            sA[e / GT][e % GT] = va[u];
-            sB[e % GK][e / GK] = vb[u];
+        for (int kb = 0; kb < T; kb++) load(n0, kb);
+    }
+    for (int e = tid; e < 64 * st * kt; e += 256) {
+        int row, k;
+        if (scs == 1) {
+            k = e % (8 * kt);
+            row = e / (8 * kt);
+        } else {
+            row = e % (8 * st);
+            k = e / (8 * st);
         }
-        __syncthreads();
-        if (k0 + GK < K) load(k0 + GK);
+        const double v = (row < s && k < c) ? S[(long long)row * srs + (long long)k * scs] : 0.0;
+        Ss[((((k >> 3) * 2 + (k & 1)) * T + (row >> 3)) << 5) + ((row & 7) << 2) + ((k & 7) >> 1)] = v;
+    }
+    __syncthreads();
+    for (; n0 < N; n0 += step) {
+        double d[T][2];
 #pragma unroll
-        for (int k4 = 0; k4 < GK; k4 += 4) {
-            const double av = sA[k4 + lk][8 * warp + li];
+        for (int r = 0; r < T; r++) d[r][0] = d[r][1] = 0.0;
+        const bool more = n0 + step < N;
 #pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const double bv = sB[k4 + lk][8 * t + li];
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                             : "+d"(d0[t]), "+d"(d1[t])
-                             : "d"(av), "d"(bv));
+        for (int kb = 0; kb < T; kb++) {
+            if (kb < kt) {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int r = 0; r < T; r++)
+                        if (r < st) {
+                            const double a = Ss[(((kb * 2 + h) * T + r) << 5) + lane];
+                            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                                         : "+d"(d[r][0]), "+d"(d[r][1])
+                                         : "d"(a), "d"(b[kb][h]));
+                        }
+                if (more) load(n0 + step, kb);
             }
         }
-        __syncthreads();
-    }
-    const int gr = m0 + 8 * warp + li;
-    if (gr < M) {
+        const long long col = n0 + 2 * q;
 #pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const int gc = n0 + 8 * t + 2 * lk;
-            if (gc < N) C[(long long)gr * crs + (long long)gc * ccs] = d0[t];
-            if (gc + 1 < N) C[(long long)gr * crs + (long long)(gc + 1) * ccs] = d1[t];
+        for (int r = 0; r < T; r++) {
+            const int row = 8 * r + lr;
+            if (row < s && col < N) C[row * crs + col * ccs] = d[r][0];
+            if (row < s && col + 1 < N) C[row * crs + (col + 1) * ccs] = d[r][1];
         }
     }
+}
+
+// CTAs of such a launch for at most ncap columns
+template <int CB>
+static int slab_ctas(long long ncap, int nsm) {
+    const long long t = (ncap + 63) / 64, w = (long long)Slab<CB>::PER_SM * nsm;
+    return (int)(t < 1 ? 1 : (t < w ? t : w));
 }
 
 // The bookkeeping that follows a bond's contraction: publish the bond's new
@@ -397,38 +412,27 @@ __device__ __forceinline__ void fin_last_block(DevDesc* D, const Fin& f, const I
 }
 
 // core[i+1] <- R * core[i+1]   (R = root factor, q x c, row-major CT)
-__global__ void __launch_bounds__(256) k_gemm_rx(DevDesc* D, int i1, Plan pl, double* ws, Fin fin) {
+template <int CB>
+__global__ void __launch_bounds__(256, Slab<CB>::PER_SM) k_gemm_rx(DevDesc* D, int i1, Plan pl, double* ws, Fin fin) {
     PTT_PDL_ENTRY();
-    const int tm = blockIdx.x, tn = blockIdx.y;
-    if (pl.info->status == 0) {
-        const int q = pl.info->q, c = pl.info->c;
-        const int N = D->n[i1] * D->r[i1 + 1];
-        if (tm * GT < q) {
-            for (int t = tn; t * GT < N; t += gridDim.y) {
-                GV A{ws + pl.o_Rn, pl.CT, 1};
-                GV B{D->core[i1], 1, c};
-                gemm_tile(A, B, D->alt[i1], 1, q, q, N, c, tm, t);
-            }
-        }
-    }
+    extern __shared__ double sm[];
+    const int q = pl.info->q, c = pl.info->c;
+    const long long N = (long long)D->n[i1] * D->r[i1 + 1];
+    if (pl.info->status == 0)
+        slab_mul<CB>(ws + pl.o_Rn, pl.CT, 1, q, c, D->core[i1], 1, c, N, D->alt[i1], 1, q, blockIdx.x, gridDim.x, sm);
     fin_last_block(D, fin, pl.info);
 }
 
-// core[i-1] <- core[i-1] * US   (US = c x rank, column-major ld CT)
-__global__ void __launch_bounds__(256) k_gemm_xm(DevDesc* D, int im1, Plan pl, double* ws, Fin fin) {
+// core[i-1] <- core[i-1] * US   (US = c x rank, column-major ld CT), as its transpose US^T core^T
+template <int CB>
+__global__ void __launch_bounds__(256, Slab<CB>::PER_SM) k_gemm_xm(DevDesc* D, int im1, Plan pl, double* ws, Fin fin) {
     PTT_PDL_ENTRY();
-    const int tn = blockIdx.y;
-    if (pl.info->status == 0) {
-        const int c = pl.info->c, rank = pl.info->rank;
-        const int M = D->r[im1] * D->n[im1];
-        if (tn * GT < rank) {
-            for (int t = blockIdx.x; t * GT < M; t += gridDim.x) {
-                GV A{D->core[im1], 1, M};
-                GV B{ws + pl.o_US, 1, pl.CT};
-                gemm_tile(A, B, D->alt[im1], 1, M, M, rank, c, t, tn);
-            }
-        }
-    }
+    extern __shared__ double sm[];
+    const int c = pl.info->c, rank = pl.info->rank;
+    const long long M = (long long)D->r[im1] * D->n[im1];
+    if (pl.info->status == 0)
+        slab_mul<CB>(ws + pl.o_US, pl.CT, 1, rank, c, D->core[im1], M, 1, M, D->alt[im1], M, 1, blockIdx.x, gridDim.x,
+                     sm);
     fin_last_block(D, fin, pl.info);
 }
 
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(256) k_gemm_xm(DevDesc* D, int im1, Plan pl, d
 // and the descriptor are read together, every warp takes 8 columns (rows) with
 // both operands' fragments straight from memory -- all its loads in flight at
 // once, no shared memory, no barrier before the ticket -- and only the tiles
-// that exist are multiplied.  The k order is gemm_tile's: the same bits.  A
+// that exist are multiplied.  A
 // launch of a 40-dimensional step (n = 256, ranks to 16) in its chain: 5.3 us
 // with 64 x 64 tiles, 2.6 here; 5120 x 20 columns 7.1 and 3.8.
 struct WGemm {
@@ -708,6 +712,10 @@ static int set_attrs() {
     }
     PTT_CUDA(cudaFuncSetAttribute(k_svd_replay, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)replay_smem<128>()));
+    constexpr int SB = CT < 64 ? 64 : CT;
+    PTT_CUDA(cudaFuncSetAttribute(k_gemm_rx<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
+    PTT_CUDA(cudaFuncSetAttribute(k_gemm_xm<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
+    PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_write<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
     if constexpr (CT >= 64) {
         PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_rows<CT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)gq::Cfg<CT>::SM_ROWS));
@@ -793,6 +801,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     const int d = x->d;
     int rc = set_attrs<CT>();
     if (rc) return rc;
+    constexpr int SB = CT < 64 ? 64 : CT;  // tile bound of the contractions
     const bool use_gq = CT >= 64 && !c->no_cholqr;
     // plan: largest leaf count over all bonds decides the workspace
     const int KC = (CT + KG - 1) / KG * KG;
@@ -896,8 +905,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         if ((rc = launch_factor<CT>(c, x, i, LEFT, pl, ws, g, mcap))) return rc;
         if ((rc = launch_apply<CT>(c, x, i, LEFT, pl, ws, &info->q, CT))) return rc;
         const long long ncap = (long long)x->n[i + 1] * rk[i + 2];
-        int gy = (int)((ncap + GT - 1) / GT);
-        if (gy > 4096) gy = 4096;
+        const int gy = (int)((ncap + 63) / 64 > 4096 ? 4096 : (ncap + 63) / 64);
         // then the rank q and the swap of both rewritten cores
         if (c->ozaki && CT <= oz::KG) {  // one wave, R split once per CTA
             PTT_CUDA(ptt_launch(c, k_gemm_rx_oz, dim3(1, gy < c->nsm ? gy : c->nsm), dim3(256), oz::SMEM_GEMM,
@@ -905,8 +913,8 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             PTT_LAUNCHED(c);
             if ((rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
         } else {
-            PTT_CUDA(ptt_launch(c, k_gemm_rx, dim3((CT + GT - 1) / GT, gy), dim3(256), 0, x->dd, i + 1, pl, ws,
-                                Fin{tmain, i + 1, i + 1, &info->q, i}));
+            PTT_CUDA(ptt_launch(c, k_gemm_rx<SB>, dim3(slab_ctas<SB>(ncap, c->nsm)), dim3(256), Slab<SB>::SMEM, x->dd,
+                                i + 1, pl, ws, Fin{tmain, i + 1, i + 1, &info->q, i}));
             PTT_LAUNCHED(c);
             if (!tmain && (rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
         }
@@ -945,10 +953,8 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             int r2 = launch_apply<CT>(c, x, i, RIGHT_T, pl, ws, &info->rank, CT);
             if (r2) return r2;
             if (g) {  // Q V_r for a bond the grid Cholesky QR finished
-                int gx = (int)((mcap + GT - 1) / GT);
-                gx = gx < 1 ? 1 : (gx > 4096 ? 4096 : gx);
-                PTT_CUDA(ptt_launch(c, gq::k_gq_write, dim3(gx, (CT + GT - 1) / GT), dim3(gq::NT), 0, x->dd, i, pl, *g,
-                                    ws, Fin{ttail, -1, i, &info->rank}));
+                PTT_CUDA(ptt_launch(c, gq::k_gq_write<SB>, dim3(slab_ctas<SB>(mcap, c->nsm)), dim3(256), Slab<SB>::SMEM,
+                                    x->dd, i, pl, *g, ws, Fin{ttail, -1, i, &info->rank}));
                 PTT_LAUNCHED(c);
                 if (ttail) return PTT_OK;
             }
@@ -978,16 +984,15 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
         }
         // core i - 1 times U_r S_r, then the new rank r_i and the swap of core i - 1
         const long long mcap2 = (long long)rk[i - 1] * x->n[i - 1];
-        int gx = (int)((mcap2 + GT - 1) / GT);
-        if (gx > 4096) gx = 4096;
+        const int gx = (int)((mcap2 + 63) / 64 > 4096 ? 4096 : (mcap2 + 63) / 64);
         if (c->ozaki && CT <= oz::KG) {  // one wave, U_r S_r split once per CTA
             PTT_CUDA(ptt_launch(c, k_gemm_xm_oz, dim3(1, gx < c->nsm ? gx : c->nsm), dim3(256), oz::SMEM_GEMM, x->dd,
                                 i - 1, pl, ws));
             PTT_LAUNCHED(c);
             if ((rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
         } else {
-            PTT_CUDA(ptt_launch(c, k_gemm_xm, dim3(gx, (CT + GT - 1) / GT), dim3(256), 0, x->dd, i - 1, pl, ws,
-                                Fin{tmain, i, i - 1, &info->rank}));
+            PTT_CUDA(ptt_launch(c, k_gemm_xm<SB>, dim3(slab_ctas<SB>(mcap2, c->nsm)), dim3(256), Slab<SB>::SMEM, x->dd,
+                                i - 1, pl, ws, Fin{tmain, i, i - 1, &info->rank}));
             PTT_LAUNCHED(c);
             if (!tmain && (rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
         }
@@ -1241,7 +1246,7 @@ static int round_impl_w(ptt_tt* x, const int* rk, double delta, const int* maxr,
                 if ((rc = factor(i, LEFT, Wl[i], pl, wsb))) return rc;
                 Wmax = Wl[i] > Wmax ? Wl[i] : Wmax;
                 const long long ncap = (long long)x->n[i + 1] * rk[i + 2];
-                int gy = (int)((ncap + GT - 1) / GT);
+                int gy = (int)((ncap + 63) / 64);
                 if (gy > 4096) gy = 4096;
                 // the contraction's last block publishes the rank and swaps the core
                 const int cb = cbound(rk[i + 1]);
@@ -1269,7 +1274,7 @@ static int round_impl_w(ptt_tt* x, const int* rk, double delta, const int* maxr,
                 ptt_time_end(c, PTT_TIME_SVD);
                 PTT_LAUNCHED(c);
                 const long long mcap = (long long)rk[i - 1] * x->n[i - 1];
-                int gx = (int)((mcap + GT - 1) / GT);
+                int gx = (int)((mcap + 63) / 64);
                 if (gx > 4096) gx = 4096;
                 const int cb = cbound(rk[i]);
                 auto kern = cb == 16 ? k_wgemm_xm<2> : (cb == 24 ? k_wgemm_xm<3> : k_wgemm_xm<4>);
