@@ -210,16 +210,74 @@ __global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int m
 #include "ptt_svd.cuh"
 
 // Rebuild rows of V (q x q, V = product of the recorded rotations) and write
-// V_r = V[:, order[0:rank]] into Bn[root].  One warp per row; each sweep's
-// rotation table is staged in shared memory once per block, the column pair
-// of each (round, pair) slot is tabulated once for all sweeps.
+// V_r = V[:, order[0:rank]] into Bn[root].  One warp per row, PP pairs a lane.
+// The chain of a row is what counts (a step reads two entries, multiplies and
+// writes them: about 100 cycles, 500 steps at 64 columns), so everything else
+// is off it: the rotations come from memory into registers RD steps ahead, the
+// pair's columns (tabulated once for all sweeps) one step ahead.  With the
+// table of each sweep staged in shared memory and both looked up inside the
+// step it took 117 us at 64 columns.
+template <int PP>
+__device__ __forceinline__ void svd_replay_rows(double* vrow, const unsigned short* cols, int npair, int npr, int nrd,
+                                                int sweeps, const double2* rot, long long per_sweep) {
+    constexpr int RD = 8;
+    const int lane = threadIdx.x & 31, total = sweeps * nrd;
+    double2 r[RD][PP];
+    const double2* next = rot + lane;  // rotations of the next step to request
+    int nleft = nrd;                   // steps left in its sweep
+    auto request = [&](double2 (&d)[PP]) {
+#pragma unroll
+        for (int u = 0; u < PP; u++) d[u] = lane + 32 * u < npr ? next[32 * u] : make_double2(1.0, 0.0);
+        next += npair;
+        if (--nleft == 0) {
+            nleft = nrd;
+            next += per_sweep - (long long)nrd * npair;
+        }
+    };
+#pragma unroll
+    for (int t = 0; t < RD; t++)
+        if (t < total) request(r[t]);
+    unsigned short pq[PP];
+    int rd = 0;
+    auto columns = [&]() {
+#pragma unroll
+        for (int u = 0; u < PP; u++) pq[u] = lane + 32 * u < npr ? cols[rd * npair + lane + 32 * u] : 0;
+        rd = rd + 1 == nrd ? 0 : rd + 1;
+    };
+    columns();
+    for (int t0 = 0; t0 < total; t0 += RD) {
+#pragma unroll
+        for (int u8 = 0; u8 < RD; u8++) {
+            if (t0 + u8 >= total) break;  // uniform
+            double2 w[PP];
+            unsigned short c[PP];
+#pragma unroll
+            for (int u = 0; u < PP; u++) {
+                w[u] = r[u8][u];
+                c[u] = pq[u];
+            }
+#pragma unroll
+            for (int u = 0; u < PP; u++)
+                if (w[u].y != 0.0) {  // (cos, tan)
+                    const int pc = c[u] & 255, qc = c[u] >> 8;
+                    const double x = vrow[pc], y = vrow[qc];
+                    vrow[pc] = w[u].x * fma(-w[u].y, y, x);
+                    vrow[qc] = w[u].x * fma(w[u].y, x, y);
+                }
+            if (t0 + u8 + RD < total) request(r[u8]);
+            columns();
+            __syncwarp();
+        }
+    }
+}
+
 __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, int bx) {
     extern __shared__ double sm[];
     const int CT = pl.CT, KC = pl.KC;
     const int SR = CT + 2;
     const int npair = (CT + 2) / 2;
-    double* vrow = sm + (threadIdx.x >> 5) * SR;   // 8 rows
-    double2* tab = (double2*)(sm + 8 * SR);         // (CT+1) rounds x npair
+    double* vrow = sm + (threadIdx.x >> 5) * SR;  // 8 rows
+    unsigned short* cols = (unsigned short*)(sm + 8 * SR);  // (CT + 1) steps x npair
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = bx * 8 + warp;
     if (info->status) return;
@@ -229,41 +287,24 @@ __device__ void svd_replay_body(const Plan& pl, double* ws, const Info* info, in
     const int G = order == ORD_RING ? (Gc > 1 ? 1 << (32 - __clz(Gc - 1)) : 1) : Gc;
     const int npr = 2 * G, nrd = 4 * G - 1;
     const int* perm = (const int*)(ws + pl.o_sig + CT) + CT;
-    // the column pair of every (step, pair) slot, once for all sweeps
-    unsigned char* pcol = (unsigned char*)(tab + (CT + 1) * npair);
-    unsigned char* qcol = pcol + (CT + 1) * npair;
+    // the columns of V of every (step, pair) slot; beyond qa (never rotated): CT
     for (int e = threadIdx.x; e < nrd * npr; e += blockDim.x) {
         const int rd = e / npr, i = e - (e / npr) * npr;
         int pc, qc;
         svd_pair(i, rd, G, order, &pc, &qc);
-        // slots of the log to columns of V; beyond qa (never rotated): CT
-        pcol[rd * npair + i] = (unsigned char)(pc < qa ? perm[pc] : CT);
-        qcol[rd * npair + i] = (unsigned char)(qc < qa ? perm[qc] : CT);
+        cols[rd * npair + i] = (unsigned short)((pc < qa ? perm[pc] : CT) | (qc < qa ? perm[qc] : CT) << 8);
     }
     for (int j = lane; j < SR; j += 32) vrow[j] = (j == row) ? 1.0 : 0.0;
-    const double2* rot = (const double2*)(ws + pl.o_rot);
-    for (int sw = 0; sw < sweeps; sw++) {
-        __syncthreads();
-        const long long base = (long long)sw * (CT + 1) * npair;
-        const int cnt = nrd * npair;
-        for (int e = threadIdx.x; e < cnt; e += blockDim.x) tab[e] = rot[base + e];
-        __syncthreads();
-        if (row < q) {
-            for (int rd = 0; rd < nrd; rd++) {
-                for (int i = lane; i < npr; i += 32) {
-                    const double2 r = tab[rd * npair + i];
-                    if (r.y != 0.0) {
-                        const int pc = pcol[rd * npair + i], qc = qcol[rd * npair + i];
-                        const double x = vrow[pc], y = vrow[qc];
-                        vrow[pc] = r.x * fma(-r.y, y, x);  // (cos, tan)
-                        vrow[qc] = r.x * fma(r.y, x, y);
-                    }
-                }
-                __syncwarp();
-            }
-        }
-    }
     __syncthreads();
+    if (row < q && sweeps > 0) {
+        const double2* rot = (const double2*)(ws + pl.o_rot);
+        const long long per = (long long)(CT + 1) * npair;
+        if (npr <= 32)
+            svd_replay_rows<1>(vrow, cols, npair, npr, nrd, sweeps, rot, per);
+        else
+            svd_replay_rows<2>(vrow, cols, npair, npr, nrd, sweeps, rot, per);
+    }
+    __syncwarp();
     if (row >= CT) return;
     const int* ord = (const int*)(ws + pl.o_sig + CT);
     double* B = ws + pl.o_Bn + (long long)row * KC;
@@ -687,12 +728,10 @@ static size_t apply_smem() {
     const int VR = CT > H ? CT : H;
     return sizeof(double) * ((size_t)CT * KG + (size_t)VR * (CT + 1));
 }
-// 8 V rows + one sweep's rotation table ((CT+1) rounds x (CT+2)/2 pairs)
+// 8 rows of V and the columns (two bytes) of a sweep's (CT + 1) x (CT + 2) / 2 pairs
 template <int CT>
 static size_t replay_smem() {
-    // 8 rows of V, one sweep's rotations, the two column tables (bytes)
-    return sizeof(double) * (8 * (size_t)(CT + 2) + 2 * (size_t)(CT + 1) * ((CT + 2) / 2)) +
-           2 * (size_t)(CT + 1) * ((CT + 2) / 2);
+    return sizeof(double) * 8 * (size_t)(CT + 2) + 2 * (size_t)(CT + 1) * ((CT + 2) / 2);
 }
 
 template <int CT>
