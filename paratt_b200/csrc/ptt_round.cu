@@ -22,6 +22,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <type_traits>
+
 using namespace tsqr;
 
 namespace {
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int m
 // is off it: the rotations come from memory into registers RD steps ahead, the
 // pair's columns (tabulated once for all sweeps) one step ahead.  With the
 // table of each sweep staged in shared memory and both looked up inside the
-// step it took 117 us at 64 columns.
+// step it took 117 us at 64 columns, now 49.
 template <int PP>
 __device__ __forceinline__ void svd_replay_rows(double* vrow, const unsigned short* cols, int npair, int npr, int nrd,
                                                 int sweeps, const double2* rot, long long per_sweep) {
@@ -335,8 +337,8 @@ __global__ void __launch_bounds__(256) k_svd_replay_b(Plan pl, double* ws, long 
 // tile's issued as the products use up this one's.  k runs in the order 8 b + 2 q
 // + s (lane q of four, step s), so a group of four lanes reads 64 contiguous
 // bytes whichever index of B is contiguous.  64 x 64 x 16 tiles staged through
-// shared memory took 18.2 us (R x core), 14.5 (core x U_r S_r) and 12.1 (Q V_r)
-// at 16384 x 64.
+// shared memory took 18.4 us (R x core), 14.7 (core x U_r S_r) and 12.1 (Q V_r)
+// at 16384 x 64; now 11.2, 11.3 and 6.9.
 // ---------------------------------------------------------------------------
 template <int CB>
 struct Slab {
@@ -407,6 +409,18 @@ __device__ __forceinline__ void slab_mul(const double* S, int srs, int scs, int 
             if (row < s && col + 1 < N) C[row * crs + (col + 1) * ccs] = d[r][1];
         }
     }
+}
+
+// f(std::integral_constant<int, CB>) with the smallest CB that holds the bond's
+// ranks: a small bond of a wide train then leaves shared memory and registers to
+// the kernels beside it (the lanes of a batch: 12 trains of ranks to 96 in 55.6
+// ms, 58.0 with the 128-wide kernels for every bond).
+template <typename F>
+static int slab_dispatch(int bound, F f) {
+    if (bound <= 32) return f(std::integral_constant<int, 32>{});
+    if (bound <= 64) return f(std::integral_constant<int, 64>{});
+    if (bound <= 96) return f(std::integral_constant<int, 96>{});
+    return f(std::integral_constant<int, 128>{});
 }
 
 // CTAs of such a launch for at most ncap columns
@@ -751,10 +765,17 @@ static int set_attrs() {
     }
     PTT_CUDA(cudaFuncSetAttribute(k_svd_replay, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)replay_smem<128>()));
-    constexpr int SB = CT < 64 ? 64 : CT;
-    PTT_CUDA(cudaFuncSetAttribute(k_gemm_rx<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
-    PTT_CUDA(cudaFuncSetAttribute(k_gemm_xm<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
-    PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_write<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<SB>::SMEM));
+    if constexpr (CT == 128) {
+        for (int cb : {96, 128}) {
+            const int err = slab_dispatch(cb, [&](auto b) -> int {
+                constexpr int CB = decltype(b)::value;
+                for (auto f : {(const void*)k_gemm_rx<CB>, (const void*)k_gemm_xm<CB>, (const void*)gq::k_gq_write<CB>})
+                    PTT_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slab<CB>::SMEM));
+                return PTT_OK;
+            });
+            if (err) return err;
+        }
+    }
     if constexpr (CT >= 64) {
         PTT_CUDA(cudaFuncSetAttribute(gq::k_gq_rows<CT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)gq::Cfg<CT>::SM_ROWS));
@@ -840,7 +861,6 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     const int d = x->d;
     int rc = set_attrs<CT>();
     if (rc) return rc;
-    constexpr int SB = CT < 64 ? 64 : CT;  // tile bound of the contractions
     const bool use_gq = CT >= 64 && !c->no_cholqr;
     // plan: largest leaf count over all bonds decides the workspace
     const int KC = (CT + KG - 1) / KG * KG;
@@ -952,8 +972,13 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             PTT_LAUNCHED(c);
             if ((rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
         } else {
-            PTT_CUDA(ptt_launch(c, k_gemm_rx<SB>, dim3(slab_ctas<SB>(ncap, c->nsm)), dim3(256), Slab<SB>::SMEM, x->dd,
-                                i + 1, pl, ws, Fin{tmain, i + 1, i + 1, &info->q, i}));
+            rc = slab_dispatch(rk[i + 1], [&](auto b) -> int {
+                constexpr int CB = decltype(b)::value;
+                PTT_CUDA(ptt_launch(c, k_gemm_rx<CB>, dim3(slab_ctas<CB>(ncap, c->nsm)), dim3(256), Slab<CB>::SMEM,
+                                    x->dd, i + 1, pl, ws, Fin{tmain, i + 1, i + 1, &info->q, i}));
+                return PTT_OK;
+            });
+            if (rc) return rc;
             PTT_LAUNCHED(c);
             if (!tmain && (rc = finalize(i + 1, i, i + 1, &info->q, info))) return rc;
         }
@@ -992,8 +1017,13 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             int r2 = launch_apply<CT>(c, x, i, RIGHT_T, pl, ws, &info->rank, CT);
             if (r2) return r2;
             if (g) {  // Q V_r for a bond the grid Cholesky QR finished
-                PTT_CUDA(ptt_launch(c, gq::k_gq_write<SB>, dim3(slab_ctas<SB>(mcap, c->nsm)), dim3(256), Slab<SB>::SMEM,
-                                    x->dd, i, pl, *g, ws, Fin{ttail, -1, i, &info->rank}));
+                r2 = slab_dispatch(rk[i], [&](auto b) -> int {
+                    constexpr int CB = decltype(b)::value;
+                    PTT_CUDA(ptt_launch(c, gq::k_gq_write<CB>, dim3(slab_ctas<CB>(mcap, c->nsm)), dim3(256),
+                                        Slab<CB>::SMEM, x->dd, i, pl, *g, ws, Fin{ttail, -1, i, &info->rank}));
+                    return PTT_OK;
+                });
+                if (r2) return r2;
                 PTT_LAUNCHED(c);
                 if (ttail) return PTT_OK;
             }
@@ -1030,8 +1060,13 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
             PTT_LAUNCHED(c);
             if ((rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
         } else {
-            PTT_CUDA(ptt_launch(c, k_gemm_xm<SB>, dim3(slab_ctas<SB>(mcap2, c->nsm)), dim3(256), Slab<SB>::SMEM, x->dd,
-                                i - 1, pl, ws, Fin{tmain, i, i - 1, &info->rank}));
+            rc = slab_dispatch(rk[i], [&](auto b) -> int {
+                constexpr int CB = decltype(b)::value;
+                PTT_CUDA(ptt_launch(c, k_gemm_xm<CB>, dim3(slab_ctas<CB>(mcap2, c->nsm)), dim3(256), Slab<CB>::SMEM,
+                                    x->dd, i - 1, pl, ws, Fin{tmain, i, i - 1, &info->rank}));
+                return PTT_OK;
+            });
+            if (rc) return rc;
             PTT_LAUNCHED(c);
             if (!tmain && (rc = finalize(i, i - 1, -1, &info->rank, info))) return rc;
         }
