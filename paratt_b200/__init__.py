@@ -193,7 +193,7 @@ class Context:
         _check(lib().ptt_ctx_fixed_plans(self.h, 1 if on else 0))
 
     def cholqr(self, on=True):
-        """Cholesky-QR factorisation of unfoldings with <= 32 columns (default
+        """Cholesky-QR factorisation of unfoldings with <= 128 columns (default
         on; off = Householder TSQR only)."""
         _check(lib().ptt_ctx_cholqr(self.h, 1 if on else 0))
 

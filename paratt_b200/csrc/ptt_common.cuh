@@ -79,7 +79,7 @@ struct ptt_ctx {
     // captured launch sequences (ptt_graph_run): on/off and the cache
     int graphs;
     void* graph_cache;
-    // Cholesky-QR factorisation of unfoldings with <= 32 columns: 0 = used
+    // Cholesky-QR factorisation of unfoldings with <= 128 columns: 0 = used
     // (default), 1 = Householder TSQR only; device counters [finished,
     // fell back, Gram stages of the finished ones]
     int no_cholqr;

@@ -208,8 +208,10 @@ __device__ __forceinline__ void gram_fp64(const double* Xs, int h, int nbc, doub
 // Ozaki split on the fifth-generation tensor cores (ptt_ozaki.cuh) instead
 // of FP64 mma (64 columns only).
 // Bound by latency: at 111 rows x 64 columns the loads, the solve's chain of
-// 8 blocks and 126 products a warp.  One stage at 16384 x 64 (first / later
-// stages): see the figures in k_gq_decide.
+// 8 blocks and 126 products a warp.  One stage takes 10 us at 16384 x 64 (23 at
+// 9696 x 95) beside 23 (38) of k_gq_decide; a factorisation is two stages there
+// and took 187 us with 3.6 stages whose last CTA summed and factored alone
+// (2600 with the Householder tree at 95 columns).
 template <int CB, bool OZ>
 __global__ void __launch_bounds__(NT, 1) k_gq_rows(const DevDesc* D, int k, int mode, Plan pl, GQ g, int stage) {
     PTT_PDL_ENTRY();
@@ -387,7 +389,9 @@ __device__ void chol_tiles(double* sG, int nbc, int c, const unsigned char* aliv
 }
 
 // Sum of the partial Gram matrices (CTA t: tile t) and, in the last CTA to
-// finish, the decision of the stage.
+// finish, the decision of the stage.  What counts is that CTA's chain after the
+// sums: the norms and tests, the c-step Cholesky (a warp's 8 x 8 tile, then all
+// warps' solves and updates, one barrier each) and the accumulated R.
 template <int CB>
 __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, int mode, Plan pl, GQ g, double* ws,
                                                      int stage, long long* qstat) {
