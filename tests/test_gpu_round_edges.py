@@ -21,6 +21,7 @@ CASES = [
     ([40, 600, 9], [1, 40, 9, 1], [1, 33, 8, 1], 64),       # 64-wide contractions, ranks on both sides of 8
     ([70, 19, 65], [1, 63, 65, 1], [1, 31, 33, 1], 64),     # 128-wide
     ([127, 9, 128], [1, 127, 121, 1], [1, 64, 57, 1], 128),
+    ([40, 5000, 40], [1, 32, 32, 1], [1, 9, 17, 1], 64),    # 160000 rows: the block-level tree at 32 columns
 ]
 
 
