@@ -379,18 +379,20 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
     }
     cl.sync();  // no CTA leaves while another may still read its partials
     if (dec == DONE) {
+        // a column dropped by the deciding stage is still in Xs: zero in Q, as its row of R
         if (mode == LEFT) {
             double* out = D->alt[k];
             for (int col = warp; col < c; col += NT / 32) {
                 double* g = out + (long long)r0 + (long long)col * m;
-                for (int row = lane; row < h; row += 32) g[row] = Xs[row * XP + col];
+                const bool on = (live >> col) & 1u;
+                for (int row = lane; row < h; row += 32) g[row] = on ? Xs[row * XP + col] : 0.0;
             }
         } else {
             double* out = A.p + (long long)r0 * c;  // in place over A: this CTA's rows only
             const int dq = NT / c, dr = NT - dq * c, tot = h * c;
             int row = tid / c, col = tid - row * c;
             for (int f = tid; f < tot; f += NT) {
-                out[f] = Xs[row * XP + col];
+                out[f] = (live >> col) & 1u ? Xs[row * XP + col] : 0.0;
                 row += dq;
                 col += dr;
                 if (col >= c) {
@@ -403,7 +405,6 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
             double* Rs = wsb + wp.o_R;  // root slot, row-major 32 x 32
             for (int e = tid; e < 1024; e += NT) {
                 const int i = e >> 5, j = e & 31;
-                // a column dropped by the deciding stage takes its row of R with it
                 Rs[e] = (i < c && j < c && j >= i && ((live >> i) & 1u)) ? sT[telem(i, j)] : 0.0;
             }
             if (tid == 0) {

@@ -12,7 +12,12 @@
 //     Unfoldings of sums are numerically rank-deficient: without this the
 //     noise directions kept the sequence busy for up to eight stages, and 11
 //     of the 78 factorisations of a rank-64 rounding with d = 40 fell back;
-//   * s >= 1 and max|G - I| <= TAU over the other columns: done, R = T;
+//   * s >= 1 and max|G - I| <= TAU over the other columns: done, R = T.  A
+//     column that this very stage drops was not part of that test and may lie
+//     along the others (|q_j q_i| to 1e-8 seen), and a caller may use Q as a
+//     projector without R: it is cleared before Q is final (the cluster masks
+//     it as it writes Q; the grid, whose Q_s is in memory already, finishes by
+//     the first-order factor, whose inverse pivot is zero there);
 //   * s >= 1 and max|G - I| <= FIRST: R_{s+1} = I + striu(E) + diag(E)/2 with E
 //     = G - I, the Cholesky factor of I + E to first order; when max|E| <=
 //     FIRST_DONE that finishes without another Gram stage;

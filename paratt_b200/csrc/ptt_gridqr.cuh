@@ -491,6 +491,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
         s_tm[j] = 0ull;
         if (j < c && !(gjj >= 0.0 && gjj < LARGE)) atomicOr(&s_flags, 1);      // NaN, Inf or near overflow
         if (j < c && gjj != 0.0 && gjj < SMALL) atomicOr(&s_flags, 1);
+        if (gjj > 0.0 && !on) atomicOr(&s_flags, 2);  // dropped by this stage: q_j is still in Q_s
         const unsigned bits = __ballot_sync(0xffffffffu, on);
         if ((lane & 7) == 0) s_alive[j >> 3] = (unsigned char)((bits >> lane) & 0xffu);
         if (lane == 0 && j < c) atomicAdd(&s_nd, __popc(bits));
@@ -517,9 +518,9 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
     for (int w = 0; w < NT / 32; w++) emax = fmax(emax, s_red[w]);
     int nst = (stage == 0) ? 0 : ldcg(&st->nst);
     int dec;
-    if (s_flags || nlive == 0) {
+    if ((s_flags & 1) || nlive == 0) {
         dec = FALLBACK;
-    } else if (stage >= 1 && emax <= TAU) {
+    } else if (stage >= 1 && emax <= TAU && !(s_flags & 2)) {
         dec = DONE;
     } else if (stage == MAXST - 1) {
         dec = FALLBACK;  // no launch left to apply another factor
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
             tile_of(t, &I, &J);
             const double2 v = *(const double2*)(sT + t * 64 + tix(li, 2 * lk));
             const int i = 8 * I + li, j = 8 * J + 2 * lk;
-            const bool oi = (s_alive[I] >> li) & 1;  // a column dropped in this stage takes its row of R with it
+            const bool oi = (s_alive[I] >> li) & 1;  // a zero q_j needs no row of R
             Rs[(long long)i * CB + j] = oi && j >= i ? v.x : 0.0;
             Rs[(long long)i * CB + j + 1] = oi && j + 1 >= i ? v.y : 0.0;
         }
