@@ -136,20 +136,21 @@ __device__ __forceinline__ double widen(float f, bool on) {
 // theta = sqrt((1 + cos 2theta) / 2), tan theta = sin 2theta / (1 + cos
 // 2theta) -- dd and ga scaled by the exponent of max(al, be).
 struct Pre {
-    double lim, lim9;  // squares of tol and of 1e-9, times al be
-    float ds;          // dd, scaled
-    int E;             // exponent field of max(al, be)
+    double lim, small;  // squared dot products: of a cosine of tol, and of a rotation that leaves the others alone
+    float ds;           // dd, scaled
+    int E;              // exponent field of max(al, be)
     bool big;
 };
-__device__ __forceinline__ Pre svd_pre(double al, double be, int thr, double tol2, bool act) {
+// gap2: see the stop rule of the sweeps
+__device__ __forceinline__ Pre svd_pre(double al, double be, int thr, double tol2, double gap2, bool act) {
     Pre r;
     const int ha = __double2hiint(al), hb = __double2hiint(be);
     r.big = act && min(ha, hb) > thr;
     r.E = max(ha, hb) & 0x7ff00000;
-    r.ds = scaled_float(be - al, r.E);
-    const double ab = al * be;
+    const double dd = be - al, ab = al * be;
+    r.ds = scaled_float(dd, r.E);
     r.lim = tol2 * ab;
-    r.lim9 = 1e-18 * ab;
+    r.small = fmin(1e-18 * ab, gap2 * (dd * dd));
     return r;
 }
 __device__ __forceinline__ void svd_angle(const Pre& r, double ga, bool on, double* t, double* cs) {
@@ -319,13 +320,22 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
         mx = norms();
         // (sqrt(q) * 2^-53)^2 * max |a_j|^2, compared by the high words
         const int thr = __double2hiint((double)q * 1.232595164407831e-32 * mx);
+        // The sweeps may end after one whose rotations all were small: cosine
+        // <= 1e-9 and tangent (ga / |dd| at that size) <= 1e-7.  A rotation by t
+        // adds t times the cosine of (q, r) to that of a pair (p, r) already
+        // zeroed, so what they leave is ~1e-16, as the single-precision angle
+        // leaves 1e-7 of each cosine.  The cosines alone do not tell: equal
+        // singular values make a tangent O(1) at any cosine, and stopping on
+        // them left a cluster's values wrong by 1e-10.  Only the sweep limit
+        // does without the tangents (infinity: fmin takes the other).
+        const double gap2 = sw < MAXSW - 1 ? 1e-14 : 1.0 / 0.0;
         int myrot = 0;
         double2* lg = rot + (long long)sw * (CT + 1) * npair + 2 * grp;
         // rotate two independent pairs of the group; log them as pairs 2 grp, 2 grp + 1
         auto step = [&](double(&x0)[NR], double(&y0)[NR], double& nx0, double& ny0, double(&x1)[NR], double(&y1)[NR],
                         double& nx1, double& ny1) {
             double g0 = dot_rows(x0, y0), g1 = dot_rows(x1, y1);
-            const Pre r0 = svd_pre(nx0, ny0, thr, tol2, act), r1 = svd_pre(nx1, ny1, thr, tol2, act);
+            const Pre r0 = svd_pre(nx0, ny0, thr, tol2, gap2, act), r1 = svd_pre(nx1, ny1, thr, tol2, gap2, act);
 #pragma unroll
             for (int o = LP / 2; o >= 1; o >>= 1) {
                 g0 += __shfl_xor_sync(FULL, g0, o);
@@ -350,8 +360,8 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
                 ny0 = fma(t0, g0, ny0);
                 nx1 = fma(-t1, g1, nx1);
                 ny1 = fma(t1, g1, ny1);
-                // bit 1: a rotation of a pair whose cosine exceeded 1e-9
-                myrot |= (on0 ? (q0 > r0.lim9 ? 3 : 1) : 0) | (on1 ? (q1 > r1.lim9 ? 3 : 1) : 0);
+                // bit 1: a rotation that was not small
+                myrot |= (on0 ? (q0 > r0.small ? 3 : 1) : 0) | (on1 ? (q1 > r1.small ? 3 : 1) : 0);
             }
             if (p == 0 && act) {
                 lg[0] = make_double2(c0, t0);
@@ -468,11 +478,7 @@ __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double*
             conv = true;
         } else {
             sweeps = sw + 1;
-            // cyclic Jacobi converges quadratically at the end: after a sweep
-            // whose cosines all stayed below 1e-9 the next one would only
-            // meet cosines ~1e-16 (the single-precision angles leave 1e-7 of
-            // each), so it is not run
-            if (!(any & 2)) conv = true;
+            if (!(any & 2)) conv = true;  // the next one would only meet cosines ~1e-16
         }
     }
     if (!conv && tid == 0) PTT_STATUS_SET(status, PTT_ERR_NUMERIC);
