@@ -148,8 +148,13 @@ __global__ void __launch_bounds__(DNT, 1) k_dot_part(const DevDesc* X, const Dev
                     if (t < nb1) dot_mma(c0[t], c1[t], av, Ys[(8 * t + li) * DP + k4 + lk]);
             }
 #pragma unroll
-            for (int t = 0; t < 8; t++)
-                if (t < nb1) *(double2*)(Ts + (8 * warp + li) * DP + 8 * t + 2 * lk) = make_double2(c0[t], c1[t]);
+            for (int t = 0; t < 8; t++) {
+                // rows past rx: zero, not the padding's 0 x y_j (NaN where y_j is not finite), which the
+                // second product would carry into a'
+                if (t < nb1)
+                    *(double2*)(Ts + (8 * warp + li) * DP + 8 * t + 2 * lk) =
+                        8 * warp + li < rx ? make_double2(c0[t], c1[t]) : make_double2(0.0, 0.0);
+            }
         }
         __syncthreads();
         if (8 * warp < rx1) {
