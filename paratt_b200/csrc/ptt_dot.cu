@@ -12,6 +12,8 @@
 
 #include <mutex>
 
+#include <string.h>
+
 // T[i, j, e] = sum_k a[i, k] * y[k, j, e]      (a: rx x ry, column-major ld rx)
 __global__ void k_dot_t(const DevDesc* X, const DevDesc* Y, int k, const double* a, double* T) {
     const int rx = X->r[k], ry = Y->r[k], n = X->n[k], ry1 = Y->r[k + 1];
@@ -267,23 +269,41 @@ extern "C" int ptt_dot(const ptt_tt* x, const ptt_tt* y, double* out) {
         PTT_CUDA(cudaEventRecord(y->ctx->ev_fork, y->ctx->stream));
         PTT_CUDA(cudaStreamWaitEvent(c->stream, y->ctx->ev_fork, 0));
     }
+    // The ranks decide, not the capacities: a state of rank 7 in buffers for 128
+    // takes the fused kernel, and the value does not depend on the buffers.  They
+    // are read back (two small copies, one wait) only where a capacity leaves it
+    // open.
+    int rx[PTT_MAX_DIM + 1], ry[PTT_MAX_DIM + 1], rc;
+    bool known = true;
+    for (int k = 0; k <= x->d; k++) {
+        rx[k] = x->rcap[k];
+        ry[k] = y->rcap[k];
+        known = known && rx[k] <= DR && ry[k] <= DR;
+    }
+    if (!known) {
+        const size_t bytes = sizeof(int) * (size_t)(x->d + 1);
+        int* h = (int*)c->h_scalars;  // 512 doubles
+        PTT_CUDA(cudaMemcpyAsync(h, x->dd->r, bytes, cudaMemcpyDeviceToHost, c->stream));
+        PTT_CUDA(cudaMemcpyAsync(h + PTT_MAX_DIM + 1, y->dd->r, bytes, cudaMemcpyDeviceToHost, c->stream));
+        PTT_CUDA(cudaStreamSynchronize(c->stream));
+        memcpy(rx, h, bytes);
+        memcpy(ry, h + PTT_MAX_DIM + 1, bytes);
+    }
     long long amax = 1, tmax = 1;
-    for (int k = 0; k <= x->d; k++) amax = (long long)x->rcap[k] * y->rcap[k] > amax ? (long long)x->rcap[k] * y->rcap[k] : amax;
+    for (int k = 0; k <= x->d; k++) amax = (long long)rx[k] * ry[k] > amax ? (long long)rx[k] * ry[k] : amax;
     for (int k = 0; k < x->d; k++) {
-        long long t = (long long)x->rcap[k] * x->n[k] * y->rcap[k + 1];
+        long long t = (long long)rx[k] * x->n[k] * ry[k + 1];
         tmax = t > tmax ? t : tmax;
     }
-    if (amax <= DR * DR && tmax < c->nsm * amax) tmax = c->nsm * amax;  // room for every CTA's partial: the sums
-                                                                       // do not depend on the capacities
+    if (amax <= DR * DR && tmax < c->nsm * amax) tmax = c->nsm * amax;  // room for every CTA's partial
     size_t bytes = sizeof(double) * (size_t)(2 * amax + tmax) + 1024;
-    int rc = ptt_ws_reserve(c, bytes);
-    if (rc) return rc;
+    if ((rc = ptt_ws_reserve(c, bytes))) return rc;
     double* A0 = (double*)c->ws;
     double* A1 = A0 + amax;
     double* T = A1 + amax;
     k_set_one<<<1, 1, 0, c->stream>>>(A0);
     PTT_LAUNCHED(c);
-    if ((rc = dot_chain(c, x, y, x->rcap, y->rcap, A0, A1, T, tmax, &A0))) return rc;
+    if ((rc = dot_chain(c, x, y, rx, ry, A0, A1, T, tmax, &A0))) return rc;
     PTT_CUDA(cudaMemcpyAsync(c->h_scalars, A0, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     rc = ptt_ctx_synchronize(c);
     if (rc) return rc;
@@ -426,7 +446,8 @@ extern "C" int ptt_dot_noalloc(const ptt_tt* x, const ptt_tt* y, double* out) {
     double* T = A1 + amax;
     k_set_one<<<1, 1, 0, c->stream>>>(A0);
     PTT_LAUNCHED(c);
-    if ((rc = dot_chain(c, x, y, rx, ry, A0, A1, T, tmax, &A0))) return rc;
+    // all the array has left: as many partials as ptt_dot takes, so the same sums (148 SMs x 64 x 64 would be more)
+    if ((rc = dot_chain(c, x, y, rx, ry, A0, A1, T, PTT_DOT_NOALLOC_MAX_DOUBLES - 2 * amax, &A0))) return rc;
     PTT_CUDA(cudaMemcpyAsync(c->h_scalars, A0, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     rc = ptt_ctx_synchronize(c);
     if (rc) return rc;

@@ -25,3 +25,22 @@ def test_infinite_entry(ctx, r, mode, side):
     assert X.dot_noalloc(Y) == np.inf
     X.close()
     Y.close()
+
+
+@pytest.mark.parametrize("dims,r,q", [([40, 5, 40, 4], 1, 1), ([256, 5, 150, 4], 7, 20), ([9, 5, 9, 4], 63, 64),
+                                      ([12, 5, 9, 4], 64, 64), ([16, 5, 9, 4], 20, 65)])
+def test_capacity_does_not_matter(ctx, dims, r, q):
+    """The same bits whatever the buffers hold, by either entry point."""
+    x = O.random_tt(dims, [1, r, max(1, r - 1), r, 1], 3, std=0.3)
+    y = O.random_tt(dims, [1, q, q, max(1, q - 3), 1], 4, std=0.3)
+    X, Y = P.TT.from_cores(ctx, x), P.TT.from_cores(ctx, y)
+    want = X.dot(Y)
+    assert abs(want - O.dot(x, y)) <= 1e-13 * O.norm(x) * O.norm(y)
+    assert X.dot_noalloc(Y) == want
+    for cx in (max(r, 64), 65, 128):
+        Z = P.TT.from_cores(ctx, x, [1] + [cx] * 3 + [1])
+        assert Z.dot(Y) == want
+        assert Z.norm() == X.norm()
+        Z.close()
+    X.close()
+    Y.close()
