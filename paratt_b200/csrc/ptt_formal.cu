@@ -68,8 +68,16 @@ __device__ __forceinline__ FiberIter fiber_iter(int R) {
 
 // Walk of a core by runs of JRUN consecutive fibers of one slab l, one warp
 // per run: one division per run instead of one per fiber, and the next
-// fiber's addresses by addition.
+// fiber's addresses by addition.  It pays for even ranks from 32 on, with runs
+// enough to occupy the GPU (counted over the launch as if its d cores were
+// alike).  The ranks are only known on the device, so a kernel that may walk by
+// runs holds the walk fiber by fiber as well; it is launched where a core's
+// capacities qualify, and its registers are held to 40 and 48 (six and five
+// blocks an SM): with 56 and 64 every other rank of such a train lost up to 13 %.
 constexpr int JRUN = 16;
+__host__ __device__ __forceinline__ bool by_runs(int d, int n, int rows, int slabs, int least) {
+    return (rows & 1) == 0 && rows >= 32 && (long long)((n + JRUN - 1) / JRUN) * slabs * d >= least;
+}
 struct RunIter {
     int t, step, runs, total;  // run t of `runs` per slab
 };
@@ -240,7 +248,16 @@ extern "C" int ptt_axpby(double a, const ptt_tt* x, double b, const ptt_tt* y, p
 // ---------------------------------------------------------------------------
 // hadamard: z_k[(ky + ry*ix), j, (ly + ry1*jx)] = x_k[ix, j, jx] * y_k[ky, j, ly]
 // ---------------------------------------------------------------------------
-__global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* newr, int* status) {
+// RUNS: a warp walks runs of fibers (j, lz), lz = ly + ry1 jx; lane: rows iz = 2
+// lane + 64 b and the next, iz = ky + ry ix, so the row's factors are found once
+// and every store is 16 bytes.  Bound by the writes (8 bytes per element; x and y
+// come from L1/L2): d = 40, n = 256, ranks 8 x 8, 336 MB: 140 us with a division
+// and an 8-byte store per element, 73 now (4.6 TB/s, 59 back to back).  With few
+// runs it is slower: 10 modes of 17, ranks 8 x 16 (2560 runs) 20.6 us a product,
+// 16.6 fiber by fiber; 20 modes of 100, ranks 4 x 8 (4480) 18.8 and 23.4.
+constexpr int RUNS_HADAMARD = 4096;
+template <bool RUNS>
+__device__ __forceinline__ void hadamard_core(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* newr, int* status) {
     const int k = blockIdx.y;
     const int d = X->d;
     const int rx = X->r[k], rx1 = X->r[k + 1], ry = Y->r[k], ry1 = Y->r[k + 1];
@@ -258,12 +275,7 @@ __global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* 
     const double* xc = X->core[k];
     const double* yc = Y->core[k];
     double* zc = Z->alt[k];
-    if ((rz & 1) == 0 && rz >= 32) {
-        // A warp walks runs of fibers (j, lz), lz = ly + ry1 jx; lane: rows iz =
-        // 2 lane + 64 b and the next, iz = ky + ry ix, so the row's factors are
-        // found once and every store is 16 bytes.  Bound by the writes (8 bytes
-        // per element; x and y come from L1/L2): d = 40, n = 256, ranks 8 x 8, 336
-        // MB: 144 us with a division and an 8-byte store per element, 58 now.
+    if (RUNS && by_runs(d, n, rz, rz1, RUNS_HADAMARD)) {
         const RunIter it = run_iter(n, rz1);
         const int lane = threadIdx.x & 31;
         for (int b = 2 * lane; b < rz; b += 64) {
@@ -274,7 +286,7 @@ __global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* 
                 const double* xf = xc + (long long)rx * (j0 + (long long)n * jx);
                 const double* yf = yc + (long long)ry * (j0 + (long long)n * ly);
                 double2* zf = (double2*)(zc + (long long)rz * (j0 + (long long)n * lz) + b);
-#pragma unroll 4
+#pragma unroll 2
                 for (int j = 0; j < h; j++)
                     __stcs(zf + (long long)(rz / 2) * j, make_double2(xf[rx * j + i0] * yf[ry * j + k0],
                                                                       xf[rx * j + i1] * yf[ry * j + k1]));
@@ -297,6 +309,13 @@ __global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* 
         }
     }
 }
+__global__ void k_hadamard(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* newr, int* status) {
+    hadamard_core<false>(X, Y, Z, newr, status);
+}
+__global__ void __launch_bounds__(256, 6) k_hadamard_runs(const DevDesc* X, const DevDesc* Y, DevDesc* Z, int* newr,
+                                                          int* status) {
+    hadamard_core<true>(X, Y, Z, newr, status);
+}
 
 extern "C" int ptt_hadamard(const ptt_tt* x, const ptt_tt* y, ptt_tt* z) {
     int rc = check_same_modes(x, y);
@@ -311,7 +330,10 @@ extern "C" int ptt_hadamard(const ptt_tt* x, const ptt_tt* y, ptt_tt* z) {
     long long mx = 0;
     for (int k = 0; k < d; k++) mx = z->cap[k] > mx ? z->cap[k] : mx;
     (void)mx;
-    k_hadamard<<<dim3(fiber_blocks(c, z, d), d), 256, 0, c->stream>>>(x->dd, y->dd, z->dd, newr, c->d_status);
+    bool runs = false;
+    for (int k = 0; k < d; k++) runs = runs || by_runs(d, x->n[k], need[k], need[k + 1], RUNS_HADAMARD);
+    auto kern = runs ? k_hadamard_runs : k_hadamard;
+    kern<<<dim3(fiber_blocks(c, z, d), d), 256, 0, c->stream>>>(x->dd, y->dd, z->dd, newr, c->d_status);
     PTT_LAUNCHED(c);
     return finalize(z, newr, 0, d, 1);
 }
@@ -504,7 +526,22 @@ __device__ __forceinline__ double sten_at(const double* xc, int r, int n, int i,
     return acc;
 }
 
-__global__ void k_opsum(const DevDesc* X, DevDesc* Y, Stencil st, double shift, int* newr, int* status) {
+// RUNS, a middle core and three points: a warp walks runs of fibers (j, l') of x
+// and writes both of y's fibers that come from each, [x; 0] and [S x; x]; the
+// stencil slides along the run in registers, so every fiber of x is read once
+// (plus two per run) and all accesses are 16 bytes.  Bound by HBM, four bytes
+// written per byte read: d = 40, n = 256, r = 64, 1.68 GB: 504 us with 8-byte
+// accesses, a division per fiber and the stencil's neighbours re-read, 267 now (6.3
+// TB/s).  At 2000 runs both take as long (10 modes of 17, rank 100: 25.6 us an
+// operator; fiber by fiber rank 96 takes 23.1); 40 modes of 32, rank 32 (2560)
+// 21.5, and rank 31 27.0 fiber by fiber.
+//   The stencil stays in the parameters (__grid_constant__): indexed through its
+// address, a plain parameter was first copied to 128 bytes of local memory by
+// every thread, 14 us of a launch of 4700 blocks.
+constexpr int RUNS_OPSUM = 2000;
+template <bool RUNS>
+__device__ __forceinline__ void opsum_core(const DevDesc* X, DevDesc* Y, const Stencil& st, double shift, int* newr,
+                                           int* status) {
     const int k = blockIdx.y;
     const int d = X->d;
     const int r = X->r[k], r1 = X->r[k + 1], n = X->n[k];
@@ -521,22 +558,14 @@ __global__ void k_opsum(const DevDesc* X, DevDesc* Y, Stencil st, double shift, 
     }
     const double* xc = X->core[k];
     double* yc = Y->alt[k];
-    if (d > 1 && k > 0 && k < d - 1 && (r & 1) == 0 && r >= 32 && st.len == 3) {
-        // A middle core: a warp walks runs of fibers (j, l') of x and writes both
-        // of y's fibers that come from each, [x; 0] and [S x; x]; the three-point
-        // stencil slides along the run in registers, so every fiber of x is read
-        // once (plus two per run) and all accesses are 16 bytes.  Bound by HBM,
-        // four bytes written per byte read: d = 40, n = 256, r = 64, 1.68 GB: 504
-        // us with 8-byte accesses, a division per fiber and the stencil's
-        // neighbours re-read, 280 now (6.0 TB/s).
+    if (RUNS && k > 0 && k < d - 1 && st.len == 3 && by_runs(d, n, r, r1, RUNS_OPSUM)) {
         const RunIter it = run_iter(n, r1);
-        const int lane = threadIdx.x & 31;
+        const int lane = threadIdx.x & 31, r2 = r >> 1;
         const double s0 = st.s[0], s1 = st.s[1], s2 = st.s[2];
         for (int b = 2 * lane; b < r; b += 64) {
             for (int t = it.t; t < it.total; t += it.step) {
                 const int l = t / it.runs, j0 = (t - l * it.runs) * JRUN, h = min(JRUN, n - j0);
                 const double2* xs = (const double2*)(xc + (long long)r * n * l + b);  // fiber j at xs[j r / 2]
-                const int r2 = r >> 1;
                 double2* ya = (double2*)(yc + (long long)ry * (j0 + (long long)n * l) + b);
                 double2* yb = ya + (long long)r * n * r1;  // the fiber l + r1
                 double2 xm = __ldg(xs + (long long)r2 * (j0 > 0 ? j0 - 1 : n - 1)), x0 = __ldg(xs + (long long)r2 * j0);
@@ -583,6 +612,14 @@ __global__ void k_opsum(const DevDesc* X, DevDesc* Y, Stencil st, double shift, 
         }
     }
 }
+__global__ void k_opsum(const DevDesc* X, DevDesc* Y, const __grid_constant__ Stencil st, double shift, int* newr,
+                        int* status) {
+    opsum_core<false>(X, Y, st, shift, newr, status);
+}
+__global__ void __launch_bounds__(256, 5) k_opsum_runs(const DevDesc* X, DevDesc* Y, const __grid_constant__ Stencil st,
+                                                       double shift, int* newr, int* status) {
+    opsum_core<true>(X, Y, st, shift, newr, status);
+}
 
 extern "C" int ptt_op_sum(const ptt_tt* x, const double* sten, int slen, double shift, ptt_tt* y) {
     int rc = check_same_modes(x, y);
@@ -601,7 +638,11 @@ extern "C" int ptt_op_sum(const ptt_tt* x, const double* sten, int slen, double 
     long long mx = 0;
     for (int k = 0; k < d; k++) mx = y->cap[k] > mx ? y->cap[k] : mx;
     (void)mx;
-    k_opsum<<<dim3(fiber_blocks(c, y, d), d), 256, 0, c->stream>>>(x->dd, y->dd, st, shift, newr, c->d_status);
+    bool runs = false;
+    for (int k = 1; k < d - 1 && st.len == 3; k++)
+        runs = runs || by_runs(d, x->n[k], x->rcap[k], x->rcap[k + 1], RUNS_OPSUM);
+    auto kern = runs ? k_opsum_runs : k_opsum;
+    kern<<<dim3(fiber_blocks(c, y, d), d), 256, 0, c->stream>>>(x->dd, y->dd, st, shift, newr, c->d_status);
     PTT_LAUNCHED(c);
     return finalize(y, newr, 0, d, 1);
 }
