@@ -87,22 +87,29 @@ __device__ void replay_geqrt(double* Rp, const double* Vb, const double* taus, i
     }
 }
 
-// out = Q B for the Householder tree: block (p, y) takes leaf p and 32 columns
-// of B and walks from the root down to its leaf, replaying the reflectors of
-// each node on its own copy of the node's rows in shared memory (the left
-// child takes the triangle's rows, the right child the eliminated ones), then
-// those of its leaf.  B is V_r at the root slot (RIGHT_T) or the identity
-// (LEFT).  The depth of the chain is that of one launch per level; the upper
-// nodes are replayed once per leaf below them, on SMs the level launches left
-// idle.  One launch instead of one for B, one per level and one for the
-// leaves: behind the grid Cholesky QR it is nearly always skipped, and then
-// its launches are all it costs (at 16384 x 64 seven of 1.0 us each, and 2 to
-// 5 us each of a lane's time in a batch; 64 trains of ranks to 96: 64.1 ms
-// with them, 58.1 without).
+// out = Q B for the Householder tree, a launch per range of its levels: block
+// (p, y) takes node p of level l1 (the leaves are level log2 P) and 32 columns of
+// B and walks down to it from its ancestor on level l0, replaying the reflectors
+// of each node on its own copy of the node's rows in shared memory (the left
+// child takes the triangle's rows, the right child the eliminated ones).  At a
+// leaf it replays the leaf's reflectors too and writes Q B; above, it replays its
+// own node and leaves both children's rows at their slots of Bn for the next
+// launch.  B is V_r at the root slot (RIGHT_T) or the identity (LEFT).
+//   Up to APPLY_LEAVES leaves one launch does it all: the chain is as deep as
+// with a launch per level, and the upper nodes, replayed once per leaf below
+// them, run on SMs that were idle.  Behind the grid Cholesky QR, which plans no
+// more leaves than that, the launch is nearly always skipped and is all the tree
+// costs (at 16384 x 64 seven launches of 1.0 us before, each 2 to 5 us of a
+// lane's time in a batch: 12 trains of ranks to 96 took 64.1 ms, then 58.1).
+//   With more leaves every SM is busy and the repeated replays cost time (1024
+// modes of ranks 128, Householder only, 512 leaves: a rounding took 59 ms with a
+// launch per level, 83 in one), so the launches after the first five levels
+// take one level each.
 // LEFT: out(row, col) at alt[row + m*col];  RIGHT_T: alt[row*k + col]
+constexpr int APPLY_LEAVES = 32;
 template <int CT>
 __global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int mode, Plan pl, double* ws,
-                                              const int* kptr) {
+                                              const int* kptr, int l0, int l1) {
     PTT_PDL_ENTRY();
     if (gq_finished(pl)) return;
     extern __shared__ double sm[];
@@ -129,21 +136,23 @@ __global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int m
     double* outp = D->alt[kcore];
     const long long ors = (mode == LEFT) ? 1 : kk;
     const long long ocs = (mode == LEFT) ? m : 1;
-    int r0, r1;
-    leaf_range(m, pl.L, pl.P, p, &r0, &r1);
+    int r0, r1;  // rows of the leaf, or of the node's first leaf (the empty leaves come last)
+    const int below = 31 - __clz(pl.P) - l1;
+    leaf_range(m, pl.L, pl.P, p << below, &r0, &r1);
     const int rows = r1 - r0;
     if (rows <= 0) return;
     const int rb = rows < c ? rows : c;
-    const int slot = pl.P - 1 + p;
-    const double* B = ws + pl.o_Bn;  // V_r, CT x KC
+    const int slot = (1 << l1) - 1 + p;
+    double* Bn = ws + pl.o_Bn;  // CT x KC a slot
+    const double* B = Bn + (long long)(((slot + 1) >> (l1 - l0)) - 1) * CT * pl.KC;
     for (int e = tid; e < CT * KG; e += NT) {
         const int a = e / KG, b = kg0 + e - a * KG;
-        Rp[e] = mode == LEFT ? (a == b && a < q ? 1.0 : 0.0) : B[(long long)a * pl.KC + b];
+        Rp[e] = mode == LEFT && l0 == 0 ? (a == b && a < q ? 1.0 : 0.0) : B[(long long)a * pl.KC + b];
     }
-    for (int l = 31 - __clz(pl.P); l > 0; l--) {
-        const int node = ((slot + 1) >> l) - 1;                       // ancestor l levels up
-        const bool right = ((((slot + 1) >> (l - 1)) - 1) & 1) == 0;  // its child on the path
-        if (pl.pass[node] != 0) continue;                             // one child without rows: nothing was eliminated
+    for (int l = l1 - l0; l >= (below > 0 ? 0 : 1); l--) {
+        const int node = ((slot + 1) >> l) - 1;                                // ancestor l levels up, or the node
+        const bool right = l > 0 && ((((slot + 1) >> (l - 1)) - 1) & 1) == 0;  // its child on the path
+        if (pl.pass[node] != 0) continue;  // the right child has no rows: nothing was eliminated
         const double* RR = ws + pl.o_Rn + (long long)(2 * node + 2) * CT * CT;
         double out[NHC][H / 8];
 #pragma unroll
@@ -170,7 +179,22 @@ __global__ void __launch_bounds__(NT) k_apply(const DevDesc* D, int kcore, int m
                     const int t = half * H + part + 8 * v;
                     if (t < CT) Rp[t * KG + col] = out[half][v];
                 }
+        } else if (l == 0) {
+            double* Bcr = Bn + (long long)(2 * node + 2) * CT * pl.KC;
+#pragma unroll
+            for (int half = 0; half < NHC; half++)
+#pragma unroll
+                for (int v = 0; v < H / 8; v++) {
+                    const int t = half * H + part + 8 * v;
+                    if (t < CT) Bcr[(long long)t * pl.KC + kg0 + col] = out[half][v];
+                }
         }
+    }
+    if (below > 0) {
+        double* Bcl = Bn + (long long)(2 * slot + 1) * CT * pl.KC;
+        __syncthreads();
+        for (int e = tid; e < CT * KG; e += NT) Bcl[(long long)(e / KG) * pl.KC + kg0 + e % KG] = Rp[e];
+        return;
     }
     const double* tau_leaf = ws + pl.o_tau_leaf + (long long)p * pl.KL * CT;
     const int ocol = kg0 + col;
@@ -723,7 +747,7 @@ static long long carve(Plan* pl, int PMAX, int LMAXKL) {
     pl->o_tau_leaf = take((long long)PMAX * LMAXKL * CT);
     pl->o_Rn = take((long long)(2 * PMAX - 1) * CT * CT);
     pl->o_tau_node = take((long long)PMAX * pl->NH * CT);
-    pl->o_Bn = take((long long)CT * KC);
+    pl->o_Bn = take((long long)(PMAX > APPLY_LEAVES ? 2 * PMAX - 1 : 1) * CT * KC);
     pl->o_US = take((long long)CT * CT);
     pl->o_rot = take((long long)MAXSW * (CT + 1) * ((CT + 2) / 2) * 2);
     pl->o_sig = take(2LL * CT + 64);
@@ -840,12 +864,16 @@ static int launch_factor(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, doubl
     return PTT_OK;
 }
 
-// out = Q B (k_apply); k columns read from *kptr, at most kcap.
+// out = Q B (k_apply); B and out have k columns, read from *kptr, at most kcap.
 template <int CT>
 static int launch_apply(ptt_ctx* c, ptt_tt* x, int k, int mode, Plan& pl, double* ws, const int* kptr, int kcap) {
-    PTT_CUDA(ptt_launch(c, k_apply<CT>, dim3(pl.P, (kcap + KG - 1) / KG), dim3(NT), apply_smem<CT>(),
-                        (const DevDesc*)x->dd, k, mode, pl, ws, kptr));
-    PTT_LAUNCHED(c);
+    const int depth = 31 - __builtin_clz((unsigned)pl.P);
+    for (int l0 = 0, l1; l0 <= depth; l0 = l1 + 1) {
+        l1 = pl.P <= APPLY_LEAVES ? depth : (l0 == 0 ? 4 : l0);
+        PTT_CUDA(ptt_launch(c, k_apply<CT>, dim3(1 << l1, (kcap + KG - 1) / KG), dim3(NT), apply_smem<CT>(),
+                            (const DevDesc*)x->dd, k, mode, pl, ws, kptr, l0, l1));
+        PTT_LAUNCHED(c);
+    }
     return PTT_OK;
 }
 
@@ -866,7 +894,7 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     const int KC = (CT + KG - 1) / KG * KG;
     int PMAX = 1, KLMAX = 1, NBMAX = 1;
     long long MQMAX = 1;
-    const int pmax = use_gq ? 32 : 512;
+    const int pmax = use_gq ? APPLY_LEAVES : 512;
     for (int i = 0; i < d; i++) {
         Plan t;
         long long ml = (long long)rk[i] * x->n[i], mr = (long long)x->n[i] * rk[i + 1];
