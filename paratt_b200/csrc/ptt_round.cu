@@ -889,39 +889,48 @@ static int round_impl(ptt_tt* x, const int* rk, double delta, const int* maxr, i
     const int d = x->d;
     int rc = set_attrs<CT>();
     if (rc) return rc;
-    const bool use_gq = CT >= 64 && !c->no_cholqr;
-    // plan: largest leaf count over all bonds decides the workspace
+    bool use_gq = CT >= 64 && !c->no_cholqr;
     const int KC = (CT + KG - 1) / KG * KG;
-    int PMAX = 1, KLMAX = 1, NBMAX = 1;
-    long long MQMAX = 1;
-    const int pmax = use_gq ? APPLY_LEAVES : 512;
-    for (int i = 0; i < d; i++) {
-        Plan t;
-        long long ml = (long long)rk[i] * x->n[i], mr = (long long)x->n[i] * rk[i + 1];
-        plan_bond(CT, ml > mr ? ml : mr, KC, &t, pmax);
-        if (t.P > PMAX) PMAX = t.P;
-        if (t.KL > KLMAX) KLMAX = t.KL;
-        for (long long mm : {ml, mr}) {
-            const int nb = gq::ctas(mm, gq::rows_per_cta(mm, c->nsm, gq::Cfg<CT >= 64 ? CT : 64>::RPB_MAX));
-            NBMAX = nb > NBMAX ? nb : NBMAX;
-        }
-        MQMAX = mr > MQMAX ? mr : MQMAX;
-    }
-    Plan base;
-    plan_bond(CT, 1, KC, &base);
-    base.NH = (CT + H - 1) / H;
-    long long total = carve(&base, PMAX, KLMAX);
-    // grid Cholesky QR: record, partial Gram matrices, Q rows of RIGHT_T bonds
     using GC = gq::Cfg<CT >= 64 ? CT : 64>;
     const long long gq_rec = (GC::REC + 31) / 32 * 32;
-    long long o_gq = (total + 31) / 32 * 32, gq_len = 0;
-    if (use_gq) gq_len = gq_rec + (long long)NBMAX * GC::UP + MQMAX * CT;
-    // two slots of the whole region (bond parity): the truncation sweep runs
-    // the tail of bond i (V replay, Q V_r, swap of core i) on the side stream
-    // while bond i - 1 is factored in the other slot
-    const long long SLOT = (o_gq + gq_len + 31) / 32 * 32;
-    size_t bytes = (size_t)(2 * SLOT) * sizeof(double) + 256;
-    if ((rc = ptt_ws_reserve(c, bytes))) return rc;
+    int PMAX, KLMAX, NBMAX, pmax;
+    long long MQMAX, o_gq, SLOT;
+    Plan base;
+    for (;;) {
+        // plan: largest leaf count over all bonds decides the workspace
+        PMAX = KLMAX = NBMAX = 1;
+        MQMAX = 1;
+        pmax = use_gq ? APPLY_LEAVES : 512;
+        for (int i = 0; i < d; i++) {
+            Plan t;
+            long long ml = (long long)rk[i] * x->n[i], mr = (long long)x->n[i] * rk[i + 1];
+            plan_bond(CT, ml > mr ? ml : mr, KC, &t, pmax);
+            if (t.P > PMAX) PMAX = t.P;
+            if (t.KL > KLMAX) KLMAX = t.KL;
+            for (long long mm : {ml, mr}) {
+                const int nb = gq::ctas(mm, gq::rows_per_cta(mm, c->nsm, GC::RPB_MAX));
+                NBMAX = nb > NBMAX ? nb : NBMAX;
+            }
+            MQMAX = mr > MQMAX ? mr : MQMAX;
+        }
+        plan_bond(CT, 1, KC, &base);
+        base.NH = (CT + H - 1) / H;
+        o_gq = (carve(&base, PMAX, KLMAX) + 31) / 32 * 32;
+        // two slots of the whole region (bond parity): the truncation sweep runs
+        // the tail of bond i (V replay, Q V_r, swap of core i) on the side stream
+        // while bond i - 1 is factored in the other slot
+        SLOT = o_gq;
+        // grid Cholesky QR: record, partial Gram matrices, Q rows of RIGHT_T bonds
+        if (use_gq) SLOT += (gq_rec + (long long)NBMAX * GC::UP + MQMAX * CT + 31) / 32 * 32;
+        if (!(rc = ptt_ws_reserve(c, (size_t)(2 * SLOT) * sizeof(double) + 256))) break;
+        if (!use_gq) return rc;
+        // the grid's share grows with rows x columns, the Householder tree's
+        // hardly: where the first does not fit the GPU beside the train, the
+        // tree alone factors the bonds
+        cudaGetLastError();
+        ptt_set_error(PTT_OK, "");
+        use_gq = false;
+    }
     const size_t cnt_tree = (size_t)PMAX * 4 + 64;
     if ((rc = ptt_counters_reserve(c, cnt_tree + 3))) return rc;
     int* const tick_main = c->d_counters + cnt_tree + 1;  // Fin tickets: the contractions of the main stream,
