@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
     double* sTn = sT + UP;          // the other buffer of it
     double* s_rinv = sTn + UP;      // inverse pivots of sF
     double* s_an = s_rinv + 32;     // 1 / |a_j|
-    double* s_d = s_an + 32;        // |q_j| of the columns kept, their inverses
+    double* s_d = s_an + 32;        // D of the columns kept, its inverse
     double* s_di = s_d + 32;
     unsigned long long* s_tm = (unsigned long long*)(s_di + 32);  // max_j |T_ij| / |a_j|, two buffers
     double* Xs = s_di + 96;         // rpb x XP rows of this CTA
@@ -310,10 +310,11 @@ __global__ void __launch_bounds__(NT, 1) k_cq_factor(const DevDesc* D, int k, in
         // scalars by each warp (the same values)
         {
             const bool on = (live >> lane) & 1u;
-            const double di = on ? 1.0 / dj : 0.0;
-            s_d[lane] = on ? dj : 0.0;
-            s_di[lane] = di;
-            if (stage == 0) s_an[lane] = di;
+            double p2, ip2;
+            pow2_above(dj, &p2, &ip2);
+            s_d[lane] = on ? p2 : 0.0;
+            s_di[lane] = on ? ip2 : 0.0;
+            if (stage == 0) s_an[lane] = on ? 1.0 / dj : 0.0;
             if (warp == 0) s_tm[32 * ((stage + 1) & 1) + lane] = 0ull;
             __syncwarp();
         }

@@ -21,8 +21,12 @@
 //   * s >= 1 and max|G - I| <= FIRST: R_{s+1} = I + striu(E) + diag(E)/2 with E
 //     = G - I, the Cholesky factor of I + E to first order; when max|E| <=
 //     FIRST_DONE that finishes without another Gram stage;
-//   * otherwise R_{s+1} = chol(H) D with D = diag(|q_j|) and H = D^-1 G D^-1
-//     (unit diagonal, so the scale of a column does not matter).  A pivot
+//   * otherwise R_{s+1} = chol(H) D with H = D^-1 G D^-1 and D = diag(the power
+//     of two above |q_j|) (a diagonal in [1/4, 1], so the scale of a column does
+//     not matter, and no rounding: with D = diag(|q_j|) the pivots and their
+//     inverses were each off by the roundings of |q_j|, 1 / |q_j| and H, whose
+//     product is 1 + 1.2e-16 on average, not 1, and a time step added that up to
+//     an error of 5e-15).  A pivot
 //     below PIV is set to PIV and the rest of its row of R to zero: the column
 //     is only rescaled and is orthogonalised against the others in the next
 //     stage, where it has unit norm again.  So every stage resolves another
@@ -49,6 +53,13 @@ constexpr double SMALL = 1e-280;       // squared norms below this lose digits t
 constexpr double LARGE = 1e300;        // and above this are near overflow
 
 enum { RUN = 0, DONE = 1, FALLBACK = 2, FINISH = 4 };
+
+// the power of two above a column norm d > 0, and its inverse
+__device__ __forceinline__ void pow2_above(double d, double* p, double* ip) {
+    const int e = (__double2hiint(d) & 0x7ff00000) + 0x00100000;
+    *p = __hiloint2double(e, 0);
+    *ip = __hiloint2double(0x7fe00000 - e, 0);
+}
 
 // A symmetric or upper triangular matrix is kept as its upper 8 x 8 tiles:
 // tile (I, J), I <= J, is number J (J + 1) / 2 + I (so c columns use the first

@@ -486,8 +486,10 @@ __global__ void __launch_bounds__(NT, 1) k_gq_decide(const DevDesc* D, int k, in
             s_an[j] = on ? 1.0 / dj : 0.0;
             g.rec[C::O_AN + j] = s_an[j];
         }
-        s_d[j] = on ? dj : 0.0;
-        s_di[j] = on ? 1.0 / dj : 0.0;
+        double p2, ip2;
+        pow2_above(dj, &p2, &ip2);
+        s_d[j] = on ? p2 : 0.0;
+        s_di[j] = on ? ip2 : 0.0;
         s_tm[j] = 0ull;
         if (j < c && !(gjj >= 0.0 && gjj < LARGE)) atomicOr(&s_flags, 1);      // NaN, Inf or near overflow
         if (j < c && gjj != 0.0 && gjj < SMALL) atomicOr(&s_flags, 1);

@@ -56,15 +56,15 @@ def stages(A, maxst, tau, clear=True):
             return "done", Q * on if clear else Q, T * on[:, None], s
         if s == maxst - 1:
             return "fallback", Q, T, s
-        di = np.where(on, 1.0 / np.where(on, d, 1.0), 0.0)
         first = s >= 1 and e <= FIRST
         if first:
             diag = np.where(on, 1.0 + 0.5 * (g - 1.0), 0.0)
             F = np.triu(G, 1) * both + np.diag(diag)
             inv = np.where(on, 1.0 / np.where(on, diag, 1.0), 0.0)
         else:
-            R1, inv = factor(G * np.outer(di, di), on)
-            F, inv = R1 * np.where(on, d, 0.0), inv * di
+            p2 = 2.0 ** np.frexp(np.where(on, d, 1.0))[1]  # D: the powers of two above the norms
+            R1, inv = factor(G / np.outer(p2, p2), on)
+            F, inv = R1 * np.where(on, p2, 0.0), inv / p2
         T = F if s == 0 else F @ T
         tm = (np.abs(T) * an).max(axis=1)
         Q = solve(Q, F, inv)
