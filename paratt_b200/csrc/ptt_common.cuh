@@ -120,6 +120,11 @@ static inline bool ptt_device_done(std::atomic<unsigned long long>& mask, unsign
 // previous grid has completed and its writes are visible -- before any memory
 // access -- and then lets the next kernel be scheduled in turn.  Launched
 // without the attribute, the two instructions have no effect.
+// One kernel reads before it waits: k_dot_part (ptt_dot.cu) requests slices of
+// the trains, which nothing in its chain writes.  That holds because the chain
+// starts with a plain launch (k_set_one): everything older on the stream is
+// complete before it starts, and every later kernel of the chain has waited for
+// the one before.
 #define PTT_PDL_ENTRY()                                          \
     do {                                                         \
         asm volatile("griddepcontrol.wait;" ::: "memory");       \

@@ -258,6 +258,9 @@ static int dot_chain(ptt_ctx* c, const ptt_tt* x, const ptt_tt* y, const int* rx
     return PTT_OK;
 }
 
+// The start of a chain of products, to be launched without the programmatic
+// attribute: k_dot_part reads the trains before its wait, which is only safe
+// behind a launch that waited for everything before it.
 __global__ void k_set_one(double* a) { a[0] = 1.0; }
 
 extern "C" int ptt_dot(const ptt_tt* x, const ptt_tt* y, double* out) {

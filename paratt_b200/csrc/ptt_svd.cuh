@@ -89,14 +89,10 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
-// lanes per group (measured against half and twice as many)
-template <int RB>
-__host__ __device__ constexpr int svd_lp() {
-    return 8;
-}
+constexpr int SVD_LP = 8;  // lanes per group: 16 took 888-946 cycles a step at 64 columns where 8 take 800
 template <int RB>
 __host__ __device__ constexpr int svd_nt() {
-    return RB / 4 * svd_lp<RB>();
+    return RB / 4 * SVD_LP;
 }
 // buffers of the moving blocks: two where they fit (one barrier a move), else one
 template <int RB>
@@ -180,7 +176,7 @@ template <int RB>
 __global__ void __launch_bounds__(svd_nt<RB>(), 1) k_svd_jacobi(Plan pl, double* ws, double delta, int maxr, int bond,
                                                                 int* status) {
     PTT_PDL_ENTRY();
-    constexpr int LP = svd_lp<RB>(), NTH = svd_nt<RB>(), NW = NTH / 32, NR = RB / LP;
+    constexpr int LP = SVD_LP, NTH = svd_nt<RB>(), NW = NTH / 32, NR = RB / LP;
     constexpr int S = RB + 2, NBLK = RB / 2, NBUF = svd_nb<RB>();
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) double sm[];
