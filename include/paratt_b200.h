@@ -85,9 +85,11 @@ PTT_API int ptt_ctx_graphs(ptt_ctx* ctx, int on);
  * default) a repeated, column-equilibrated Cholesky-QR sequence -- by one
  * thread-block cluster up to 32 columns, by all SMs (two launches per Gram
  * stage) for 33 to 128 -- which falls back to the Householder TSQR for a bond
- * it cannot make orthonormal; with on == 0 the Householder TSQR only.
- * ptt_ctx_qr_counts returns, summed over the context and its batch workers: [0] factorisations finished by Cholesky QR, [1] fell
- * back, [2] Gram stages of the finished ones (synchronises). */
+ * it cannot make orthonormal, and for a rounding whose workspace does not fit
+ * the GPU; with on == 0 the Householder TSQR only.  ptt_ctx_qr_counts returns,
+ * summed over the context and its batch workers: [0] factorisations finished
+ * by Cholesky QR, [1] fell back, [2] Gram stages of the finished ones
+ * (synchronises). */
 PTT_API int ptt_ctx_cholqr(ptt_ctx* ctx, int on);
 /* Precision of the contractions of the rounding's 33- to 64-column bonds
  * (no counterpart in the reference): with on != 0 the Gram matrices of the

@@ -251,8 +251,8 @@ extern "C" int ptt_axpby(double a, const ptt_tt* x, double b, const ptt_tt* y, p
 // RUNS: a warp walks runs of fibers (j, lz), lz = ly + ry1 jx; lane: rows iz = 2
 // lane + 64 b and the next, iz = ky + ry ix, so the row's factors are found once
 // and every store is 16 bytes.  Bound by the writes (8 bytes per element; x and y
-// come from L1/L2): d = 40, n = 256, ranks 8 x 8, 336 MB: 140 us with a division
-// and an 8-byte store per element, 73 now (4.6 TB/s, 59 back to back).  With few
+// come from L1/L2): d = 40, n = 256, ranks 8 x 8, 329 MB: 140 us with a division
+// and an 8-byte store per element, 73 now (4.5 TB/s, 59 back to back).  With few
 // runs it is slower: 10 modes of 17, ranks 8 x 16 (2560 runs) 20.6 us a product,
 // 16.6 fiber by fiber; 20 modes of 100, ranks 4 x 8 (4480) 18.8 and 23.4.
 constexpr int RUNS_HADAMARD = 4096;
@@ -530,8 +530,8 @@ __device__ __forceinline__ double sten_at(const double* xc, int r, int n, int i,
 // and writes both of y's fibers that come from each, [x; 0] and [S x; x]; the
 // stencil slides along the run in registers, so every fiber of x is read once
 // (plus two per run) and all accesses are 16 bytes.  Bound by HBM, four bytes
-// written per byte read: d = 40, n = 256, r = 64, 1.68 GB: 504 us with 8-byte
-// accesses, a division per fiber and the stencil's neighbours re-read, 267 now (6.3
+// written per byte read: d = 40, n = 256, r = 64, 1.59 GB: 499 us with 8-byte
+// accesses, a division per fiber and the stencil's neighbours re-read, 267 now (6.0
 // TB/s).  At 2000 runs both take as long (10 modes of 17, rank 100: 25.6 us an
 // operator; fiber by fiber rank 96 takes 23.1); 40 modes of 32, rank 32 (2560)
 // 21.5, and rank 31 27.0 fiber by fiber.
